@@ -1356,26 +1356,23 @@ struct RebalanceGraph {
 
 struct RefineWork {
     Buf<unsigned char> cache_raw;
-    Buf<i32> targets, list, movers, saved_labels, clist, clist_alt, cand;
-    Buf<i64> gains, pos;
+    Buf<i32> targets, list, movers, saved_labels, cand, bucket;
+    Buf<i64> gains;
     Buf<PropRec> props;
-    Buf<unsigned char> locks, flags;
-    Buf<double> gpw;
-    Buf<i32> bucket;
-    Buf<u64> rank, counts, offsets, saved_pw, excl, keys, keys_alt, bucket_base, scratch;
+    Buf<unsigned char> locks, flags, item_part;
+    Buf<CrossItem> items;
+    Buf<CrossParts> cross;   // of the sources, of the destinations
+    Buf<u64> counts, saved_pw, scratch;
     Buf<RefineCounters> ctr;
     void ensure(Device& d, i64 n, int k, size_t cache_bytes) {
         const size_t s = static_cast<size_t>(n) + 1;
         cache_raw.ensure(d, cache_bytes);
         targets.ensure(d, s); list.ensure(d, s); movers.ensure(d, s); saved_labels.ensure(d, s);
-        clist.ensure(d, s); clist_alt.ensure(d, s); cand.ensure(d, s);
-        gains.ensure(d, s); pos.ensure(d, s); props.ensure(d, s);
-        locks.ensure(d, s); flags.ensure(d, s);
-        gpw.ensure(d, s); bucket.ensure(d, s);
-        rank.ensure(d, s); excl.ensure(d, s); keys.ensure(d, s); keys_alt.ensure(d, s);
+        cand.ensure(d, s); bucket.ensure(d, s);
+        gains.ensure(d, s); props.ensure(d, s);
+        locks.ensure(d, s); flags.ensure(d, s); item_part.ensure(d, s);
+        items.ensure(d, s); cross.ensure(d, 2);
         counts.ensure(d, static_cast<size_t>(k) * kBalWidth);
-        offsets.ensure(d, static_cast<size_t>(k) * kBalWidth);
-        bucket_base.ensure(d, static_cast<size_t>(k) * kBalWidth);
         saved_pw.ensure(d, 32);
         scratch.ensure(d, 8);
         ctr.ensure(d, 1);
@@ -1560,33 +1557,6 @@ gp_refine_stats refine_level(Device& d, const DGraph<T>& g, RefineWork& w, i32* 
         }
         return h.c.movers;
     };
-    auto deterministic_ranks = [&]() {
-        // candidates in ascending vertex order, sorted by (bucket, gpw desc)
-        exclusive_scan<i64>(d, HasBucket{w.bucket.get(), w.cand.get()}, w.pos.get(), ncand,
-                            reinterpret_cast<i64*>(w.scratch.get() + 1));
-        launch(d, "compact_bucket_kernel", compact_bucket_kernel, blocks_for(ncand, kThreads), kThreads, 0, ncand,
-               w.cand.get(), w.bucket.get(), w.pos.get(), w.clist.get());
-        GP_LAUNCH();
-        i64 count = 0;
-        fetch(d, &count, reinterpret_cast<i64*>(w.scratch.get() + 1), 1);
-        w.counts.zero(d);
-        if (count == 0) return;
-        launch(d, "rank_keys_kernel", rank_keys_kernel, blocks_for(count, kThreads), kThreads, 0, count, w.clist.get(), w.gpw.get(),
-                                                                                w.bucket.get(), 0, w.keys.get());
-        GP_LAUNCH();
-        radix_sort<u64, i32>(d, w.keys.get(), w.clist.get(), w.keys_alt.get(), w.clist_alt.get(), count, 0, 64);
-        launch(d, "rank_keys_kernel", rank_keys_kernel, blocks_for(count, kThreads), kThreads, 0, count, w.clist.get(), w.gpw.get(),
-                                                                                w.bucket.get(), 1, w.keys.get());
-        GP_LAUNCH();
-        radix_sort<u64, i32>(d, w.keys.get(), w.clist.get(), w.keys_alt.get(), w.clist_alt.get(), count, 0,
-                             std::max(1, bit_width_u64(static_cast<u64>(k) * kBalWidth)));
-        exclusive_scan<u64>(d, ListWeight<W>{w.clist.get(), vw}, w.excl.get(), count);
-        launch(d, "bucket_heads_kernel", bucket_heads_kernel, blocks_for(count, kThreads), kThreads, 0, count, w.clist.get(), w.bucket.get(),
-                                                                                   w.excl.get(), w.bucket_base.get());
-        launch(d, "bucket_ranks_kernel", bucket_ranks_kernel<W>, blocks_for(count, kThreads), kThreads, 0, 
-            count, w.clist.get(), w.bucket.get(), w.excl.get(), w.bucket_base.get(), vw, w.rank.get(), w.counts.get());
-        GP_LAUNCH();
-    };
     // The rebalance loop as one graph launch: the iterations' launches are
     // captured once per level into the body of a WHILE node, and
     // rebalance_continue_kernel decides on the device whether another
@@ -1654,44 +1624,47 @@ gp_refine_stats refine_level(Device& d, const DGraph<T>& g, RefineWork& w, i32* 
     auto rebalance = [&]() -> bool {
         if (maximum() <= cap) return true;
         i64* cand_count = reinterpret_cast<i64*>(w.scratch.get() + 6);
-        exclusive_scan<i64>(d, InOverloaded{labels, pw, cap}, w.pos.get(), n, cand_count);
-        launch(d, "compact_overloaded_kernel", compact_overloaded_kernel, blocks_for(n, kThreads), kThreads, 0, n,
-               labels, pw, cap, w.pos.get(), w.cand.get());
-        // The candidate count stays on the device unless the host needs it
-        // (the deterministic ranks size their sorts by it): the kernels read
-        // it, and the grids are sized for the level's n.
-        const bool host_count = deterministic || d.prof || trace().on;
+        GP_CUDA(cudaMemsetAsync(cand_count, 0, sizeof(i64), d.stream));
+        launch(d, "collect_overloaded_kernel", collect_overloaded_kernel, stride_grid(d, n, kCollectTile), kThreads, 0, n,
+               labels, k, pw, cap, w.cand.get(), cand_count);
+        // The candidate count stays on the device unless the host needs it:
+        // the kernels read it, and the grids are sized for the level's n.
+        const bool host_count = d.prof || trace().on;
         if (host_count) fetch(d, &ncand, cand_count, 1);
         else ncand = n;
         const i64* dev_count = host_count ? nullptr : cand_count;
-        const int cgrid = host_count ? blocks_for(std::max<i64>(ncand, 1), kThreads) : stride_grid(d, n);
-        w.counts.zero(d);   // bucket_scan_kernel leaves the counts zero for the next pass
-        // one iteration's launches up to the movers (refine_incremental.cuh:303-326)
+        const int cgrid = stride_grid(d, std::max<i64>(ncand, 1));
+        w.counts.zero(d);   // every pass over the counts leaves them zero for the next one
+        CrossParts* sources = w.cross.get();
+        CrossParts* dests = sources + 1;
+        // one iteration's launches up to the movers (refine_incremental.cuh:303-326).
+        // Selecting by threshold replaced two sorts of all candidates by
+        // (bucket, gain, vertex) per iteration, about 50 launches and two round
+        // trips: RMAT-20 k = 32 190 -> 109 ms, 320^3 grid k = 8 275 -> 157 ms,
+        // 64x64 grid 14.0 -> 8.8 ms per deterministic partition.
         auto select = [&]() {
-            GP_CUDA(cudaMemsetAsync(ctr, 0, sizeof(RefineCounters), d.stream));
             launch(d, "rebalance_proposals_kernel", rebalance_proposals_kernel<C, W>, cgrid, kThreads, 0, ncand,
-                   dev_count, w.cand.get(), cache, labels, vw, k, pw, cap, thresholds.t, deterministic ? 1 : 0, w.targets.get(),
-                   w.gpw.get(), w.bucket.get(), w.rank.get(), w.counts.get());
-            GP_LAUNCH();
-            if (deterministic) deterministic_ranks();
-            launch(d, "bucket_scan_kernel", bucket_scan_kernel, k, kThreads, 0, w.counts.get(), w.offsets.get());
-            launch(d, "select_sources_kernel", select_sources_kernel<W>, cgrid, kThreads, 0, ncand, dev_count,
-                   w.cand.get(),
-                   w.bucket.get(), w.rank.get(), w.offsets.get(), pw, cap, w.targets.get(), vw, deterministic ? 1 : 0,
-                   w.counts.get());
-            GP_LAUNCH();
-            if (deterministic) deterministic_ranks();
-            launch(d, "bucket_scan_kernel", bucket_scan_kernel, k, kThreads, 0, w.counts.get(), w.offsets.get());
-            launch(d, "select_destinations_kernel", select_destinations_kernel<W>, cgrid, kThreads, 0, ncand,
-                   dev_count, w.cand.get(), w.bucket.get(), w.rank.get(), w.offsets.get(), pw, cap, vw, w.flags.get(),
-                   w.movers.get(), ctr);
+                   dev_count, w.cand.get(), cache, labels, vw, k, pw, cap, thresholds.t, w.targets.get(),
+                   w.bucket.get(), w.counts.get());
+            launch(d, "cross_sources_kernel", cross_sources_kernel, k, kSelectThreads, 0, pw, cap, w.counts.get(),
+                   sources, ctr);
+            launch(d, "select_sources_kernel", select_sources_kernel<C, W>, cgrid, kThreads, 0, ncand, dev_count,
+                   w.cand.get(), w.bucket.get(), cache, labels, w.targets.get(), vw, k, w.counts.get(), sources,
+                   w.items.get(), w.item_part.get());
+            launch(d, "resolve_sources_kernel", resolve_sources_kernel<W>, kSelectCluster, kSelectThreads, 0, k, pw,
+                   cap, w.bucket.get(), vw, w.counts.get(), sources, dests, w.items.get(), w.item_part.get());
+            launch(d, "select_destinations_kernel", select_destinations_kernel<C, W>, cgrid, kThreads, 0, ncand,
+                   dev_count, w.cand.get(), w.bucket.get(), cache, labels, w.targets.get(), vw, k, dests,
+                   w.items.get(), w.item_part.get(), w.flags.get(), w.movers.get(), ctr);
+            launch(d, "resolve_destinations_kernel", resolve_destinations_kernel<W>, k, kSelectThreads, 0, vw, dests,
+                   w.items.get(), w.item_part.get(), w.flags.get(), w.movers.get(), ctr);
             GP_LAUNCH();
         };
         const int limit = 2 * k + 4;
         // Building the graph costs a few hundred microseconds per level, about
         // the host round trips of ten iterations: mode 1 captures once this
         // level's host loop has run kGraphLoopAfter iterations, mode 2 at once.
-        if (!host_count && (d.graph_loops == 2 || (d.graph_loops == 1 && (rgraph.exec ||
+        if (!host_count && !deterministic && (d.graph_loops == 2 || (d.graph_loops == 1 && (rgraph.exec ||
                                                                            host_iterations >= kGraphLoopAfter))))
             return rebalance_on_device(select, limit);
         for (int it = 0; it < limit && maximum() > cap; ++it) {

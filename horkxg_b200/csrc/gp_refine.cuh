@@ -7,12 +7,15 @@
 //   cache+cut update and the commit then touch proposers/movers only;
 // * list-driven kernels use a fixed grid with grid-stride loops so the host
 //   never has to size a launch from a device count;
-// * the rebalance ranks vertices inside a (source, gain bucket, section)
-//   bucket either with atomics in arbitrary order (the reference's
-//   behaviour) or, in deterministic mode, by (gain per weight descending,
-//   vertex ascending) through a stable radix sort, which makes labels
-//   bit-reproducible.
+// * the rebalance moves, per (source part, gain bucket, section), vertices in
+//   the order (gain per weight descending, vertex ascending).  The order is
+//   needed inside one bucket per part only: buckets before the one that
+//   crosses the part's quota are taken whole, later ones not at all, and the
+//   crossing bucket is cut at a threshold found by a weighted radix selection,
+//   so nothing is sorted and labels are bit-reproducible.
 #pragma once
+
+#include <cooperative_groups.h>
 
 #include "gp_prim.cuh"
 #include "gp_sclp.cuh"
@@ -100,6 +103,13 @@ __device__ __forceinline__ u64 group_sum(unsigned peers, u64 w) {
         }
         return sum;
     }
+}
+
+// group_sum of weights that usually are small: one 32-bit reduction when no
+// lane's weight reaches 2^26 (32 of them then fit 32 bits).  All 32 lanes call it.
+__device__ __forceinline__ u64 weight_group_sum(unsigned peers, u64 w) {
+    if (__any_sync(0xffffffffu, (w >> 26) != 0)) return group_sum<u64>(peers, w);
+    return __reduce_add_sync(peers, static_cast<u32>(w));
 }
 
 // One vertex's k cache entries into registers, with 16-byte loads when the
@@ -511,26 +521,38 @@ __global__ void __launch_bounds__(kThreads) apply_big_rows_kernel(
 }
 
 // incremental_commit (src/refine_incremental.cuh:97-109); also clears the
-// mover flag so that `flags` is all-zero outside an apply.  Part-weight
-// changes are summed per block in shared memory first: all movers hit the
-// same k counters, so global atomics would serialise.
+// mover flag so that `flags` is all-zero outside an apply.  All movers hit the
+// same k part weights, and after an LP round or a rebalance most lanes of a
+// warp share a part, so the changes are summed per warp and part, then per
+// block in shared memory, before one global atomic per block and part.
 template <typename W>
 __global__ void commit_kernel(const i32* __restrict__ movers, const RefineCounters* ctr_in,
                               i32* labels, const i32* __restrict__ targets, const W* __restrict__ vw, u64* pw,
                               unsigned char* locks, unsigned char* flags, int lp) {
     __shared__ unsigned long long delta[32];
+    const i64 count = ctr_in->movers;
+    if (static_cast<i64>(blockIdx.x) * blockDim.x >= count) return;
     if (threadIdx.x < 32) delta[threadIdx.x] = 0;
     __syncthreads();
-    const i64 count = ctr_in->movers;
-    for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * blockDim.x) {
-        const i32 v = movers[i];
-        const i32 s = labels[v], t = targets[v];
-        const u64 w = static_cast<u64>(weight_at(vw, v));
-        atomicAdd(&delta[s], 0ULL - w);
-        atomicAdd(&delta[t], static_cast<unsigned long long>(w));
-        labels[v] = t;
-        if (lp) locks[v] = 1;
-        flags[v] = 0;
+    const int lane = threadIdx.x & 31;
+    for (i64 base = static_cast<i64>(blockIdx.x) * blockDim.x; base < count; base += static_cast<i64>(gridDim.x) * blockDim.x) {
+        const i64 i = base + threadIdx.x;
+        i32 s = -1, t = -1;
+        u64 w = 0;
+        if (i < count) {
+            const i32 v = movers[i];
+            s = labels[v];
+            t = targets[v];
+            w = static_cast<u64>(weight_at(vw, v));
+            labels[v] = t;
+            if (lp) locks[v] = 1;
+            flags[v] = 0;
+        }
+        const unsigned from = __match_any_sync(0xffffffffu, s), to = __match_any_sync(0xffffffffu, t);
+        const u64 out = vw ? weight_group_sum(from, w) : static_cast<u64>(__popc(from));
+        const u64 in = vw ? weight_group_sum(to, w) : static_cast<u64>(__popc(to));
+        if (s >= 0 && lane == __ffs(from) - 1) atomicAdd(&delta[s], 0ULL - out);
+        if (t >= 0 && lane == __ffs(to) - 1) atomicAdd(&delta[t], static_cast<unsigned long long>(in));
     }
     __syncthreads();
     if (threadIdx.x < 32 && delta[threadIdx.x]) atomic_add_u64(&pw[threadIdx.x], delta[threadIdx.x]);
@@ -555,51 +577,49 @@ __device__ __forceinline__ int gain_bucket(double g, const BucketThresholds& th)
     return 25 + (lo - 23);
 }
 
-// Ranks of weighted items in per-key counters with one atomic per key and
-// warp: the lanes that share a key take consecutive ranges in lane order, as
-// if their atomicAdds had run back to back (the reference's ranks come from
-// plain atomicAdds in scheduling order, so any such order is one it can
-// produce).  All 32 lanes call it; key < 0 means no item.
-__device__ __forceinline__ u64 warp_rank_add(int key, u64 w, bool unit, u64* counts) {
-    const int lane = threadIdx.x & 31;
-    const unsigned peers = __match_any_sync(0xffffffffu, key);
-    const unsigned lower = peers & lanemask_lt();
-    u64 before = 0, total = 0;
-    if (unit) {
-        before = static_cast<u64>(__popc(lower));
-        total = static_cast<u64>(__popc(peers));
-    } else {
-#pragma unroll
-        for (int s = 0; s < 32; ++s) {
-            const u64 x = __shfl_sync(0xffffffffu, w, s);
-            if ((peers >> s) & 1u) {
-                total += x;
-                if (s < lane) before += x;
-            }
-        }
+// Weight sums per bucket gathered by one block in shared memory and added to
+// the global counts once at its end.  The candidates of a large part crowd
+// into a few buckets (the interior of a grid part has one gain: 16 buckets),
+// so a global atomic per warp and bucket would queue at a few addresses.
+// A key that finds its few slots taken goes to the global count directly.
+struct BucketTable {
+    static constexpr int kSlots = 512, kProbes = 4;
+    int key[kSlots];
+    u64 sum[kSlots];
+    __device__ void clear() {
+        for (int i = threadIdx.x; i < kSlots; i += blockDim.x) { key[i] = -1; sum[i] = 0; }
     }
-    const int leader = __ffs(peers) - 1;
-    u64 base = 0;
-    if (key >= 0 && lane == leader) base = atomic_add_u64(&counts[key], total);
-    base = __shfl_sync(0xffffffffu, base, leader);
-    return base + before;
-}
+    // All 32 lanes of a warp call it; b < 0 means no item.
+    __device__ void add(int b, u64 w, bool unit, u64* counts) {
+        const unsigned peers = __match_any_sync(0xffffffffu, b);
+        const u64 total = unit ? static_cast<u64>(__popc(peers)) : weight_group_sum(peers, w);
+        if (b < 0 || (threadIdx.x & 31) != __ffs(peers) - 1) return;
+        int slot = static_cast<int>(mix32(static_cast<u32>(b)) % kSlots);
+        for (int probe = 0; probe < kProbes; ++probe) {
+            const int found = atomicCAS(&key[slot], -1, b);
+            if (found == -1 || found == b) {
+                atomic_add_u64(&sum[slot], total);
+                return;
+            }
+            slot = (slot + 1) % kSlots;
+        }
+        atomic_add_u64(&counts[b], total);
+    }
+    __device__ void flush(u64* counts) {
+        for (int i = threadIdx.x; i < kSlots; i += blockDim.x)
+            if (key[i] >= 0) atomic_add_u64(&counts[key[i]], sum[i]);
+    }
+};
 
-// incremental_rebalance_proposals + balance_source_histogram
-// (src/refine_incremental.cuh:111-186).  Atomic mode ranks here; the
-// deterministic mode appends candidates (ascending vertex order is restored by
-// the scan-based compaction that follows).
-// One rebalance candidate: the destination with slack that it is best
-// connected to (ties: more slack), a zero-connection vertex spread over the
-// parts with slack by a hashed ticket; returns the vertex's bucket
-// (source part, gain-per-weight bucket, hashed section) or -1.
+// One rebalance candidate (incremental_rebalance_proposals,
+// src/refine_incremental.cuh:111-165): the destination with slack that it is
+// best connected to (ties: more slack), a zero-connection vertex spread over
+// the parts with slack by a hashed ticket; returns the vertex's bucket (source
+// part, gain-per-weight bucket, hashed section) or -1.
 template <typename C, typename W>
-__device__ __forceinline__ int rebalance_choice(i64 v, const C* __restrict__ cache, const i32* __restrict__ labels,
-                                                const W* __restrict__ vw, int k, const u64* spw, u64 cap,
-                                                const BucketThresholds& th, i32* targets, double* gpw, i32* bucket,
-                                                u64& w) {
-    targets[v] = -1;
-    bucket[v] = -1;
+__device__ __forceinline__ int rebalance_choice(i64 v, const C* cache, const i32* labels, const W* __restrict__ vw,
+                                                int k, const u64* spw, u64 cap, const BucketThresholds& th,
+                                                i32* targets, u64& w) {
     const i32 s = labels[v];
     if (spw[s] <= cap) return -1;
     w = static_cast<u64>(weight_at(vw, v));
@@ -638,193 +658,491 @@ __device__ __forceinline__ int rebalance_choice(i64 v, const C* __restrict__ cac
     if (best < 0) return -1;
     const double gain = best_conn >= current ? static_cast<double>(best_conn - current)
                                              : -static_cast<double>(current - best_conn);
-    const double g = gain / static_cast<double>(w);
     targets[v] = best;
-    gpw[v] = g;
-    const int b = s * kBalWidth + gain_bucket(g, th) * kBalSections +
-                  static_cast<int>(mix32(static_cast<u32>(v)) % kBalSections);
-    bucket[v] = b;
-    return b;
+    return s * kBalWidth + gain_bucket(gain / static_cast<double>(w), th) * kBalSections +
+           static_cast<int>(mix32(static_cast<u32>(v)) % kBalSections);
 }
+
+// Order of vertex v inside its bucket: gain per weight descending as an
+// ascending integer (v itself breaks ties).  The gain is that of the chosen
+// destination, whose connection rebalance_choice compared: a destination taken
+// by ticket has connection 0 there as here.
+template <typename C, typename W>
+__device__ __forceinline__ u64 bucket_order(i64 v, i32 s, i32 t, const C* cache, const W* __restrict__ vw, int k) {
+    const u64 current = static_cast<u64>(cache[v * k + s]), conn = static_cast<u64>(cache[v * k + t]);
+    const double gain = conn >= current ? static_cast<double>(conn - current) : -static_cast<double>(current - conn);
+    double g = gain / static_cast<double>(static_cast<u64>(weight_at(vw, v)));
+    if (g == 0.0) g = 0.0;   // -0 and +0 tie
+    const u64 b = static_cast<u64>(__double_as_longlong(g));
+    const u64 ord = (b & 0x8000000000000000ULL) ? ~b : (b | 0x8000000000000000ULL);
+    return ~ord;
+}
+
+// The list of items whose bucket crosses its part's quota, and per part the
+// crossing bucket (kBalWidth: none) with the quota left for it.
+struct CrossItem {
+    u64 key;   // bucket_order
+    i32 i;     // candidate index
+    i32 v;     // vertex
+};
+
+struct CrossParts {
+    u64 left[32];
+    int bucket[32];
+    u32 count;      // items in the list
+    u32 pad;
+};
 
 // The rebalance kernels run over list[0, n), or over list[0, *count) when
 // `count` is given (the candidate count left on the device, no round trip);
-// their grid-stride loops keep whole warps together for the warp ranks.
+// their grid-stride loops keep whole warps together for the warp collectives.
 __device__ __forceinline__ i64 list_length(i64 n, const i64* count) { return count ? *count : n; }
 
-// Over the candidate list (vertices of overloaded parts); part weights are
-// staged in shared memory.
+// Vertices of the parts above capacity, in any order: the only rebalance
+// candidates, and a superset of them for the whole rebalance (destinations
+// never exceed the capacity, so no part becomes overloaded and vertices only
+// leave).
+// Each block appends the vertices of 2048 consecutive ids at once: one atomic
+// per tile, and the cache rows of neighbouring list entries stay close.
+constexpr int kCollectItems = 8;
+constexpr int kCollectTile = kThreads * kCollectItems;
+
+__global__ void __launch_bounds__(kThreads) collect_overloaded_kernel(i64 n, const i32* __restrict__ labels, int k,
+                                                                      const u64* __restrict__ pw, u64 cap, i32* list,
+                                                                      i64* count) {
+    __shared__ u32 over;
+    __shared__ int warp_base[kWarps];
+    __shared__ i64 tile_base;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 0) {
+        const u32 m = __ballot_sync(0xffffffffu, lane < k && pw[lane] > cap);
+        if (lane == 0) over = m;
+    }
+    __syncthreads();
+    const u32 parts = over;
+    for (i64 base = static_cast<i64>(blockIdx.x) * kCollectTile; base < n; base += static_cast<i64>(gridDim.x) * kCollectTile) {
+        unsigned took[kCollectItems];
+        int mine = 0;
+        const i64 v0 = base + warp * 32 * kCollectItems + lane;
+#pragma unroll
+        for (int j = 0; j < kCollectItems; ++j) {
+            const i64 v = v0 + j * 32;
+            took[j] = __ballot_sync(0xffffffffu, v < n && ((parts >> labels[v]) & 1u));
+            mine += __popc(took[j]);
+        }
+        if (lane == 0) warp_base[warp] = mine;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int sum = 0;
+            for (int w = 0; w < kWarps; ++w) { const int c = warp_base[w]; warp_base[w] = sum; sum += c; }
+            tile_base = sum ? static_cast<i64>(atomic_add_u64(reinterpret_cast<u64*>(count), static_cast<u64>(sum))) : 0;
+        }
+        __syncthreads();
+        i64 at = tile_base + warp_base[warp];
+#pragma unroll
+        for (int j = 0; j < kCollectItems; ++j) {
+            if ((took[j] >> lane) & 1u) list[at + __popc(took[j] & lanemask_lt())] = static_cast<i32>(v0 + j * 32);
+            at += __popc(took[j]);
+        }
+        __syncthreads();   // warp_base and tile_base are free again
+    }
+}
+
+// Choices of the candidates and the weight of every source bucket
+// (balance_source_histogram, src/refine_incremental.cuh:167-186); part weights
+// are staged in shared memory.
 template <typename C, typename W>
 __global__ void rebalance_proposals_kernel(i64 n, const i64* count, const i32* __restrict__ list,
                                            const C* __restrict__ cache, const i32* __restrict__ labels,
                                            const W* __restrict__ vw, int k, const u64* __restrict__ pw, u64 cap,
-                                           BucketThresholds th, int deterministic, i32* targets, double* gpw,
-                                           i32* bucket, u64* rank, u64* counts) {
+                                           BucketThresholds th, i32* targets, i32* bucket, u64* counts) {
     __shared__ u64 spw[32];
+    __shared__ BucketTable table;
+    n = list_length(n, count);
+    if (static_cast<i64>(blockIdx.x) * blockDim.x >= n) return;
     if (threadIdx.x < 32) spw[threadIdx.x] = static_cast<int>(threadIdx.x) < k ? pw[threadIdx.x] : ~0ULL;
+    table.clear();
     __syncthreads();
-    n = list_length(n, count);
     for (i64 base = static_cast<i64>(blockIdx.x) * blockDim.x; base < n; base += static_cast<i64>(gridDim.x) * blockDim.x) {
         const i64 i = base + threadIdx.x;
-        const i64 v = i < n ? (list ? list[i] : i) : 0;
         u64 w = 0;
-        const int b = i < n ? rebalance_choice(v, cache, labels, vw, k, spw, cap, th, targets, gpw, bucket, w) : -1;
-        if (!deterministic) {
-            const u64 r = warp_rank_add(b, w, vw == nullptr, counts);
-            if (b >= 0) rank[v] = r;
-        }
-    }
-}
-
-// balance_scan_buckets (src/refine_incremental.cuh:188-202): exclusive scan
-// of the 800 buckets of each part, block per part.  The counts are left
-// zero for the next ranking pass.
-__global__ void __launch_bounds__(kThreads) bucket_scan_kernel(u64* counts, u64* offsets) {
-    __shared__ u64 sh[kWarps + 1];
-    constexpr int kPer = (kBalWidth + kThreads - 1) / kThreads;   // 4
-    u64 vals[kPer];
-    u64 local = 0;
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-        const int b = threadIdx.x * kPer + i;
-        vals[i] = b < kBalWidth ? counts[blockIdx.x * kBalWidth + b] : 0;
-        if (b < kBalWidth) counts[blockIdx.x * kBalWidth + b] = 0;
-        local += vals[i];
-    }
-    u64 run = block_exclusive_sum(local, sh, static_cast<u64*>(nullptr));
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-        const int b = threadIdx.x * kPer + i;
-        if (b < kBalWidth) offsets[blockIdx.x * kBalWidth + b] = run;
-        run += vals[i];
-    }
-}
-
-// balance_select_sources (src/refine_incremental.cuh:204-217)
-template <typename W>
-__global__ void select_sources_kernel(i64 n, const i64* count, const i32* __restrict__ list, i32* bucket, u64* rank,
-                                      const u64* offsets, const u64* pw, u64 cap, const i32* targets, const W* vw,
-                                      int deterministic, u64* counts) {
-    n = list_length(n, count);
-    for (i64 base = static_cast<i64>(blockIdx.x) * blockDim.x; base < n; base += static_cast<i64>(gridDim.x) * blockDim.x) {
-        const i64 i = base + threadIdx.x;
-        const i64 v = i < n ? (list ? list[i] : i) : 0;
-        int d = -1;
-        if (i < n && bucket[v] >= 0) {
-            const int b = bucket[v], s = b / kBalWidth;
-            if (offsets[b] + rank[v] >= pw[s] - cap) {
-                bucket[v] = -1;
-            } else {
-                d = targets[v] * kBalWidth + b % kBalWidth;
-                bucket[v] = d;
-            }
-        }
-        if (!deterministic) {
-            const u64 r = warp_rank_add(d, i < n ? static_cast<u64>(weight_at(vw, v)) : 0, vw == nullptr, counts);
-            if (d >= 0) rank[v] = r;
-        }
-    }
-}
-
-// balance_select_destinations (src/refine_incremental.cuh:219-232).
-template <typename W>
-__global__ void select_destinations_kernel(i64 n, const i64* count, const i32* __restrict__ list, const i32* bucket,
-                                           const u64* rank, const u64* offsets, const u64* pw, u64 cap, const W* vw,
-                                           unsigned char* flags, i32* movers, RefineCounters* ctr) {
-    n = list_length(n, count);
-    for (i64 base = static_cast<i64>(blockIdx.x) * blockDim.x; base < n; base += static_cast<i64>(gridDim.x) * blockDim.x) {
-        const i64 i = base + threadIdx.x;
-        bool move = false;
-        i64 v = 0;
+        int b = -1;
         if (i < n) {
-            v = list ? list[i] : i;
-            const int b = bucket[v];
-            if (b >= 0) {
-                const u64 before = offsets[b] + rank[v];
-                const u64 slack = cap - pw[b / kBalWidth];
-                move = before <= slack && static_cast<u64>(weight_at(vw, v)) <= slack - before;
+            b = rebalance_choice(static_cast<i64>(list[i]), cache, labels, vw, k, spw, cap, th, targets, w);
+            bucket[i] = b;
+        }
+        table.add(b, w, vw == nullptr, counts);
+    }
+    __syncthreads();
+    table.flush(counts);
+}
+
+constexpr int kSelectThreads = 1024;
+constexpr int kSelectWarps = kSelectThreads / 32;
+static_assert(kBalWidth <= kSelectThreads, "one thread per bucket of a part");
+
+// Exclusive block-wide sum over kSelectThreads threads; `shared` needs
+// kSelectWarps entries.
+__device__ __forceinline__ u64 select_exclusive_sum(u64 v, u64* shared) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const u64 inc = warp_inclusive_sum(v);
+    __syncthreads();
+    if (lane == 31) shared[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        const u64 s = shared[lane];
+        shared[lane] = warp_inclusive_sum(s) - s;
+    }
+    __syncthreads();
+    return shared[warp] + inc - v;
+}
+
+// Finds the bucket that crosses part p's quota among its kBalWidth bucket
+// weights, which are left zero for the next pass (balance_scan_buckets,
+// src/refine_incremental.cuh:188-202).  The quota is used up before a bucket's
+// end: an item is taken while the weight before it is below the quota
+// (SOURCES), or while the weight up to its own end is within it
+// (!SOURCES).  A block of kSelectThreads.
+template <bool SOURCES>
+__device__ void cross_bucket(int p, u64 quota, u64* counts, CrossParts* cross, u64* shared) {
+    const int b = threadIdx.x;
+    u64 w = 0;
+    if (b < kBalWidth) {
+        w = counts[p * kBalWidth + b];
+        counts[p * kBalWidth + b] = 0;
+    }
+    if (b == 0) cross->bucket[p] = kBalWidth;
+    const u64 before = select_exclusive_sum(w, shared);
+    const bool crosses = SOURCES ? before < quota && before + w >= quota : before <= quota && before + w > quota;
+    if (crosses && b < kBalWidth) {
+        cross->bucket[p] = b;
+        cross->left[p] = quota - before;
+    }
+    __syncthreads();
+}
+
+struct SelectShared {
+    u64 scan[kSelectWarps];
+    u64 hist[256];
+    u32 members[256];
+    u64 key_and, key_or;
+    u32 v_and, v_or;
+    u64 left;              // quota left for the items that match the threshold
+    u32 count, few;
+    int digit;
+    static constexpr u32 kItems = 2048;
+    u64 key[kItems];
+    i32 v[kItems];
+    i32 i[kItems];
+    static constexpr u32 kFew = 128;
+    u64 few_key[kFew], few_w[kFew];
+    u32 few_v[kFew];
+};
+
+// The items of part p's crossing bucket that are taken: their order's
+// longest prefix within the quota.  A threshold is built from the high end of
+// (key, v), eight varying bits a step: the weights of the items that match it
+// so far are summed by digit, and the digit that crosses what is left of the
+// quota extends it.  Bits in which the items agree cost no step, and once at
+// most kFew items match they are ranked directly, eight lanes an item (a
+// step costs a microsecond of barriers, so most lists finish after one or
+// two).  Lists of up to kItems items are staged in shared memory.
+// f(item index, v, taken) is called for every item of the part.  A block of
+// kSelectThreads.
+template <bool SOURCES, typename W, typename F>
+__device__ void resolve_bucket(int p, const CrossParts* cross, const CrossItem* items,
+                               const unsigned char* item_part, const W* __restrict__ vw, SelectShared& sh, F f) {
+    const u32 total = cross->count;
+    if (cross->bucket[p] == kBalWidth) return;   // uniform over the block
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        sh.count = sh.few = 0;
+        sh.key_and = ~0ULL; sh.key_or = 0; sh.v_and = ~0u; sh.v_or = 0;
+        sh.left = cross->left[p];
+    }
+    __syncthreads();
+    u64 ka = ~0ULL, ko = 0;
+    u32 va = ~0u, vo = 0;
+    for (u32 j = threadIdx.x; j < total; j += kSelectThreads) {
+        if (item_part[j] != p) continue;
+        const CrossItem x = items[j];
+        ka &= x.key; ko |= x.key;
+        va &= static_cast<u32>(x.v); vo |= static_cast<u32>(x.v);
+        const u32 at = atomicAdd(&sh.count, 1u);
+        if (at < SelectShared::kItems) { sh.key[at] = x.key; sh.v[at] = x.v; sh.i[at] = x.i; }
+    }
+    __syncthreads();
+    const u32 count = sh.count;
+    if (count == 0) return;
+    const bool staged = count <= SelectShared::kItems;
+    auto for_items = [&](auto g) {
+        if (staged) {
+            for (u32 j = threadIdx.x; j < count; j += kSelectThreads) g(sh.key[j], sh.v[j], sh.i[j]);
+        } else {
+            for (u32 j = threadIdx.x; j < total; j += kSelectThreads)
+                if (item_part[j] == p) { const CrossItem x = items[j]; g(x.key, x.v, x.i); }
+        }
+    };
+    u64 hi_key = 0, key_above = 0;   // the threshold's bits so far
+    u32 hi_v = 0, v_above = 0;
+    auto matches = [&](u64 key, u32 v) { return (key & key_above) == hi_key && (v & v_above) == hi_v; };
+    u32 matching = count;
+    if (matching > SelectShared::kFew) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            ka &= __shfl_xor_sync(0xffffffffu, ka, o);
+            ko |= __shfl_xor_sync(0xffffffffu, ko, o);
+            va &= __shfl_xor_sync(0xffffffffu, va, o);
+            vo |= __shfl_xor_sync(0xffffffffu, vo, o);
+        }
+        if (lane == 0) {
+            atomicAnd(reinterpret_cast<unsigned long long*>(&sh.key_and), static_cast<unsigned long long>(ka));
+            atomicOr(reinterpret_cast<unsigned long long*>(&sh.key_or), static_cast<unsigned long long>(ko));
+            atomicAnd(&sh.v_and, va);
+            atomicOr(&sh.v_or, vo);
+        }
+        __syncthreads();
+        // one step: the digit of the matching items at which the quota is crossed
+        auto step = [&](auto digit) {
+            if (threadIdx.x < 256) { sh.hist[threadIdx.x] = 0; sh.members[threadIdx.x] = 0; }
+            if (threadIdx.x == 0) sh.digit = 255;
+            __syncthreads();
+            for_items([&](u64 key, i32 v, i32) {
+                if (!matches(key, static_cast<u32>(v))) return;
+                const u32 dg = digit(key, static_cast<u32>(v));
+                atomicAdd(&sh.members[dg], 1u);
+                if (vw) atomic_add_u64(&sh.hist[dg], static_cast<u64>(vw[v]));
+            });
+            __syncthreads();
+            u64 w = 0;
+            if (threadIdx.x < 256) w = vw ? sh.hist[threadIdx.x] : static_cast<u64>(sh.members[threadIdx.x]);
+            const u64 before = select_exclusive_sum(w, sh.scan);
+            const u64 left = sh.left;
+            __syncthreads();
+            const bool crosses = SOURCES ? before < left && before + w >= left : before <= left && before + w > left;
+            if (crosses && threadIdx.x < 256) {
+                sh.digit = static_cast<int>(threadIdx.x);
+                sh.left = left - before;
             }
+            __syncthreads();
+            const u32 dg = static_cast<u32>(sh.digit);
+            matching = sh.members[dg];
+            __syncthreads();   // the counts may be cleared again
+            return dg;
+        };
+        u64 key_vary = sh.key_and ^ sh.key_or;
+        hi_key = sh.key_and;
+        key_above = ~key_vary;            // bits in which the items agree match from the start
+        while (key_vary && matching > SelectShared::kFew) {
+            const int top = 63 - __clzll(static_cast<long long>(key_vary));
+            const int shift = top > 7 ? top - 7 : 0;
+            const u64 field = 0xffULL >> (7 - (top - shift));
+            const u32 dg = step([&](u64 key, u32) { return static_cast<u32>((key >> shift) & field); });
+            key_above |= field << shift;
+            hi_key = (hi_key & ~(field << shift)) | (static_cast<u64>(dg) << shift);
+            key_vary &= ~(~0ULL << shift);
+        }
+        u32 v_vary = 0;
+        if (matching > SelectShared::kFew) {
+            v_vary = sh.v_and ^ sh.v_or;
+            hi_v = sh.v_and;
+            v_above = ~v_vary;
+        }
+        while (v_vary && matching > SelectShared::kFew) {
+            const int top = 31 - __clz(static_cast<int>(v_vary));
+            const int shift = top > 7 ? top - 7 : 0;
+            const u32 field = 0xffu >> (7 - (top - shift));
+            const u32 dg = step([&](u64, u32 v) { return (v >> shift) & field; });
+            v_above |= field << shift;
+            hi_v = (hi_v & ~(field << shift)) | (dg << shift);
+            v_vary &= ~(~0u << shift);
+        }
+    }
+    // rank the few that still match
+    for_items([&](u64 key, i32 v, i32) {
+        if (!matches(key, static_cast<u32>(v))) return;
+        const u32 at = atomicAdd(&sh.few, 1u);
+        if (at >= SelectShared::kFew) return;   // cannot happen: vertices differ
+        sh.few_key[at] = key;
+        sh.few_v[at] = static_cast<u32>(v);
+        sh.few_w[at] = static_cast<u64>(weight_at(vw, v));
+    });
+    __syncthreads();
+    {
+        const u32 few = min(sh.few, SelectShared::kFew), at = threadIdx.x >> 3;
+        u64 key = 0, before = 0;
+        u32 v = 0;
+        if (at < few) {
+            key = sh.few_key[at];
+            v = sh.few_v[at];
+            for (u32 j = threadIdx.x & 7; j < few; j += 8)
+                if (sh.few_key[j] < key || (sh.few_key[j] == key && sh.few_v[j] < v)) before += sh.few_w[j];
+        }
+        for (int o = 4; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+        const u64 left = sh.left;
+        const bool taken = at < few && (SOURCES ? before < left : before <= left && sh.few_w[at] <= left - before);
+        __syncthreads();
+        if (at < few && (threadIdx.x & 7) == 0) sh.few_w[at] = taken ? 1 : 0;   // the weights are used up
+    }
+    __syncthreads();
+    const u32 few = min(sh.few, SelectShared::kFew);
+    for_items([&](u64 key, i32 v, i32 i) {
+        const u32 uv = static_cast<u32>(v);
+        bool taken;
+        if (matches(key, uv)) {
+            taken = false;
+            for (u32 j = 0; j < few; ++j)
+                if (sh.few_v[j] == uv) { taken = sh.few_w[j] != 0; break; }
+        } else {
+            // above the threshold's bits: ahead of every matching item or behind them
+            const u64 a = key & key_above;
+            taken = a < hi_key || (a == hi_key && (uv & v_above) < hi_v);
+        }
+        f(i, v, taken);
+    });
+    __syncthreads();
+}
+
+// One block per part: the crossing bucket of every overloaded part's
+// excess; also clears the counters that the rest of the iteration adds to.
+__global__ void __launch_bounds__(kSelectThreads) cross_sources_kernel(const u64* __restrict__ pw, u64 cap, u64* counts,
+                                                                       CrossParts* cross, RefineCounters* ctr) {
+    __shared__ u64 shared[kSelectWarps];
+    const int p = blockIdx.x;
+    if (p == 0 && threadIdx.x == 0) { *ctr = RefineCounters{}; cross->count = 0; }
+    const u64 load = pw[p];
+    cross_bucket<true>(p, load > cap ? load - cap : 0, counts, cross, shared);
+}
+
+// Appends the lanes' crossing items.  All 32 lanes call it.
+template <typename C, typename W>
+__device__ __forceinline__ void append_crossing(bool take, i64 i, i64 v, int part, const C* cache, const i32* labels,
+                                                const i32* targets, const W* __restrict__ vw, int k,
+                                                CrossParts* cross, CrossItem* items, unsigned char* item_part) {
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    if (!m) return;
+    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+    u32 base = 0;
+    if (lane == leader) base = atomicAdd(&cross->count, static_cast<u32>(__popc(m)));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (!take) return;
+    const u32 at = base + __popc(m & lanemask_lt());
+    items[at] = {bucket_order(v, labels[v], targets[v], cache, vw, k), static_cast<i32>(i), static_cast<i32>(v)};
+    item_part[at] = static_cast<unsigned char>(part);
+}
+
+// balance_select_sources (src/refine_incremental.cuh:204-217): candidates in
+// buckets before their part's crossing bucket leave it and are counted in
+// their destination's buckets; those in it are listed for the selection.
+template <typename C, typename W>
+__global__ void select_sources_kernel(i64 n, const i64* count, const i32* __restrict__ list, i32* bucket,
+                                      const C* __restrict__ cache, const i32* __restrict__ labels,
+                                      const i32* __restrict__ targets, const W* __restrict__ vw, int k, u64* counts,
+                                      CrossParts* cross, CrossItem* items, unsigned char* item_part) {
+    __shared__ int crossing[32];
+    __shared__ BucketTable table;
+    n = list_length(n, count);
+    if (static_cast<i64>(blockIdx.x) * blockDim.x >= n) return;
+    if (static_cast<int>(threadIdx.x) < k) crossing[threadIdx.x] = cross->bucket[threadIdx.x];
+    table.clear();
+    __syncthreads();
+    for (i64 base = static_cast<i64>(blockIdx.x) * blockDim.x; base < n; base += static_cast<i64>(gridDim.x) * blockDim.x) {
+        const i64 i = base + threadIdx.x;
+        int d = -1, s = 0;
+        i64 v = 0;
+        bool listed = false;
+        const int b = i < n ? bucket[i] : -1;
+        if (b >= 0) {
+            s = b / kBalWidth;
+            const int lb = b - s * kBalWidth;
+            if (lb <= crossing[s]) {
+                v = list[i];
+                d = targets[v] * kBalWidth + lb;
+                listed = lb == crossing[s];
+            }
+            bucket[i] = d;
+        }
+        const bool now = d >= 0 && !listed;
+        table.add(now ? d : -1, now ? static_cast<u64>(weight_at(vw, v)) : 0, vw == nullptr, counts);
+        append_crossing(listed, i, v, s, cache, labels, targets, vw, k, cross, items, item_part);
+    }
+    __syncthreads();
+    table.flush(counts);
+}
+
+constexpr int kSelectCluster = 8;
+
+// One thread-block cluster between the two marking passes: the source
+// selections (a block per part in turn), then, once every taken item is
+// counted, the destinations' crossing buckets.  The cluster barrier stands
+// where two launches stood.
+template <typename W>
+__global__ void __cluster_dims__(kSelectCluster, 1, 1) __launch_bounds__(kSelectThreads) resolve_sources_kernel(
+    int k, const u64* __restrict__ pw, u64 cap, i32* bucket, const W* __restrict__ vw, u64* counts,
+    CrossParts* sources, CrossParts* dests, const CrossItem* items, const unsigned char* item_part) {
+    __shared__ SelectShared sh;
+    const int rank = static_cast<int>(blockIdx.x);
+    for (int p = rank; p < k; p += kSelectCluster)
+        resolve_bucket<true>(p, sources, items, item_part, vw, sh, [&](i32 i, i32 v, bool taken) {
+            if (taken) atomic_add_u64(&counts[bucket[i]], static_cast<u64>(weight_at(vw, v)));
+            else bucket[i] = -1;
+        });
+    cooperative_groups::this_cluster().sync();
+    if (rank == 0 && threadIdx.x == 0) dests->count = 0;
+    for (int p = rank; p < k; p += kSelectCluster) {
+        const u64 load = pw[p];
+        cross_bucket<false>(p, load < cap ? cap - load : 0, counts, dests, sh.scan);
+    }
+}
+
+// balance_select_destinations (src/refine_incremental.cuh:219-232): the
+// candidates left whose destination bucket lies before the crossing bucket
+// of the destination's slack move.
+template <typename C, typename W>
+__global__ void select_destinations_kernel(i64 n, const i64* count, const i32* __restrict__ list,
+                                           const i32* __restrict__ bucket, const C* __restrict__ cache,
+                                           const i32* __restrict__ labels, const i32* __restrict__ targets,
+                                           const W* __restrict__ vw, int k, CrossParts* cross, CrossItem* items,
+                                           unsigned char* item_part, unsigned char* flags, i32* movers,
+                                           RefineCounters* ctr) {
+    __shared__ int crossing[32];
+    n = list_length(n, count);
+    if (static_cast<i64>(blockIdx.x) * blockDim.x >= n) return;
+    if (static_cast<int>(threadIdx.x) < k) crossing[threadIdx.x] = cross->bucket[threadIdx.x];
+    __syncthreads();
+    for (i64 base = static_cast<i64>(blockIdx.x) * blockDim.x; base < n; base += static_cast<i64>(gridDim.x) * blockDim.x) {
+        const i64 i = base + threadIdx.x;
+        bool move = false, listed = false;
+        int p = 0;
+        i64 v = 0;
+        const int b = i < n ? bucket[i] : -1;
+        if (b >= 0) {
+            v = list[i];
+            p = b / kBalWidth;
+            const int lb = b - p * kBalWidth;
+            move = lb < crossing[p];
+            listed = lb == crossing[p];
         }
         const u64 slot = warp_append(move, reinterpret_cast<u64*>(&ctr->movers));
         if (move) {
             flags[v] = 1;
             movers[slot] = static_cast<i32>(v);
         }
+        append_crossing(listed, i, v, p, cache, labels, targets, vw, k, cross, items, item_part);
     }
 }
 
-// Deterministic ranks: candidates (bucket >= 0) compacted in vertex order,
-// sorted by (bucket asc, gain per weight desc); rank = weight prefix inside
-// the bucket; counts = bucket totals.
-struct HasBucket {
-    const i32* bucket;
-    const i32* list;   // candidate vertices (ascending), or null for all
-    __device__ i64 operator()(i64 i) const { return bucket[list ? list[i] : i] >= 0 ? 1 : 0; }
-};
-
-__global__ void compact_bucket_kernel(i64 n, const i32* cand, const i32* bucket, const i64* pos, i32* list) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const i64 v = cand ? cand[i] : i;
-    if (bucket[v] >= 0) list[pos[i]] = static_cast<i32>(v);
-}
-
-// Vertices of the parts above capacity: the only rebalance candidates, and a
-// superset of them for the whole rebalance (destinations never exceed the
-// capacity, so no part becomes overloaded and vertices only leave).
-struct InOverloaded {
-    const i32* labels;
-    const u64* pw;
-    u64 cap;
-    __device__ i64 operator()(i64 v) const { return pw[labels[v]] > cap ? 1 : 0; }
-};
-
-__global__ void compact_overloaded_kernel(i64 n, const i32* labels, const u64* pw, u64 cap, const i64* pos,
-                                          i32* list) {
-    const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (v < n && pw[labels[v]] > cap) list[pos[v]] = static_cast<i32>(v);
-}
-
-// mode 0: ~orderable(gpw) (desc); mode 1: bucket
-__global__ void rank_keys_kernel(i64 count, const i32* list, const double* gpw, const i32* bucket, int mode, u64* keys) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const i32 v = list[i];
-    if (mode == 0) {
-        double g = gpw[v];
-        if (g == 0.0) g = 0.0;
-        const u64 b = static_cast<u64>(__double_as_longlong(g));
-        const u64 ord = (b & 0x8000000000000000ULL) ? ~b : (b | 0x8000000000000000ULL);
-        keys[i] = ~ord;
-    } else {
-        keys[i] = static_cast<u64>(bucket[v]);
-    }
-}
-
+// One block per part: the movers of its destination crossing bucket.
 template <typename W>
-struct ListWeight {
-    const i32* list;
-    const W* vw;
-    __device__ u64 operator()(i64 i) const { return static_cast<u64>(weight_at(vw, list[i])); }
-};
-
-__global__ void bucket_heads_kernel(i64 count, const i32* list, const i32* bucket, const u64* excl, u64* bucket_base) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const int b = bucket[list[i]];
-    if (i == 0 || bucket[list[i - 1]] != b) bucket_base[b] = excl[i];
-}
-
-template <typename W>
-__global__ void bucket_ranks_kernel(i64 count, const i32* list, const i32* bucket, const u64* excl,
-                                    const u64* bucket_base, const W* vw, u64* rank, u64* counts) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const i32 v = list[i];
-    const int b = bucket[v];
-    rank[v] = excl[i] - bucket_base[b];
-    if (i + 1 == count || bucket[list[i + 1]] != b)
-        counts[b] = excl[i] + static_cast<u64>(weight_at(vw, v)) - bucket_base[b];
+__global__ void __launch_bounds__(kSelectThreads) resolve_destinations_kernel(
+    const W* __restrict__ vw, const CrossParts* cross, const CrossItem* items, const unsigned char* item_part,
+    unsigned char* flags, i32* movers, RefineCounters* ctr) {
+    __shared__ SelectShared sh;
+    resolve_bucket<false>(static_cast<int>(blockIdx.x), cross, items, item_part, vw, sh, [&](i32, i32 v, bool taken) {
+        if (!taken) return;
+        flags[v] = 1;
+        movers[atomic_add_u64(reinterpret_cast<u64*>(&ctr->movers), 1)] = v;
+    });
 }
 
 __global__ void project_kernel(i64 n, const i32* map, const i32* coarse, i32* fine) {

@@ -73,7 +73,8 @@ typedef struct gp_options {
     double imbalance;            /* >= 1.0, default 1.03 */
     uint32_t seed;
     int32_t verify;              /* strict checks, the reference's --verify */
-    int32_t deterministic;       /* (gain, vertex id) ranking inside rebalance buckets */
+    int32_t deterministic;       /* (gain, vertex id) ranking inside rebalance buckets; the default
+                                  mode promises no ranking (today it uses the same one) */
     int32_t pack_isolated;       /* default 1 */
     int32_t max_levels;          /* default 24 */
     int32_t max_rounds;          /* refinement phases per level, default 32 */
