@@ -96,6 +96,7 @@ struct Device {
     // loop condition: 0 never (host loop, same kernels; the default), 1 once
     // a level's host loop has run a few iterations, 2 always.
     int graph_loops = 0;
+    int wide_cluster = 0;       // largest cluster of one-block-per-SM kernels, 0: not asked yet
     size_t total_bytes = 0;     // device memory, read once when the context is created
     int grid_limit(int per_sm) const { return std::max(sms / 2, sms * per_sm / std::max(1, share)); }
     u32* err = nullptr;         // device error word
@@ -302,6 +303,64 @@ void launch(Device& d, const char* name, void (*k)(KArgs...), dim3 grid, dim3 bl
         e.pending.push_back({a, b});
         ++e.launches;
     }
+}
+
+// The same for a kernel launched as one thread-block cluster of `blocks` (a
+// power of two up to 8; up to 16 with the non-portable attribute set on it).
+template <typename... KArgs, typename... Args>
+void launch_cluster(Device& d, const char* name, void (*k)(KArgs...), int blocks, int threads, size_t smem,
+                    Args&&... args) {
+    static_assert(sizeof...(KArgs) == sizeof...(Args), "kernel argument count");
+    cudaEvent_t a = nullptr;
+    if (d.prof) {
+        a = d.event();
+        GP_CUDA(cudaEventRecord(a, d.stream));
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = d.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(blocks);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GP_CUDA(cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...));
+    ++d.launches;
+    if (d.prof) {
+        cudaEvent_t b = d.event();
+        GP_CUDA(cudaEventRecord(b, d.stream));
+        auto& e = d.prof_table[name];
+        e.pending.push_back({a, b});
+        ++e.launches;
+    }
+}
+
+// The largest cluster a kernel of one block per SM takes: 16 blocks (a
+// non-portable size, set on the kernel here) where the device can place one,
+// else 8.  The device is asked once per context.
+template <typename... KArgs>
+int wide_cluster_blocks(Device& d, void (*k)(KArgs...), int threads, size_t smem) {
+    GP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    if (d.wide_cluster == 0) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(16);
+        cfg.blockDim = dim3(static_cast<unsigned>(threads));
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 16;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int placeable = 0;
+        GP_CUDA(cudaOccupancyMaxActiveClusters(&placeable, k, &cfg));
+        d.wide_cluster = placeable > 0 ? 16 : 8;
+    }
+    return d.wide_cluster;
 }
 
 inline void Device::throw_oom(size_t bytes) {

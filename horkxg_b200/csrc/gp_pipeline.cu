@@ -27,6 +27,7 @@
 #include "gp_initial.cuh"
 #include "gp_refine.cuh"
 #include "gp_hub.cuh"
+#include "gp_refine_small.cuh"
 #include "gp_analyze.cuh"
 #include "gp_symmetrize.cuh"
 
@@ -112,7 +113,8 @@ template <typename T>
 const typename DGraph<T>::Hubs& hub_index(Device& d, const DGraph<T>& g, i64 known_count = -1) {
     auto& h = g.hubs;
     if (h.built) return h;
-    if (known_count == 0) {
+    // no row is longer than the vertex count when rows have no duplicates
+    if (known_count == 0 || (g.unique_rows == 1 && g.n <= kHubThreshold)) {
         h.count = h.chunks = 0;
         h.built = true;
         return h;
@@ -1128,7 +1130,6 @@ void launch_diffusion(Device& d, const DGraph<T>& g, int ntasks, const InitTask*
         cfg.gridDim = dim3(cs);
         cfg.blockDim = dim3(kSmallDiffThreads);
         cfg.dynamicSmemBytes = smem;
-        cfg.stream = d.stream;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = cs;
@@ -1141,19 +1142,8 @@ void launch_diffusion(Device& d, const DGraph<T>& g, int ntasks, const InitTask*
         int placeable = 0;
         GP_CUDA(cudaOccupancyMaxActiveClusters(&placeable, small, &cfg));
         if (placeable > 0) {
-            cudaEvent_t ev0 = nullptr;
-            if (d.prof) { ev0 = d.event(); GP_CUDA(cudaEventRecord(ev0, d.stream)); }
-            const O* off = g.off.get();
-            GP_CUDA(cudaLaunchKernelEx(&cfg, small, ntasks, tasks, task_of_pos, positions, order, labels, off,
-                                       g.nbr.get(), g.ewp(), seed, steps, x_out, key));
-            ++d.launches;
-            if (d.prof) {
-                cudaEvent_t ev1 = d.event();
-                GP_CUDA(cudaEventRecord(ev1, d.stream));
-                auto& e = d.prof_table["diffusion_small_kernel"];
-                e.pending.push_back({ev0, ev1});
-                ++e.launches;
-            }
+            launch_cluster(d, "diffusion_small_kernel", small, cs, kSmallDiffThreads, smem, ntasks, tasks, task_of_pos,
+                           positions, order, labels, g.off.get(), g.nbr.get(), g.ewp(), seed, steps, x_out, key);
             return;
         }
     }
@@ -1364,6 +1354,7 @@ struct RefineWork {
     Buf<CrossParts> cross;   // of the sources, of the destinations
     Buf<u64> counts, saved_pw, scratch;
     Buf<RefineCounters> ctr;
+    Buf<SmallRefineState> small;
     void ensure(Device& d, i64 n, int k, size_t cache_bytes) {
         const size_t s = static_cast<size_t>(n) + 1;
         cache_raw.ensure(d, cache_bytes);
@@ -1376,6 +1367,7 @@ struct RefineWork {
         saved_pw.ensure(d, 32);
         scratch.ensure(d, 8);
         ctr.ensure(d, 1);
+        small.ensure(d, 1);
     }
 };
 
@@ -1383,12 +1375,91 @@ struct RefineWork {
 // the cut of the coarser level's result), else kUnknownCut.
 constexpr u64 kUnknownCut = ~0ULL;
 
+// Levels refined by one cluster (refine_small_kernel): no hub rows (their
+// chunked kernels are not part of it) and at most this many vertices and
+// entries.  One cluster is 16 of the 148 SMs, so it wins while launches and
+// round trips, not bandwidth, are the time.  Measured with the line at 32 K,
+// 128 K, 256 K and 1 M vertices, ms per partition: RGG 150,000 k = 8 11.8,
+// 11.1, 11.0, 11.0; RGG 300,000 k = 32 15.0, 14.7, 14.7, 15.8; grid 700x701
+// k = 16 28.1, 25.7, 25.1, 29.8.
+constexpr i64 kSmallRefineN = 131072;
+constexpr i64 kSmallRefineM = 1 << 21;
+
+template <typename T>
+bool refine_is_small(Device& d, const DGraph<T>& g) {
+    if (g.n > kSmallRefineN || g.m > kSmallRefineM) return false;
+    return hub_index(d, g).count == 0;
+}
+
+template <typename T, typename C>
+gp_refine_stats refine_small(Device& d, const DGraph<T>& g, RefineWork& w, i32* labels, u64* pw,
+                             std::vector<u64>& host_pw, int k, u64 cap, int rounds, bool deterministic, u64 known_cut) {
+    using O = typename T::O;
+    using W = typename T::W;
+    static const BucketThresholdsHost thresholds;
+    w.ensure(d, g.n, k, static_cast<size_t>(g.n) * k * sizeof(C));
+    SmallRefineArgs<O, W, C> a{};
+    a.n = g.n; a.m = g.m;
+    a.off = g.off.get(); a.nbr = g.nbr.get(); a.ew = g.ewp(); a.vw = g.vwp();
+    a.labels = labels; a.pw = pw; a.k = k; a.cap = cap;
+    a.known_cut = known_cut;
+    a.max_rounds = rounds;
+    // The default mode's loops are driven by the host unless a device loop was
+    // asked for (gp_ctx_set_graph_loops): it takes control back every few LP
+    // rounds.
+    a.phases = deterministic || d.graph_loops ? std::max(rounds, 1) : 4;
+    a.fraction = static_cast<u64>(std::ldexp(0.999L, 64));
+    a.cache = reinterpret_cast<C*>(w.cache_raw.get());
+    a.targets = w.targets.get(); a.list = w.list.get(); a.movers = w.movers.get();
+    a.saved_labels = w.saved_labels.get(); a.cand = w.cand.get(); a.bucket = w.bucket.get();
+    a.gains = w.gains.get(); a.props = w.props.get();
+    a.locks = w.locks.get(); a.flags = w.flags.get(); a.item_part = w.item_part.get();
+    a.items = w.items.get(); a.cross = w.cross.get();
+    a.counts = w.counts.get(); a.saved_pw = w.saved_pw.get();
+    a.state = w.small.get();
+    w.small.zero(d);
+    // A block per 512 vertices and per 4096 entries, up to 16.  Measured with
+    // at most 1, 4, 8 and 16 blocks, ms of this kernel per partition: grid
+    // 64x64 2.1, 1.4, 1.3, 1.3; RGG 20,000 3.4, 1.8, 1.6, 1.5; weighted grid
+    // 256x256 11.1, 5.1, 4.2, 3.7; RGG 60,000 k = 32 21.4, 7.5, 5.1, 4.0 (16
+    // blocks at twice the load each: 1.5, 1.8, 4.1, 4.3).
+    auto kernel = refine_small_kernel<O, W, C>;
+    const int most = wide_cluster_blocks(d, kernel, kSmallThreads, 0);
+    int blocks = 1;
+    while (blocks < most && (blocks * kSmallThreads < g.n || static_cast<i64>(blocks) * 4096 < g.m)) blocks *= 2;
+    SmallRefineState s;
+    for (;;) {
+        launch_cluster(d, "refine_small_kernel", kernel, blocks, kSmallThreads, 0, a, thresholds.t);
+        fetch(d, &s, w.small.get(), 1);
+        if (s.error & kErrOddCut) fail(GP_ERUNTIME, "refinement cut is not symmetric");
+        if (s.error & kErrCutUnderflow) fail(GP_ERUNTIME, "incremental cut underflow");
+        if (s.done) break;
+        a.resume = 1;
+    }
+    gp_refine_stats r{};
+    r.rounds = s.rounds;
+    r.proposals = s.proposals;
+    r.accepted = s.accepted;
+    r.initial_cut = s.initial_cut;
+    r.admission_iterations = s.iterations;
+    r.admission_fallbacks = s.fallbacks;
+    if (s.final_directed & 1ULL) fail(GP_ERUNTIME, "refinement cut is not symmetric");
+    r.final_cut = s.final_directed / 2;
+    std::copy(s.pw, s.pw + k, host_pw.begin());
+    r.final_max_part_weight = *std::max_element(host_pw.begin(), host_pw.end());
+    if (r.final_cut != s.best_cut || r.final_cut > r.initial_cut || r.final_max_part_weight > cap)
+        fail(GP_ERUNTIME, "incremental refinement postcondition failed");
+    return r;
+}
+
 template <typename T, typename C>
 gp_refine_stats refine_level(Device& d, const DGraph<T>& g, RefineWork& w, i32* labels, u64* pw,
                              std::vector<u64>& host_pw, int k, u64 cap, int rounds, bool deterministic, bool verify,
                              u64 known_cut) {
     using O = typename T::O;
     using W = typename T::W;
+    if (!verify && !trace().on && refine_is_small(d, g))
+        return refine_small<T, C>(d, g, w, labels, pw, host_pw, k, cap, rounds, deterministic, known_cut);
     const i64 n = g.n;
     w.ensure(d, n, k, static_cast<size_t>(n) * k * sizeof(C));
     C* cache = reinterpret_cast<C*>(w.cache_raw.get());
@@ -1446,7 +1517,6 @@ gp_refine_stats refine_level(Device& d, const DGraph<T>& g, RefineWork& w, i32* 
     // maximum edge weight decides the LP filter (refine_incremental.cuh:332-333);
     // for weighted levels it stays on the device (w.scratch[7]) and the LP
     // kernel derives the filter from it
-    const double filter = 0.25;
     const u64* max_edge_weight = nullptr;
     if (ew) {
         GP_CUDA(cudaMemsetAsync(w.scratch.get() + 7, 0, sizeof(u64), d.stream));
@@ -1682,7 +1752,7 @@ gp_refine_stats refine_level(Device& d, const DGraph<T>& g, RefineWork& w, i32* 
         GP_CUDA(cudaMemsetAsync(ctr, 0, sizeof(RefineCounters), d.stream));
         d.prof_bytes("lp_proposals_kernel", static_cast<double>(n) * (k * sizeof(C) + 4 + 1 + 4 + 8));
         launch(d, "lp_proposals_kernel", lp_proposals_kernel<C>, blocks_for(n, kThreads), kThreads, 0, n, cache, labels, k,
-               filter, max_edge_weight, w.locks.get(), w.targets.get(), w.gains.get(), w.props.get(), w.list.get(), ctr);
+               max_edge_weight, w.locks.get(), w.targets.get(), w.gains.get(), w.props.get(), w.list.get(), ctr);
         if (d.prof) {
             // per proposer its list entry, offsets, record and flag; per edge
             // of a proposer below the hub degree its neighbour, weight and

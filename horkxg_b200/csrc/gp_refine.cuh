@@ -157,15 +157,16 @@ __device__ __forceinline__ void load_row(const C* row, int k, C (&vals)[32]) {
 // The four cache rows, consecutive in memory, are then stored by the whole
 // warp in one coalesced pass.  Hub rows are left to the chunked kernel
 // (zero_hub_rows_kernel clears them after this one).
+// `rows`: one accumulator per warp of the block.
 template <typename O, typename W, typename C>
-__global__ void __launch_bounds__(kThreads) build_cache_kernel(i64 n, const O* __restrict__ off,
-                                                               const i32* __restrict__ nbr, const W* __restrict__ ew,
-                                                               const i32* __restrict__ labels, int k, C* cache) {
-    __shared__ u64 rows[kWarps][4][32];
+__device__ __forceinline__ void build_cache_rows(i64 n, const O* __restrict__ off, const i32* __restrict__ nbr,
+                                                 const W* __restrict__ ew, const i32* labels, int k, C* cache,
+                                                 u64 (*rows)[4][32]) {
     u32 (*rows32)[4][32] = reinterpret_cast<u32 (*)[4][32]>(&rows[0][0][0]);   // C = u32: 32-bit accumulators
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane >> 3, gl = lane & 7;
-    const i64 warps_total = static_cast<i64>(gridDim.x) * kWarps;
-    for (i64 q = static_cast<i64>(blockIdx.x) * kWarps + warp; q * 4 < n; q += warps_total) {
+    const int block_warps = static_cast<int>(blockDim.x >> 5);
+    const i64 warps_total = static_cast<i64>(gridDim.x) * block_warps;
+    for (i64 q = static_cast<i64>(blockIdx.x) * block_warps + warp; q * 4 < n; q += warps_total) {
         const i64 v = q * 4 + grp;
         i64 b = 0, deg = 0;
         if (v < n) {
@@ -239,65 +240,79 @@ __global__ void __launch_bounds__(kThreads) build_cache_kernel(i64 n, const O* _
     }
 }
 
-// incremental_lp_proposals (src/refine_incremental.cuh:27-46); proposers
-// are appended to `list`.
+template <typename O, typename W, typename C>
+__global__ void __launch_bounds__(kThreads) build_cache_kernel(i64 n, const O* __restrict__ off,
+                                                               const i32* __restrict__ nbr, const W* __restrict__ ew,
+                                                               const i32* __restrict__ labels, int k, C* cache) {
+    __shared__ u64 rows[kWarps][4][32];
+    build_cache_rows(n, off, nbr, ew, labels, k, cache, rows);
+}
+
+// The LP filter of refine_incremental.cuh:332-333, from the level's maximum
+// edge weight (nullptr: unit weights).
+__device__ __forceinline__ double lp_filter(const u64* max_edge_weight) {
+    return !max_edge_weight || *max_edge_weight <= 1 ? 0.25 : 0.75;
+}
+
+// incremental_lp_proposals (src/refine_incremental.cuh:27-46) for one vertex;
+// true when it proposes.
+template <typename C>
+__device__ __forceinline__ bool lp_choice(i64 v, const C* cache, const i32* labels, int k, double filter,
+                                          unsigned char* locks, i32* targets, i64* gains, PropRec* props) {
+    i32 target = -1;
+    i64 g = INT64_MIN;
+    const i32 s = labels[v];
+    if (locks[v]) {
+        locks[v] = 0;
+    } else {
+        C vals[32];
+        load_row(cache + v * k, k, vals);
+        u64 best = 0, current = 0;
+        int t = -1;
+#pragma unroll
+        for (int p = 0; p < 32; ++p) {
+            if (p >= k) break;
+            const u64 c = static_cast<u64>(vals[p]);
+            if (p == s) current = c;
+            else if (c > best) { best = c; t = p; }
+        }
+        if (t >= 0 &&
+            (best >= current || current - best < static_cast<u64>(filter * static_cast<double>(current)))) {
+            g = best >= current ? static_cast<i64>(best - current) : -static_cast<i64>(current - best);
+            target = t;
+        }
+    }
+    targets[v] = target;
+    gains[v] = g;
+    props[v] = {s, target, g};
+    return target >= 0;
+}
+
+// Proposers are appended to `list`.
 template <typename C>
 __global__ void lp_proposals_kernel(i64 n, const C* __restrict__ cache, const i32* __restrict__ labels, int k,
-                                    double filter, const u64* __restrict__ max_edge_weight, unsigned char* locks,
-                                    i32* targets, i64* gains, PropRec* props, i32* list, RefineCounters* ctr) {
+                                    const u64* __restrict__ max_edge_weight, unsigned char* locks, i32* targets,
+                                    i64* gains, PropRec* props, i32* list, RefineCounters* ctr) {
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    // the filter of refine_incremental.cuh:332-333, from the level's maximum
-    // edge weight when it was computed on the device
-    if (max_edge_weight) filter = *max_edge_weight <= 1 ? 0.25 : 0.75;
-    bool propose = false;
-    if (v < n) {
-        i32 target = -1;
-        i64 g = INT64_MIN;
-        const i32 s = labels[v];
-        if (locks[v]) {
-            locks[v] = 0;
-        } else {
-            C vals[32];
-            load_row(cache + v * k, k, vals);
-            u64 best = 0, current = 0;
-            int t = -1;
-#pragma unroll
-            for (int p = 0; p < 32; ++p) {
-                if (p >= k) break;
-                const u64 c = static_cast<u64>(vals[p]);
-                if (p == s) current = c;
-                else if (c > best) { best = c; t = p; }
-            }
-            if (t >= 0 &&
-                (best >= current || current - best < static_cast<u64>(filter * static_cast<double>(current)))) {
-                g = best >= current ? static_cast<i64>(best - current) : -static_cast<i64>(current - best);
-                target = t;
-                propose = true;
-            }
-        }
-        targets[v] = target;
-        gains[v] = g;
-        props[v] = {s, target, g};
-    }
+    const bool propose = v < n && lp_choice(v, cache, labels, k, lp_filter(max_edge_weight), locks, targets, gains, props);
     const u64 slot = warp_append(propose, reinterpret_cast<u64*>(&ctr->proposers));
     if (propose) list[slot] = static_cast<i32>(v);
 }
 
 // incremental_priority_filter (src/refine_incremental.cuh:48-67); movers are
 // appended to `movers` and flagged.
+// A warp takes up to 32 proposers and walks their edges together; each
+// row's correction is summed in shared memory (hub rows: chunked kernel).
 template <typename O, typename W>
-__global__ void __launch_bounds__(kThreads) priority_filter_kernel(
-    const i32* __restrict__ list, const RefineCounters* ctr_in, const O* __restrict__ off,
-    const i32* __restrict__ nbr, const W* __restrict__ ew, const PropRec* __restrict__ props, unsigned char* flags,
-    i32* movers, RefineCounters* ctr) {
-    // A warp takes up to 32 proposers and walks their edges together; each
-    // row's correction is summed in shared memory (hub rows: chunked kernel).
-    __shared__ long long corr_sh[kWarps][32];
+__device__ __forceinline__ void priority_filter(const i32* list, i64 count, const O* __restrict__ off,
+                                                const i32* __restrict__ nbr, const W* __restrict__ ew,
+                                                const PropRec* props, unsigned char* flags, i32* movers,
+                                                RefineCounters* ctr, long long (*corr_sh)[32]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const i64 count = ctr_in->proposers;
-    const i64 warps = static_cast<i64>(gridDim.x) * kWarps;
+    const int block_warps = static_cast<int>(blockDim.x >> 5);
+    const i64 warps = static_cast<i64>(gridDim.x) * block_warps;
     const int G = rows_per_warp(count, warps);
-    for (i64 i0 = (static_cast<i64>(blockIdx.x) * kWarps + warp) * G; i0 < count; i0 += warps * G) {
+    for (i64 i0 = (static_cast<i64>(blockIdx.x) * block_warps + warp) * G; i0 < count; i0 += warps * G) {
         const i64 i = i0 + lane;
         const bool has = lane < G && i < count;
         const i32 v = has ? list[i] : 0;
@@ -340,6 +355,15 @@ __global__ void __launch_bounds__(kThreads) priority_filter_kernel(
                       static_cast<unsigned long long>(moved_degree));
         __syncwarp();
     }
+}
+
+template <typename O, typename W>
+__global__ void __launch_bounds__(kThreads) priority_filter_kernel(
+    const i32* __restrict__ list, const RefineCounters* ctr_in, const O* __restrict__ off,
+    const i32* __restrict__ nbr, const W* __restrict__ ew, const PropRec* __restrict__ props, unsigned char* flags,
+    i32* movers, RefineCounters* ctr) {
+    __shared__ long long corr_sh[kWarps][32];
+    priority_filter(list, ctr_in->proposers, off, nbr, ew, props, flags, movers, ctr, corr_sh);
 }
 
 // incremental_update_cache_and_cut (src/refine_incremental.cuh:69-95) for
@@ -403,8 +427,8 @@ __device__ __forceinline__ long long apply_edges_batched(i32 v, i32 s, i32 t, i6
 template <typename W, typename C>
 __device__ __forceinline__ long long warp_apply_rows(i32 v, i32 s, i32 t, i64 begin, i64 deg,
                                                      const i32* __restrict__ nbr, const W* __restrict__ ew,
-                                                     const i32* __restrict__ labels, const i32* __restrict__ targets,
-                                                     const unsigned char* __restrict__ flags, int k, C* cache) {
+                                                     const i32* labels, const i32* targets,
+                                                     const unsigned char* flags, int k, C* cache) {
     const int lane = threadIdx.x & 31;
     const i64 inc = warp_inclusive_sum(deg);
     const i64 pre = inc - deg;
@@ -526,12 +550,10 @@ __global__ void __launch_bounds__(kThreads) apply_big_rows_kernel(
 // warp share a part, so the changes are summed per warp and part, then per
 // block in shared memory, before one global atomic per block and part.
 template <typename W>
-__global__ void commit_kernel(const i32* __restrict__ movers, const RefineCounters* ctr_in,
-                              i32* labels, const i32* __restrict__ targets, const W* __restrict__ vw, u64* pw,
-                              unsigned char* locks, unsigned char* flags, int lp) {
-    __shared__ unsigned long long delta[32];
-    const i64 count = ctr_in->movers;
-    if (static_cast<i64>(blockIdx.x) * blockDim.x >= count) return;
+__device__ __forceinline__ void commit_moves(const i32* movers, i64 count, i32* labels, const i32* targets,
+                                             const W* __restrict__ vw, u64* pw, unsigned char* locks,
+                                             unsigned char* flags, bool lp, unsigned long long* delta) {
+    if (static_cast<i64>(blockIdx.x) * blockDim.x >= count) return;   // uniform over the block
     if (threadIdx.x < 32) delta[threadIdx.x] = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -556,6 +578,14 @@ __global__ void commit_kernel(const i32* __restrict__ movers, const RefineCounte
     }
     __syncthreads();
     if (threadIdx.x < 32 && delta[threadIdx.x]) atomic_add_u64(&pw[threadIdx.x], delta[threadIdx.x]);
+}
+
+template <typename W>
+__global__ void commit_kernel(const i32* __restrict__ movers, const RefineCounters* ctr_in,
+                              i32* labels, const i32* __restrict__ targets, const W* __restrict__ vw, u64* pw,
+                              unsigned char* locks, unsigned char* flags, int lp) {
+    __shared__ unsigned long long delta[32];
+    commit_moves(movers, ctr_in->movers, labels, targets, vw, pw, locks, flags, lp != 0, delta);
 }
 
 // Rebalance gain bucket (refine_incremental.cuh:167-171) restated with host
@@ -752,13 +782,10 @@ __global__ void __launch_bounds__(kThreads) collect_overloaded_kernel(i64 n, con
 // (balance_source_histogram, src/refine_incremental.cuh:167-186); part weights
 // are staged in shared memory.
 template <typename C, typename W>
-__global__ void rebalance_proposals_kernel(i64 n, const i64* count, const i32* __restrict__ list,
-                                           const C* __restrict__ cache, const i32* __restrict__ labels,
-                                           const W* __restrict__ vw, int k, const u64* __restrict__ pw, u64 cap,
-                                           BucketThresholds th, i32* targets, i32* bucket, u64* counts) {
-    __shared__ u64 spw[32];
-    __shared__ BucketTable table;
-    n = list_length(n, count);
+__device__ __forceinline__ void rebalance_proposals(i64 n, const i32* list, const C* cache, const i32* labels,
+                                                    const W* __restrict__ vw, int k, const u64* pw, u64 cap,
+                                                    const BucketThresholds& th, i32* targets, i32* bucket, u64* counts,
+                                                    u64* spw, BucketTable& table) {
     if (static_cast<i64>(blockIdx.x) * blockDim.x >= n) return;
     if (threadIdx.x < 32) spw[threadIdx.x] = static_cast<int>(threadIdx.x) < k ? pw[threadIdx.x] : ~0ULL;
     table.clear();
@@ -777,12 +804,22 @@ __global__ void rebalance_proposals_kernel(i64 n, const i64* count, const i32* _
     table.flush(counts);
 }
 
-constexpr int kSelectThreads = 1024;
-constexpr int kSelectWarps = kSelectThreads / 32;
-static_assert(kBalWidth <= kSelectThreads, "one thread per bucket of a part");
+template <typename C, typename W>
+__global__ void rebalance_proposals_kernel(i64 n, const i64* count, const i32* __restrict__ list,
+                                           const C* __restrict__ cache, const i32* __restrict__ labels,
+                                           const W* __restrict__ vw, int k, const u64* __restrict__ pw, u64 cap,
+                                           BucketThresholds th, i32* targets, i32* bucket, u64* counts) {
+    __shared__ u64 spw[32];
+    __shared__ BucketTable table;
+    rebalance_proposals(list_length(n, count), list, cache, labels, vw, k, pw, cap, th, targets, bucket, counts, spw,
+                        table);
+}
 
-// Exclusive block-wide sum over kSelectThreads threads; `shared` needs
-// kSelectWarps entries.
+constexpr int kSelectThreads = 1024;
+static_assert(kBalWidth <= 2 * 512, "at most two buckets of a part per thread of a 512-thread block");
+
+// Exclusive block-wide sum for blocks of 512 or 1024 threads; `shared` needs
+// 32 entries.
 __device__ __forceinline__ u64 select_exclusive_sum(u64 v, u64* shared) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const u64 inc = warp_inclusive_sum(v);
@@ -790,8 +827,9 @@ __device__ __forceinline__ u64 select_exclusive_sum(u64 v, u64* shared) {
     if (lane == 31) shared[warp] = inc;
     __syncthreads();
     if (warp == 0) {
-        const u64 s = shared[lane];
-        shared[lane] = warp_inclusive_sum(s) - s;
+        const u64 s = lane < static_cast<int>(blockDim.x >> 5) ? shared[lane] : 0;
+        const u64 si = warp_inclusive_sum(s);
+        shared[lane] = si - s;
     }
     __syncthreads();
     return shared[warp] + inc - v;
@@ -802,27 +840,37 @@ __device__ __forceinline__ u64 select_exclusive_sum(u64 v, u64* shared) {
 // src/refine_incremental.cuh:188-202).  The quota is used up before a bucket's
 // end: an item is taken while the weight before it is below the quota
 // (SOURCES), or while the weight up to its own end is within it
-// (!SOURCES).  A block of kSelectThreads.
+// (!SOURCES).  A block of 512 or 1024 threads.
 template <bool SOURCES>
 __device__ void cross_bucket(int p, u64 quota, u64* counts, CrossParts* cross, u64* shared) {
-    const int b = threadIdx.x;
-    u64 w = 0;
+    // two neighbouring buckets per thread
+    const int b = 2 * static_cast<int>(threadIdx.x);
+    u64 w[2] = {0, 0};
     if (b < kBalWidth) {
-        w = counts[p * kBalWidth + b];
-        counts[p * kBalWidth + b] = 0;
+        ulonglong2* c = reinterpret_cast<ulonglong2*>(counts + p * kBalWidth + b);
+        const ulonglong2 x = *c;
+        *c = make_ulonglong2(0, 0);
+        w[0] = x.x; w[1] = x.y;
     }
     if (b == 0) cross->bucket[p] = kBalWidth;
-    const u64 before = select_exclusive_sum(w, shared);
-    const bool crosses = SOURCES ? before < quota && before + w >= quota : before <= quota && before + w > quota;
-    if (crosses && b < kBalWidth) {
-        cross->bucket[p] = b;
-        cross->left[p] = quota - before;
+    u64 before = select_exclusive_sum(w[0] + w[1], shared);
+    if (b < kBalWidth) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const bool crosses = SOURCES ? before < quota && before + w[j] >= quota
+                                         : before <= quota && before + w[j] > quota;
+            if (crosses) {
+                cross->bucket[p] = b + j;
+                cross->left[p] = quota - before;
+            }
+            before += w[j];
+        }
     }
     __syncthreads();
 }
 
 struct SelectShared {
-    u64 scan[kSelectWarps];
+    u64 scan[32];
     u64 hist[256];
     u32 members[256];
     u64 key_and, key_or;
@@ -844,11 +892,11 @@ struct SelectShared {
 // (key, v), eight varying bits a step: the weights of the items that match it
 // so far are summed by digit, and the digit that crosses what is left of the
 // quota extends it.  Bits in which the items agree cost no step, and once at
-// most kFew items match they are ranked directly, eight lanes an item (a
+// most kFew items match they are ranked directly, 4 or 8 lanes an item (a
 // step costs a microsecond of barriers, so most lists finish after one or
 // two).  Lists of up to kItems items are staged in shared memory.
 // f(item index, v, taken) is called for every item of the part.  A block of
-// kSelectThreads.
+// 512 or 1024 threads.
 template <bool SOURCES, typename W, typename F>
 __device__ void resolve_bucket(int p, const CrossParts* cross, const CrossItem* items,
                                const unsigned char* item_part, const W* __restrict__ vw, SelectShared& sh, F f) {
@@ -863,7 +911,7 @@ __device__ void resolve_bucket(int p, const CrossParts* cross, const CrossItem* 
     __syncthreads();
     u64 ka = ~0ULL, ko = 0;
     u32 va = ~0u, vo = 0;
-    for (u32 j = threadIdx.x; j < total; j += kSelectThreads) {
+    for (u32 j = threadIdx.x; j < total; j += static_cast<u32>(blockDim.x)) {
         if (item_part[j] != p) continue;
         const CrossItem x = items[j];
         ka &= x.key; ko |= x.key;
@@ -877,9 +925,9 @@ __device__ void resolve_bucket(int p, const CrossParts* cross, const CrossItem* 
     const bool staged = count <= SelectShared::kItems;
     auto for_items = [&](auto g) {
         if (staged) {
-            for (u32 j = threadIdx.x; j < count; j += kSelectThreads) g(sh.key[j], sh.v[j], sh.i[j]);
+            for (u32 j = threadIdx.x; j < count; j += static_cast<u32>(blockDim.x)) g(sh.key[j], sh.v[j], sh.i[j]);
         } else {
-            for (u32 j = threadIdx.x; j < total; j += kSelectThreads)
+            for (u32 j = threadIdx.x; j < total; j += static_cast<u32>(blockDim.x))
                 if (item_part[j] == p) { const CrossItem x = items[j]; g(x.key, x.v, x.i); }
         }
     };
@@ -969,20 +1017,21 @@ __device__ void resolve_bucket(int p, const CrossParts* cross, const CrossItem* 
     });
     __syncthreads();
     {
-        const u32 few = min(sh.few, SelectShared::kFew), at = threadIdx.x >> 3;
+        const u32 few = min(sh.few, SelectShared::kFew), lanes = blockDim.x / SelectShared::kFew;
+        const u32 at = threadIdx.x / lanes;
         u64 key = 0, before = 0;
         u32 v = 0;
         if (at < few) {
             key = sh.few_key[at];
             v = sh.few_v[at];
-            for (u32 j = threadIdx.x & 7; j < few; j += 8)
+            for (u32 j = threadIdx.x % lanes; j < few; j += lanes)
                 if (sh.few_key[j] < key || (sh.few_key[j] == key && sh.few_v[j] < v)) before += sh.few_w[j];
         }
-        for (int o = 4; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+        for (int o = static_cast<int>(lanes) >> 1; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
         const u64 left = sh.left;
         const bool taken = at < few && (SOURCES ? before < left : before <= left && sh.few_w[at] <= left - before);
         __syncthreads();
-        if (at < few && (threadIdx.x & 7) == 0) sh.few_w[at] = taken ? 1 : 0;   // the weights are used up
+        if (at < few && threadIdx.x % lanes == 0) sh.few_w[at] = taken ? 1 : 0;   // the weights are used up
     }
     __syncthreads();
     const u32 few = min(sh.few, SelectShared::kFew);
@@ -1007,7 +1056,7 @@ __device__ void resolve_bucket(int p, const CrossParts* cross, const CrossItem* 
 // excess; also clears the counters that the rest of the iteration adds to.
 __global__ void __launch_bounds__(kSelectThreads) cross_sources_kernel(const u64* __restrict__ pw, u64 cap, u64* counts,
                                                                        CrossParts* cross, RefineCounters* ctr) {
-    __shared__ u64 shared[kSelectWarps];
+    __shared__ u64 shared[32];
     const int p = blockIdx.x;
     if (p == 0 && threadIdx.x == 0) { *ctr = RefineCounters{}; cross->count = 0; }
     const u64 load = pw[p];
@@ -1035,13 +1084,10 @@ __device__ __forceinline__ void append_crossing(bool take, i64 i, i64 v, int par
 // buckets before their part's crossing bucket leave it and are counted in
 // their destination's buckets; those in it are listed for the selection.
 template <typename C, typename W>
-__global__ void select_sources_kernel(i64 n, const i64* count, const i32* __restrict__ list, i32* bucket,
-                                      const C* __restrict__ cache, const i32* __restrict__ labels,
-                                      const i32* __restrict__ targets, const W* __restrict__ vw, int k, u64* counts,
-                                      CrossParts* cross, CrossItem* items, unsigned char* item_part) {
-    __shared__ int crossing[32];
-    __shared__ BucketTable table;
-    n = list_length(n, count);
+__device__ __forceinline__ void select_sources(i64 n, const i32* list, i32* bucket, const C* cache, const i32* labels,
+                                               const i32* targets, const W* __restrict__ vw, int k, u64* counts,
+                                               CrossParts* cross, CrossItem* items, unsigned char* item_part,
+                                               int* crossing, BucketTable& table) {
     if (static_cast<i64>(blockIdx.x) * blockDim.x >= n) return;
     if (static_cast<int>(threadIdx.x) < k) crossing[threadIdx.x] = cross->bucket[threadIdx.x];
     table.clear();
@@ -1068,6 +1114,17 @@ __global__ void select_sources_kernel(i64 n, const i64* count, const i32* __rest
     }
     __syncthreads();
     table.flush(counts);
+}
+
+template <typename C, typename W>
+__global__ void select_sources_kernel(i64 n, const i64* count, const i32* __restrict__ list, i32* bucket,
+                                      const C* __restrict__ cache, const i32* __restrict__ labels,
+                                      const i32* __restrict__ targets, const W* __restrict__ vw, int k, u64* counts,
+                                      CrossParts* cross, CrossItem* items, unsigned char* item_part) {
+    __shared__ int crossing[32];
+    __shared__ BucketTable table;
+    select_sources(list_length(n, count), list, bucket, cache, labels, targets, vw, k, counts, cross, items, item_part,
+                   crossing, table);
 }
 
 constexpr int kSelectCluster = 8;
@@ -1099,14 +1156,11 @@ __global__ void __cluster_dims__(kSelectCluster, 1, 1) __launch_bounds__(kSelect
 // candidates left whose destination bucket lies before the crossing bucket
 // of the destination's slack move.
 template <typename C, typename W>
-__global__ void select_destinations_kernel(i64 n, const i64* count, const i32* __restrict__ list,
-                                           const i32* __restrict__ bucket, const C* __restrict__ cache,
-                                           const i32* __restrict__ labels, const i32* __restrict__ targets,
-                                           const W* __restrict__ vw, int k, CrossParts* cross, CrossItem* items,
-                                           unsigned char* item_part, unsigned char* flags, i32* movers,
-                                           RefineCounters* ctr) {
-    __shared__ int crossing[32];
-    n = list_length(n, count);
+__device__ __forceinline__ void select_destinations(i64 n, const i32* list, const i32* bucket, const C* cache,
+                                                    const i32* labels, const i32* targets, const W* __restrict__ vw,
+                                                    int k, CrossParts* cross, CrossItem* items,
+                                                    unsigned char* item_part, unsigned char* flags, i32* movers,
+                                                    RefineCounters* ctr, int* crossing) {
     if (static_cast<i64>(blockIdx.x) * blockDim.x >= n) return;
     if (static_cast<int>(threadIdx.x) < k) crossing[threadIdx.x] = cross->bucket[threadIdx.x];
     __syncthreads();
@@ -1130,6 +1184,18 @@ __global__ void select_destinations_kernel(i64 n, const i64* count, const i32* _
         }
         append_crossing(listed, i, v, p, cache, labels, targets, vw, k, cross, items, item_part);
     }
+}
+
+template <typename C, typename W>
+__global__ void select_destinations_kernel(i64 n, const i64* count, const i32* __restrict__ list,
+                                           const i32* __restrict__ bucket, const C* __restrict__ cache,
+                                           const i32* __restrict__ labels, const i32* __restrict__ targets,
+                                           const W* __restrict__ vw, int k, CrossParts* cross, CrossItem* items,
+                                           unsigned char* item_part, unsigned char* flags, i32* movers,
+                                           RefineCounters* ctr) {
+    __shared__ int crossing[32];
+    select_destinations(list_length(n, count), list, bucket, cache, labels, targets, vw, k, cross, items, item_part,
+                        flags, movers, ctr, crossing);
 }
 
 // One block per part: the movers of its destination crossing bucket.

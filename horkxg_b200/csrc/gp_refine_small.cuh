@@ -1,0 +1,325 @@
+// The whole refinement of one small level (src/refine_incremental.cuh:235-361)
+// in one launch: a thread-block cluster builds the affinity cache and runs the
+// LP rounds and their rebalances, with the hardware cluster barrier where the
+// general path has a launch or a round trip to the host.
+//
+// On small levels the general path's time is launches and host waits (about
+// 9 launches and a wait per rebalance iteration, 7 and a wait per LP round);
+// the barrier costs a fraction of a launch.  The steps are the functions of
+// gp_refine.cuh, so both paths give the same labels; every decision of the
+// host loop is taken by all threads from the same counters.
+//
+// Mutable arrays are passed without __restrict__: blocks read what other
+// blocks wrote before the last barrier.
+#pragma once
+
+#include "gp_hub.cuh"
+#include "gp_refine.cuh"
+
+namespace gp {
+
+constexpr int kSmallThreads = 512;
+constexpr int kSmallWarps = kSmallThreads / 32;
+
+struct SmallRefineState {
+    i32 done;
+    i32 rounds, stale, empty, iterations, fallbacks;
+    u32 error;                    // DeviceError bits
+    u32 pass;                     // parity of the counters in use
+    u64 proposals, accepted, initial_cut, current_cut, best_cut;
+    u64 max_edge_weight;
+    u64 initial_directed, final_directed;
+    i64 candidates;
+    u64 pw[32];                   // part weights of the result
+    RefineCounters ctr[2];        // one in use, the other cleared for the next pass
+};
+
+template <typename O, typename W, typename C>
+struct SmallRefineArgs {
+    i64 n, m;
+    const O* off;
+    const i32* nbr;
+    const W* ew;
+    const W* vw;
+    i32* labels;
+    u64* pw;
+    int k;
+    u64 cap;
+    u64 known_cut;      // ~0: counted here
+    int max_rounds;
+    int phases;         // LP rounds of this launch
+    int resume;         // continue from the state
+    u64 fraction;       // 0.999L as a 64-bit fraction
+    C* cache;
+    i32 *targets, *list, *movers, *saved_labels, *cand, *bucket;
+    i64* gains;
+    PropRec* props;
+    unsigned char *locks, *flags, *item_part;
+    CrossItem* items;
+    CrossParts* cross;
+    u64 *counts, *saved_pw;
+    SmallRefineState* state;
+};
+
+union SmallRefineShared {
+    SelectShared select;
+    u64 rows[kSmallWarps][4][32];
+    long long corr[kSmallWarps][32];
+    struct { BucketTable table; u64 spw[32]; int crossing[32]; } rebalance;
+    unsigned long long delta[32];
+    u64 scan[32];
+};
+
+// current < RN64(fraction / 2^64 * best), RN64 rounding to 64 significant
+// bits: the host loop's long double comparison with 0.999L * best
+// (refine_incremental.cuh:350), which x87 arithmetic rounds that way.
+__host__ __device__ inline bool below_fraction(u64 current, u64 best, u64 fraction) {
+    unsigned __int128 p = static_cast<unsigned __int128>(fraction) * best;
+    const u64 high = static_cast<u64>(p >> 64);
+    if (high) {
+        int s = 0;   // bits below the 64 significant ones
+        for (u64 x = high; x; x >>= 1) ++s;
+        const unsigned __int128 unit = static_cast<unsigned __int128>(1) << s;
+        const unsigned __int128 rem = p & (unit - 1), half = unit >> 1;
+        p -= rem;
+        if (rem > half || (rem == half && (p & unit))) p += unit;
+    }
+    return (static_cast<unsigned __int128>(current) << 64) < p;
+}
+
+template <typename T>
+__device__ __forceinline__ T load_shared_state(const T* p) { return *reinterpret_cast<const volatile T*>(p); }
+
+// Exact directed cut of the rows of this launch's warps, added to *out.
+template <typename O, typename W>
+__device__ __forceinline__ void small_cut(i64 n, const O* __restrict__ off, const i32* __restrict__ nbr,
+                                          const W* __restrict__ ew, const i32* labels, u64* out) {
+    const int lane = threadIdx.x & 31, grp = lane >> 3, gl = lane & 7;
+    const i64 warps = static_cast<i64>(gridDim.x) * kSmallWarps;
+    u64 sum = 0;
+    for (i64 q = static_cast<i64>(blockIdx.x) * kSmallWarps + (threadIdx.x >> 5); q * 4 < n; q += warps) {
+        const i64 v = q * 4 + grp;
+        if (v >= n) continue;
+        const i32 s = labels[v];
+        for (i64 e = static_cast<i64>(off[v]) + gl; e < static_cast<i64>(off[v + 1]); e += 8)
+            if (labels[nbr[e]] != s) sum += static_cast<u64>(weight_at(ew, e));
+    }
+    sum = warp_sum(sum);
+    if (lane == 0 && sum) atomic_add_u64(out, sum);
+}
+
+template <typename O, typename W, typename C>
+__global__ void __launch_bounds__(kSmallThreads) refine_small_kernel(const SmallRefineArgs<O, W, C> a,
+                                                                     const BucketThresholds th) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ SmallRefineShared sh;
+    __shared__ u64 seen_max;
+    const int rank = static_cast<int>(blockIdx.x), blocks = static_cast<int>(gridDim.x);
+    const int lane = threadIdx.x & 31;
+    const i64 tid = static_cast<i64>(rank) * kSmallThreads + threadIdx.x;
+    const i64 threads = static_cast<i64>(blocks) * kSmallThreads;
+    const bool first = tid == 0;
+    const i64 n = a.n;
+    const int k = a.k;
+    SmallRefineState* st = a.state;
+    CrossParts* sources = a.cross;
+    CrossParts* dests = a.cross + 1;
+    const u64* max_edge_weight = a.ew ? &st->max_edge_weight : nullptr;
+
+    auto max_part = [&]() {   // of the current part weights, in every thread
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const u64 x = warp_max(lane < k ? load_shared_state(&a.pw[lane]) : u64{0});
+            if (lane == 0) seen_max = x;
+        }
+        __syncthreads();
+        return seen_max;
+    };
+    auto checkpoint = [&]() {
+        for (i64 v = tid; v < n; v += threads) a.saved_labels[v] = a.labels[v];
+        if (tid < k) a.saved_pw[tid] = load_shared_state(&a.pw[tid]);
+    };
+
+    u32 pass, error = 0;
+    int rounds, stale, empty, iterations, fallbacks;
+    u64 proposals, accepted, initial_cut, current, best;
+    if (!a.resume) {
+        for (i64 v = tid; v < n; v += threads) { a.locks[v] = 0; a.flags[v] = 0; }
+        for (i64 i = tid; i < static_cast<i64>(k) * kBalWidth; i += threads) a.counts[i] = 0;
+        build_cache_rows(n, a.off, a.nbr, a.ew, a.labels, k, a.cache, sh.rows);
+        if (a.ew) {
+            u64 mx = 0;
+            for (i64 e = tid; e < a.m; e += threads) {
+                const u64 x = static_cast<u64>(a.ew[e]);
+                mx = x > mx ? x : mx;
+            }
+            mx = warp_max(mx);
+            if (lane == 0 && mx) atomic_max_u64(&st->max_edge_weight, mx);
+        }
+        if (a.known_cut == ~0ULL) small_cut(n, a.off, a.nbr, a.ew, a.labels, &st->initial_directed);
+        checkpoint();
+        cluster.sync();
+        const u64 directed = load_shared_state(&st->initial_directed);
+        if (directed & 1ULL) error = kErrOddCut;
+        current = a.known_cut == ~0ULL ? directed / 2 : a.known_cut;
+        initial_cut = best = current;
+        pass = 0;
+        rounds = stale = empty = iterations = fallbacks = 0;
+        proposals = accepted = 0;
+    } else {
+        pass = st->pass;
+        rounds = st->rounds; stale = st->stale; empty = st->empty;
+        iterations = st->iterations; fallbacks = st->fallbacks;
+        proposals = st->proposals; accepted = st->accepted;
+        initial_cut = st->initial_cut; current = st->current_cut; best = st->best_cut;
+        cluster.sync();   // the state is read before block 0 writes it again
+    }
+
+    // Updates the cache along the movers' edges, then commits their labels;
+    // the movers' count and the cut change come back in every thread.
+    auto apply = [&](RefineCounters* ctr, i64 count, bool lp) {
+        const i64 warps = static_cast<i64>(blocks) * kSmallWarps;
+        const int G = rows_per_warp(count, warps);
+        long long gain = 0;
+        for (i64 i0 = (static_cast<i64>(rank) * kSmallWarps + (threadIdx.x >> 5)) * G; i0 < count; i0 += warps * G) {
+            const i64 i = i0 + lane;
+            const bool has = lane < G && i < count;
+            const i32 v = has ? a.movers[i] : 0;
+            const i64 b = has ? static_cast<i64>(a.off[v]) : 0;
+            const i64 deg = has ? static_cast<i64>(a.off[v + 1]) - b : 0;
+            const i32 s = has ? a.labels[v] : 0, t = has ? a.targets[v] : 0;
+            gain += warp_apply_rows(v, s, t, b, deg, a.nbr, a.ew, a.labels, a.targets, a.flags, k, a.cache);
+        }
+        gain = warp_sum(gain);
+        if (lane == 0 && gain)
+            atomicAdd(reinterpret_cast<unsigned long long*>(&ctr->delta), static_cast<unsigned long long>(gain));
+        cluster.sync();
+        commit_moves(a.movers, count, a.labels, a.targets, a.vw, a.pw, a.locks, a.flags, lp, sh.delta);
+        const long long delta = load_shared_state(&ctr->delta);
+        cluster.sync();
+        if (delta >= 0 && static_cast<u64>(delta) > current) error |= kErrCutUnderflow;
+        current -= static_cast<u64>(delta);   // modulo 2^64: a negative delta raises it
+        accepted += static_cast<u64>(count);
+    };
+
+    bool done = rounds >= a.max_rounds;
+    for (int budget = a.phases; !done && !error && budget > 0; --budget) {
+        ++rounds;
+        RefineCounters* ctr = &st->ctr[pass & 1];
+        const double filter = lp_filter(max_edge_weight);
+        for (i64 base = tid - lane; base < n; base += threads) {
+            const i64 v = base + lane;
+            const bool propose = v < n && lp_choice(v, a.cache, a.labels, k, filter, a.locks, a.targets, a.gains, a.props);
+            const u64 slot = warp_append(propose, reinterpret_cast<u64*>(&ctr->proposers));
+            if (propose) a.list[slot] = static_cast<i32>(v);
+        }
+        cluster.sync();
+        ++pass;
+        if (first) { st->ctr[pass & 1] = RefineCounters{}; st->candidates = 0; }
+        priority_filter(a.list, load_shared_state(&ctr->proposers), a.off, a.nbr, a.ew, a.props, a.flags, a.movers,
+                        ctr, sh.corr);
+        cluster.sync();
+        const i64 count = load_shared_state(&ctr->movers);
+        if (count == 0) {
+            if (++empty >= 2) { done = true; break; }
+            ++stale;
+            done = stale >= 3 || rounds >= a.max_rounds;
+            continue;
+        }
+        apply(ctr, count, true);
+        proposals += static_cast<u64>(count);
+        empty = 0;
+        // rebalance (refine_incremental.cuh:296-330)
+        bool balanced = max_part() <= a.cap;
+        if (!balanced) {
+            for (i64 base = tid - lane; base < n; base += threads) {
+                const i64 v = base + lane;
+                const bool take = v < n && load_shared_state(&a.pw[a.labels[v]]) > a.cap;
+                const u64 slot = warp_append(take, reinterpret_cast<u64*>(&st->candidates));
+                if (take) a.cand[slot] = static_cast<i32>(v);
+            }
+            cluster.sync();
+            const i64 ncand = load_shared_state(&st->candidates);
+            const int limit = 2 * k + 4;
+            for (int it = 0; it < limit && !balanced && !error; ++it) {
+                ++iterations;
+                ctr = &st->ctr[pass & 1];
+                rebalance_proposals(ncand, a.cand, a.cache, a.labels, a.vw, k, a.pw, a.cap, th, a.targets, a.bucket,
+                                    a.counts, sh.rebalance.spw, sh.rebalance.table);
+                cluster.sync();
+                ++pass;
+                if (first) { st->ctr[pass & 1] = RefineCounters{}; sources->count = 0; }
+                for (int p = rank; p < k; p += blocks) {
+                    const u64 load = load_shared_state(&a.pw[p]);
+                    cross_bucket<true>(p, load > a.cap ? load - a.cap : 0, a.counts, sources, sh.scan);
+                }
+                cluster.sync();
+                select_sources(ncand, a.cand, a.bucket, a.cache, a.labels, a.targets, a.vw, k, a.counts, sources,
+                               a.items, a.item_part, sh.rebalance.crossing, sh.rebalance.table);
+                cluster.sync();
+                for (int p = rank; p < k; p += blocks)
+                    resolve_bucket<true>(p, sources, a.items, a.item_part, a.vw, sh.select, [&](i32 i, i32 v, bool taken) {
+                        if (taken) atomic_add_u64(&a.counts[a.bucket[i]], static_cast<u64>(weight_at(a.vw, v)));
+                        else a.bucket[i] = -1;
+                    });
+                cluster.sync();
+                if (first) dests->count = 0;
+                for (int p = rank; p < k; p += blocks) {
+                    const u64 load = load_shared_state(&a.pw[p]);
+                    cross_bucket<false>(p, load < a.cap ? a.cap - load : 0, a.counts, dests, sh.scan);
+                }
+                cluster.sync();
+                select_destinations(ncand, a.cand, a.bucket, a.cache, a.labels, a.targets, a.vw, k, dests, a.items,
+                                    a.item_part, a.flags, a.movers, ctr, sh.rebalance.crossing);
+                cluster.sync();
+                for (int p = rank; p < k; p += blocks)
+                    resolve_bucket<false>(p, dests, a.items, a.item_part, a.vw, sh.select, [&](i32, i32 v, bool taken) {
+                        if (!taken) return;
+                        a.flags[v] = 1;
+                        a.movers[atomic_add_u64(reinterpret_cast<u64*>(&ctr->movers), 1)] = v;
+                    });
+                cluster.sync();
+                const i64 moved = load_shared_state(&ctr->movers);
+                if (moved == 0) break;
+                apply(ctr, moved, false);
+                balanced = max_part() <= a.cap;
+            }
+        }
+        if (!balanced) {
+            ++fallbacks;
+            done = true;
+            break;
+        }
+        ++stale;
+        if (current < best) {
+            if (below_fraction(current, best, a.fraction)) stale = 0;
+            best = current;
+            checkpoint();
+        }
+        done = stale >= 3 || rounds >= a.max_rounds;
+    }
+    if (done || error) {
+        // the best labels, recounted, once no block reads the part weights any more
+        cluster.sync();
+        for (i64 v = tid; v < n; v += threads) a.labels[v] = a.saved_labels[v];
+        if (tid < k) {
+            const u64 x = load_shared_state(&a.saved_pw[tid]);
+            a.pw[tid] = x;
+            st->pw[tid] = x;
+        }
+        cluster.sync();
+        small_cut(n, a.off, a.nbr, a.ew, a.labels, &st->final_directed);
+    }
+    if (first) {
+        st->done = done ? 1 : 0;
+        st->rounds = rounds; st->stale = stale; st->empty = empty;
+        st->iterations = iterations; st->fallbacks = fallbacks;
+        st->error = error;
+        st->pass = pass;
+        st->proposals = proposals; st->accepted = accepted;
+        st->initial_cut = initial_cut; st->current_cut = current; st->best_cut = best;
+    }
+}
+
+}  // namespace gp

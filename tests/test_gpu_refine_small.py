@@ -1,0 +1,73 @@
+"""The one-cluster refinement of small levels against the oracle, over the
+sizes at which its cluster grows and at which the general path takes over
+(131,072 vertices, 2^21 entries, a hub row), both widths and both cache
+widths, with and without weights."""
+import numpy as np
+import pytest
+
+import horkxg_b200 as hb
+import pyoracle as O
+from horkxg_b200 import graphs
+
+pytestmark = pytest.mark.gpu
+
+
+def inputs(n, k, weighted, scale, seed, degree=10.0):
+    off, nbr = graphs.rgg_csr(n, degree, seed)
+    rng = np.random.default_rng(seed)
+    ew = vw = None
+    if weighted:
+        src = np.repeat(np.arange(n), np.diff(off))
+        a, b = np.minimum(src, nbr), np.maximum(src, nbr)
+        ew = (((a * 2654435761 + b * 40503) % 97 + 1) * scale).astype(np.uint64)
+        vw = rng.integers(1, 4, n).astype(np.uint64)
+    # blocks of equal size in id order, one vertex in ten exchanged
+    labels = (np.arange(n) * k // n).astype(np.int32)
+    moved = rng.permutation(n)[:n // 10]
+    labels[moved] = labels[rng.permutation(moved)]
+    return off, nbr, ew, vw, labels
+
+
+def compare(ctx, off, nbr, ew, vw, labels, k, width, rounds=32, ratio=1.2):
+    g = hb.HostGraph(off, nbr, ew, vw, width=width)
+    lab, st = ctx.refine(g, labels, k, ratio, rounds, True)
+    olab, ost = O.refine(O.Graph(off, nbr, ew, vw), labels, k, ratio, rounds)
+    assert np.array_equal(lab, olab)
+    assert (st.rounds, st.initial_cut, st.final_cut) == (ost.rounds, ost.initial_cut, ost.final_cut)
+    assert (st.admission_iterations, st.final_max_part_weight) == (ost.admission_iterations, ost.final_max_part_weight)
+    return st
+
+
+@pytest.mark.parametrize("n,k", [(40, 2), (511, 4), (513, 32), (1025, 7), (4097, 8), (20000, 31), (131072, 8), (131073, 8)])
+def test_small_refine_matches_oracle(ctx, n, k):
+    compare(ctx, *inputs(n, k, False, 1, n), k, hb.STANDARD, ratio=1.03 if n > 10000 else 1.2)
+
+
+@pytest.mark.parametrize("width,scale", [(hb.STANDARD, 1), (hb.BIG, 1), (hb.BIG, 1 << 34)])
+@pytest.mark.parametrize("n,k", [(700, 3), (9000, 16)])
+def test_small_refine_weighted_widths(ctx, n, k, width, scale):
+    compare(ctx, *inputs(n, k, True, scale, n + k), k, width)
+
+
+@pytest.mark.parametrize("degree", [600.0, 1100.0])
+def test_small_refine_long_rows_and_entry_limit(ctx, degree):
+    """Rows of hundreds of entries, on either side of the entry limit."""
+    compare(ctx, *inputs(4000, 6, False, 1, 5, degree), 6, hb.STANDARD)
+
+
+@pytest.mark.parametrize("rounds", [0, 1, 3, 5])
+def test_small_refine_round_limits_and_modes(ctx, rounds):
+    """The default mode returns to the host every few rounds and continues."""
+    off, nbr, ew, vw, labels = inputs(3000, 8, True, 1, 12)
+    st = compare(ctx, off, nbr, ew, vw, labels, 8, hb.STANDARD, rounds)
+    g = hb.HostGraph(off, nbr, ew, vw)
+    a, _ = ctx.refine(g, labels, 8, 1.2, rounds, True)
+    b, sb = ctx.refine(g, labels, 8, 1.2, rounds, False)
+    assert np.array_equal(a, b) and (sb.rounds, sb.accepted) == (st.rounds, st.accepted)
+
+
+def test_small_refine_asymmetric_input(ctx):
+    off, nbr = np.array([0, 1, 1, 1, 1]), np.array([2])
+    with pytest.raises(hb.PartitionError) as e:
+        ctx.refine(hb.HostGraph(off, nbr), np.array([0, 0, 1, 1], np.int32), 2)
+    assert e.value.status == hb.GP_ERUNTIME and "symmetric" in str(e.value)
