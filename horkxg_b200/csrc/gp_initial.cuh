@@ -6,11 +6,10 @@
 //   one bounded grid barrier per step; the per-task weighted moments are
 //   reduced redundantly by every block in a fixed order (deterministic), and
 //   the normalisation is folded into the next step's reads;
-// * the split sort by (x, vertex id) is one launch: a block per task sorts its
-//   slice with an LSD radix sort on (orderable x << 32 | id);
-// * the weight-prefix split, its capacity checks and the child task
-//   descriptors are computed on the device (block per task): the host never
-//   waits inside the recursion.
+// * the split sort by (x, vertex id) -- keys (orderable x << 32 | id) -- the
+//   weight-prefix split, its capacity checks and the child task descriptors
+//   are computed on the device, one block per task: the host never waits
+//   inside the recursion.
 //
 // The diffusion is FP32 (the reference uses FP64); each diffusion vector is
 // checked against the FP64 oracle within 1e-5 relative L2.
@@ -33,7 +32,6 @@ struct InitTask {
 };
 
 struct Moments { float mass, sum, squares; };
-struct alignas(16) Moments4 { float mass, sum, squares, pad; };   // one 16-byte store
 
 // Bounded grid barrier for cooperative launches: gives up after ~2^24 polls
 // and records kErrTimeout (the kernel then finishes with garbage values that
@@ -52,7 +50,7 @@ __device__ __forceinline__ void grid_barrier(u32* counter, volatile u32* generat
             u32 polls = 0;
             while (*generation == gen) {
                 if (++polls > (1u << 24)) { set_error(err, kErrTimeout); break; }
-                __nanosleep(64);
+                if (polls > 256) __nanosleep(64);
             }
         }
         __threadfence();
@@ -247,185 +245,302 @@ __global__ void __launch_bounds__(kThreads) diffusion_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// Small coarsest graphs: the same diffusion in ONE thread-block cluster of up
-// to kSmallDiffCluster blocks (1024 threads each; at least one block per 1024
-// positions, so each thread owns at most one row, and one per
-// kSmallDiffBlockEdges edges, for dense graphs whose rows go to warps), every
-// per-vertex and
-// per-position array in shared memory and the hardware cluster barrier in
-// place of the grid barrier (no cooperative launch, no polling).  Each block
-// owns the positions p with p % cluster size == its rank.  The new values of
-// its rows are written into every block's shared memory (distributed shared
-// memory), their moment contributions into block 0's only; block 0 runs
-// compute_norms and sends the per-task mean and scale to the others.  It
-// computes exactly the values of diffusion_kernel, operation for operation:
-// * rows of more than 32 edges are summed by a warp with the same row_sum and
-//   warp_sum;
-// * rows of at most 32 edges are summed by one thread: in row_sum (stride 32)
-//   each lane then holds at most one edge, so the thread forms the 32 lane
-//   values and adds them in the butterfly order of warp_sum;
-// * the moments use compute_norms on the first kWarps warps.
-// Rows of more than kHeavyRow edges (block sums) are not taken: the host
-// sends such graphs to diffusion_kernel.
+// Coarsest graphs whose vectors fit shared memory (rows of at most kHeavyRow
+// entries): the same diffusion with every vector replicated in each block's
+// shared memory and one barrier a step.  A block copies its rows' new values
+// to every other block (a thread-block cluster: distributed shared memory,
+// 16 bytes a store, and the hardware barrier) or writes them to a global
+// vector that every block reads back (GRID: a cooperative grid, for graphs of
+// more edges than a cluster's SMs can walk);
+// after the barrier each block computes every task's moments, mean and scale
+// itself and normalises its copy, so no second exchange is needed.
+//
+// It computes exactly the values of diffusion_kernel, operation for operation:
+// * rows of at most 32 edges belong to eight lanes; lane j holds edges j,
+//   j + 8, j + 16, j + 24 in registers for all steps.  In row_sum each of
+//   32 lanes would hold one such edge, and warp_sum's butterfly adds lanes 16
+//   apart, then 8, 4, 2, 1: the first two levels are this lane's own adds,
+//   the others shuffles.  Edges that leave the group read a zero.
+// * longer rows are walked by a warp with row_sum and warp_sum;
+// * the moments are formed from the replicated values with the operations of
+//   diffusion_kernel's records and added in the order of compute_norms.
 // ---------------------------------------------------------------------------
-constexpr int kSmallDiffThreads = 1024;
-constexpr int kSmallDiffWarps = kSmallDiffThreads / 32;
-constexpr int kSmallDiffCluster = 16;      // largest cluster (a non-portable size above 8)
-constexpr i32 kSmallDiffN = 4096;          // positions (= vertices of the coarsest graph)
-constexpr i64 kSmallDiffBlockEdges = 131072;                         // edges per block and step
-constexpr i64 kSmallDiffM = kSmallDiffCluster * kSmallDiffBlockEdges;   // edges
-constexpr i32 kThreadRowMax = 32;          // rows summed by a single thread
+constexpr int kFastThreads = 1024;
+constexpr int kFastWarps = kFastThreads / 32;
+constexpr int kFastRows = 2;               // short rows per eight lanes
+constexpr i32 kFastRowMax = 32;            // edges of a short row
+constexpr i32 kFastBlockRows = kFastRows * kFastThreads / 8;
+constexpr i32 kFastN = 8192;               // positions of the GRID form
 
-// Lane 0's result of warp_sum over the 32 lane values lane(l), l = 0..31.
-template <typename L>
-__device__ __forceinline__ float butterfly_sum(L lane) {
-    float r[32];
-#pragma unroll
-    for (int l = 0; l < 32; ++l) r[l] = lane(l);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-#pragma unroll
-        for (int l = 0; l < o; ++l) r[l] = r[l] + r[l + o];
-    }
-    return r[0];
+inline size_t fast_diffusion_smem(i32 n, bool grid) {
+    // values by position (double-buffered where blocks write them), normalised
+    // values by vertex, degrees, order, labels, tasks
+    const size_t n4 = (static_cast<size_t>(n) + 3) / 4 * 4;
+    return n4 * ((grid ? 1 : 2) * sizeof(float) + 2 * sizeof(float) + 2 * sizeof(i32) + 1) + 64;
 }
 
-inline size_t small_diffusion_smem(i32 n) {
-    // moment records (per position; used in block 0), x, y, degree
-    // (vertex-indexed floats), labels, position records {vertex,
-    // degree << 8 | task} and the list of rows summed by warps
-    return static_cast<size_t>(n) * (sizeof(Moments4) + 3 * sizeof(float) + 4 * sizeof(i32));
-}
+struct FastShared {
+    float mean[kMaxInitTasks], scale[kMaxInitTasks];
+    i32 begin[kMaxInitTasks], count[kMaxInitTasks], group[kMaxInitTasks];
+    float red[kFastWarps / kWarps][3][kWarps];
+};
 
-template <typename O, typename W>
-__global__ void __launch_bounds__(kSmallDiffThreads) diffusion_small_kernel(
-    int tasks, const InitTask* __restrict__ task, const i32* __restrict__ task_of_pos, i32 positions,
-    const i32* __restrict__ order, const i32* __restrict__ labels_g, const O* __restrict__ off,
-    const i32* __restrict__ nbr, const W* __restrict__ ew, u32 seed, int steps, float* x_out, u64* key) {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank = static_cast<int>(cluster.block_rank());
-    const int cs = static_cast<int>(cluster.num_blocks());
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const i32 n = positions;
-    Moments4* contrib = reinterpret_cast<Moments4*>(smem_raw);
-    float* xa = reinterpret_cast<float*>(contrib + n);
-    float* xb = xa + n;
-    float* deg = xb + n;
-    i32* labels = reinterpret_cast<i32*>(deg + n);
-    i32* pv = labels + n;
-    i32* pdt = pv + n;
-    i32* heavy = pdt + n;
-    __shared__ NormShared sh;
-    __shared__ float norm_mean[kMaxInitTasks], norm_scale[kMaxInitTasks];
-    __shared__ int nheavy;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) nheavy = 0;
-    for (i32 v = threadIdx.x; v < n; v += kSmallDiffThreads) labels[v] = labels_g[v];
-    __syncthreads();
-    const i32 first = rank + cs * static_cast<i32>(threadIdx.x);
-    const i32 stride = cs * kSmallDiffThreads;
-    for (i32 p = first; p < n; p += stride) {
-        const i32 t = task_of_pos[p];
-        const i32 v = order[p];
-        const i32 dg = static_cast<i32>(off[v + 1] - off[v]);
-        pv[p] = v;
-        pdt[p] = t < 0 ? -1 : (dg << 8) | t;
-        if (t >= 0 && dg > kThreadRowMax) heavy[atomicAdd(&nheavy, 1)] = p;
-    }
-    cluster.sync();   // every block has started: its shared memory may be written
-    const int nh = nheavy;
-    Moments4* contrib0 = cluster.map_shared_rank(contrib, 0);
-    // a row's new value goes to every block, its moment record to block 0
-    auto put = [&](float* xlocal, i32 p, i32 v, float mass, float a) {
-        for (int r = 0; r < cs; ++r) cluster.map_shared_rank(xlocal, r)[v] = a;
-        contrib0[p] = Moments4{mass, mass * a, mass * a * a, 0.f};
-    };
-    auto start_row = [&](i32 p, float d) {
-        const i32 v = pv[p];
-        const i32 group = task[pdt[p] & 0xff].first_part;
-        const u32 h = mix32(static_cast<u32>(v) ^ (seed ^ static_cast<u32>(group)));
-        const float a = static_cast<float>(static_cast<double>(h) / 4294967296.0 - 0.5);
-        deg[v] = d;
-        put(xa, p, v, d > 0.f ? d : 1.f, a);
-    };
-    // row sum of f over the group, as diffusion_kernel forms it: lane l of
-    // row_sum holds edge l alone, a0 = 0 + w * f(u) if u is in the group,
-    // and returns (a0 + a1) + (a2 + a3) with a1 = a2 = a3 = 0
-    auto sum_thread = [&](i32 p, auto f) {
-        const i32 v = pv[p];
-        const i64 b = static_cast<i64>(off[v]);
-        const int dg = pdt[p] >> 8;
-        const i32 group = task[pdt[p] & 0xff].first_part;
-        return butterfly_sum([&](int l) {
-            float a0 = 0.f;
-            if (l < dg) {
-                const i32 u = nbr[b + l];
-                if (labels[u] == group) a0 += static_cast<float>(weight_at(ew, b + l)) * f(u);
+// compute_norms over replicated values: the same warps per task and the same
+// additions, with the rounds of tasks side by side on the block's other warps.
+__device__ __forceinline__ void fast_norms(int tasks, const float* x, const float* deg, FastShared& sh) {
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % kWarps, round = (threadIdx.x >> 5) / kWarps;
+    int wpt = kWarps;
+    while (wpt > 1 && tasks * wpt > kWarps) wpt >>= 1;
+    const int per_round = kWarps / wpt;
+    constexpr int kRounds = kFastWarps / kWarps;
+    for (int r = 0; r * per_round < tasks; r += kRounds) {
+        const int t0 = (r + round) * per_round;
+        const int t = t0 + warp / wpt;
+        const int part = warp % wpt;
+        float m = 0.f, s = 0.f, q = 0.f;
+        if (t < tasks) {
+            const i32 b = sh.begin[t], c = sh.count[t];
+            for (i32 i = part * 32 + lane; i < c; i += wpt * 32) {
+                const float d = deg[b + i], a = x[b + i];
+                const float w = d > 0.f ? d : 1.f;   // the mass
+                const float wa = __fmul_rn(w, a);
+                m += w; s += wa; q += __fmul_rn(wa, a);
             }
-            const float a1 = 0.f, a2 = 0.f, a3 = 0.f;
-            return (a0 + a1) + (a2 + a3);
-        });
-    };
-    auto sum_warp = [&](i32 p, auto f) {
-        const i32 v = pv[p];
-        const i64 b = static_cast<i64>(off[v]);
-        const i64 e = b + (pdt[p] >> 8);
-        const i32 group = task[pdt[p] & 0xff].first_part;
-        return warp_sum(row_sum<O, W>(b, e, lane, 32, nbr, labels, group, ew, f));
-    };
-    for (i32 p = first; p < n; p += stride)
-        if (pdt[p] >= 0 && (pdt[p] >> 8) <= kThreadRowMax) start_row(p, sum_thread(p, One{}));
-    for (int h = warp; h < nh; h += kSmallDiffWarps) {
-        const float d = sum_warp(heavy[h], One{});
-        if (lane == 0) start_row(heavy[h], d);
+#pragma unroll
+            for (int o = 16; o; o >>= 1) {
+                m += __shfl_xor_sync(0xffffffffu, m, o);
+                s += __shfl_xor_sync(0xffffffffu, s, o);
+                q += __shfl_xor_sync(0xffffffffu, q, o);
+            }
+        }
+        if (lane == 0) { sh.red[round][0][warp] = m; sh.red[round][1][warp] = s; sh.red[round][2][warp] = q; }
+        __syncthreads();
+        const int local = static_cast<int>(threadIdx.x) - round * kThreads;   // thread of this round's warps
+        if (local < per_round && t0 + local < tasks) {
+            float M = 0.f, S = 0.f, Q = 0.f;
+            for (int w = local * wpt; w < (local + 1) * wpt; ++w) {
+                M += sh.red[round][0][w]; S += sh.red[round][1][w]; Q += sh.red[round][2][w];
+            }
+            const float mean = S / M;
+            const float var = fmaxf(0.f, Q / M - mean * mean);
+            sh.mean[t0 + local] = mean;
+            sh.scale[t0 + local] = var > 1e-30f ? 1.0f / sqrtf(var) : 1.0f;
+        }
+        __syncthreads();
     }
+}
+
+// The normalised value of vertex u from a block's copy: weighted graphs store
+// it normalised; unit-weight graphs store it centred, because diffusion_kernel
+// adds (x - mean) * scale to a row's sum with one fused multiply-add in the
+// last, partial block of 128 edges of such a row (the multiplication by the
+// unit weight is folded away there), see unit_row_sum.
+struct Gathered {
+    const float* x;
+    float scale;
+    bool unit;
+    __device__ float operator()(i32 u) const { return unit ? __fmul_rn(x[u], scale) : x[u]; }
+};
+
+// row_sum of a unit-weight row for one warp over centred values.
+__device__ __forceinline__ float unit_row_sum(i64 begin, i64 end, int lane, const i32* __restrict__ nbr,
+                                              const i32* labels, i32 group, const float* x, float scale) {
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+    i64 e = begin + lane;
+    for (; e + 96 < end; e += 128) {
+        const i32 u0 = nbr[e], u1 = nbr[e + 32], u2 = nbr[e + 64], u3 = nbr[e + 96];
+        if (labels[u0] == group) a0 = __fadd_rn(a0, __fmul_rn(x[u0], scale));
+        if (labels[u1] == group) a1 = __fadd_rn(a1, __fmul_rn(x[u1], scale));
+        if (labels[u2] == group) a2 = __fadd_rn(a2, __fmul_rn(x[u2], scale));
+        if (labels[u3] == group) a3 = __fadd_rn(a3, __fmul_rn(x[u3], scale));
+    }
+    for (; e < end; e += 32) {
+        const i32 u = nbr[e];
+        if (labels[u] == group) a0 = fmaf(x[u], scale, a0);
+    }
+    return (a0 + a1) + (a2 + a3);
+}
+
+// exchange: GRID only, 3 n floats (two value vectors, the degrees).
+template <bool GRID, typename O, typename W>
+__global__ void __launch_bounds__(kFastThreads, 1) diffusion_fast_kernel(
+    int tasks, const InitTask* __restrict__ task, i32 n, const i32* __restrict__ order,
+    const i32* __restrict__ labels_g, const O* __restrict__ off, const i32* __restrict__ nbr,
+    const W* __restrict__ ew, u32 seed, int steps, float* exchange, float* x_out, u64* key, u32* bar_counter,
+    u32* bar_gen, u32* err) {
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ FastShared sh;
+    const int rank = static_cast<int>(blockIdx.x), blocks = static_cast<int>(gridDim.x);
+    const i32 n4 = (n + 3) / 4 * 4;
+    float* xa = reinterpret_cast<float*>(smem_raw);
+    float* xb = GRID ? xa : xa + n4;
+    float* deg = xb + n4;                                 // by position, inside the group
+    float* xn = deg + n4;                                 // by vertex; xn[n] = 0
+    i32* ord = reinterpret_cast<i32*>(xn + n4 + 4);
+    i32* lab = ord + n;
+    unsigned char* task_of = reinterpret_cast<unsigned char*>(lab + n);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = threadIdx.x & 7;
+    auto barrier = [&]() {
+        if constexpr (GRID) grid_barrier(bar_counter, bar_gen, err);
+        else cg::this_cluster().sync();
+    };
+    if (threadIdx.x < static_cast<unsigned>(tasks)) {
+        sh.begin[threadIdx.x] = task[threadIdx.x].begin;
+        sh.count[threadIdx.x] = task[threadIdx.x].count;
+        sh.group[threadIdx.x] = task[threadIdx.x].first_part;
+    }
+    if (threadIdx.x == 0) xn[n] = 0.f;
+    __syncthreads();
+    for (i32 p = threadIdx.x; p < n; p += kFastThreads) {
+        ord[p] = order[p];
+        lab[p] = labels_g[p];
+        int t = 0;
+        while (t < tasks && (p < sh.begin[t] || p >= sh.begin[t] + sh.count[t])) ++t;
+        task_of[p] = static_cast<unsigned char>(t < tasks ? t : 255);
+    }
+    if constexpr (GRID) __syncthreads();
+    else cg::this_cluster().sync();   // every block's shared memory may be written
+    // This block's rows: a contiguous chunk of a cluster block, every
+    // blocks-th position of a grid block (which spreads the long rows).
+    const i32 chunk = GRID ? 1 : ((n + blocks - 1) / blocks + 3) / 4 * 4;
+    const i32 lo = rank * chunk, hi = GRID ? n : min(n, lo + chunk), stride = GRID ? blocks : 1;
+    auto put = [&](float* local, float* global, i32 p, float a) {
+        if constexpr (GRID) global[p] = a;
+        else local[p] = a;
+    };
+    // the chunk's new values to the other blocks' copies
+    auto share = [&](float* local) {
+        if constexpr (!GRID) {
+            __syncthreads();
+            const int quads = (hi - lo + 3) / 4;
+            for (int r = 1 + warp; r < blocks; r += kFastWarps) {
+                const int to = (rank + r) % blocks;
+                float4* there = reinterpret_cast<float4*>(cg::this_cluster().map_shared_rank(local, to) + lo);
+                for (int q = lane; q < quads; q += 32) there[q] = reinterpret_cast<const float4*>(local + lo)[q];
+            }
+        }
+    };
+    // this thread's short rows
+    i32 row[kFastRows], edge[kFastRows][4];
+    float weight[kFastRows][4], degree[kFastRows];
+    int row_task[kFastRows];
+    auto short_sum = [&](int r, auto f) {
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = fmaf(weight[r][q], f(edge[r][q]), 0.f);
+        float s = (v[0] + v[2]) + (v[1] + v[3]);
+#pragma unroll
+        for (int o = 4; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return s;
+    };
+    auto start_value = [&](i32 p, int t) {
+        const u32 h = mix32(static_cast<u32>(ord[p]) ^ (seed ^ static_cast<u32>(sh.group[t])));
+        return static_cast<float>(static_cast<double>(h) / 4294967296.0 - 0.5);
+    };
+    float* xg[2] = {exchange, exchange + n};
+    float* deg_g = exchange + 2 * static_cast<i64>(n);
+#pragma unroll
+    for (int r = 0; r < kFastRows; ++r) {
+        const i32 p = lo + stride * (static_cast<i32>(threadIdx.x >> 3) + r * (kFastThreads / 8));
+        row[r] = -1;
+        row_task[r] = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) { edge[r][q] = n; weight[r][q] = 0.f; }
+        if (p < hi && task_of[p] != 255) {
+            const i32 v = ord[p];
+            const i64 b = off[v];
+            const i64 dg = static_cast<i64>(off[v + 1]) - b;
+            if (dg <= kFastRowMax) {
+                row[r] = p;
+                row_task[r] = task_of[p];
+                const i32 group = sh.group[row_task[r]];
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (sub + 8 * q < dg) {
+                        const i64 e = b + sub + 8 * q;
+                        const i32 u = nbr[e];
+                        if (lab[u] == group) { edge[r][q] = u; weight[r][q] = static_cast<float>(weight_at(ew, e)); }
+                    }
+            }
+        }
+        degree[r] = short_sum(r, One{});
+        if (row[r] >= 0 && sub == 0) {
+            put(deg, deg_g, row[r], degree[r]);
+            put(xa, xg[0], row[r], start_value(row[r], row_task[r]));
+        }
+    }
+    // long rows, a warp each
+    auto long_rows = [&](auto f) {
+        for (i32 p = lo + stride * warp; p < hi; p += stride * kFastWarps) {
+            const int t = task_of[p];
+            if (t == 255) continue;
+            const i32 v = ord[p];
+            const i64 b = off[v], e = off[v + 1];
+            if (e - b > kFastRowMax) f(p, t, b, e);
+        }
+    };
+    long_rows([&](i32 p, int t, i64 b, i64 e) {
+        const float d = warp_sum(row_sum<O, W>(b, e, lane, 32, nbr, lab, sh.group[t], ew, One{}));
+        if (lane == 0) {
+            put(deg, deg_g, p, d);
+            put(xa, xg[0], p, start_value(p, t));
+        }
+    });
+    share(deg);
+    share(xa);
     float* x = xa;
     float* y = xb;
+    int cur = 0;
     for (int it = 0; it <= steps; ++it) {
-        cluster.sync();                       // all records of the step are in block 0
-        if (rank == 0) {
-            compute_norms(tasks, task, contrib, sh);
-            if (threadIdx.x < static_cast<unsigned>(tasks))
-                for (int r = 0; r < cs; ++r) {
-                    cluster.map_shared_rank(norm_mean, r)[threadIdx.x] = sh.mean[threadIdx.x];
-                    cluster.map_shared_rank(norm_scale, r)[threadIdx.x] = sh.scale[threadIdx.x];
+        barrier();
+        if constexpr (GRID) {
+            for (i32 p = threadIdx.x; p < n; p += kFastThreads)
+                if (task_of[p] != 255) {
+                    x[p] = __ldcg(&xg[cur][p]);
+                    if (it == 0) deg[p] = __ldcg(&deg_g[p]);
                 }
+            __syncthreads();
         }
-        cluster.sync();                       // mean and scale are everywhere
+        fast_norms(tasks, x, deg, sh);
         if (it == steps) break;
-        auto step_row = [&](i32 p, float s) {
-            const i32 v = pv[p];
-            const int t = pdt[p] & 0xff;
-            const float d = deg[v];
-            const float xv = (x[v] - norm_mean[t]) * norm_scale[t];
-            const float a = d > 0.f ? 0.5f * (xv + s / d) : xv;
-            put(y, p, v, d > 0.f ? d : 1.f, a);
+        for (i32 p = threadIdx.x; p < n; p += kFastThreads) {
+            const int t = task_of[p];
+            if (t == 255) continue;
+            const float centred = x[p] - sh.mean[t];
+            xn[ord[p]] = ew ? centred * sh.scale[t] : centred;
+        }
+        __syncthreads();
+        auto step_value = [&](i32 p, int t, float d, float s) {
+            const float xv = (x[p] - sh.mean[t]) * sh.scale[t];
+            return d > 0.f ? 0.5f * (xv + s / d) : xv;
         };
-        for (i32 p = first; p < n; p += stride) {
-            if (pdt[p] < 0 || (pdt[p] >> 8) > kThreadRowMax) continue;
-            const int t = pdt[p] & 0xff;
-            step_row(p, sum_thread(p, Normalised{x, norm_mean[t], norm_scale[t]}));
+#pragma unroll
+        for (int r = 0; r < kFastRows; ++r) {
+            const float s = short_sum(r, Gathered{xn, sh.scale[row_task[r]], ew == nullptr});
+            if (row[r] >= 0 && sub == 0) put(y, xg[cur ^ 1], row[r], step_value(row[r], row_task[r], degree[r], s));
         }
-        for (int h = warp; h < nh; h += kSmallDiffWarps) {
-            const i32 p = heavy[h];
-            const int t = pdt[p] & 0xff;
-            const float s = sum_warp(p, Normalised{x, norm_mean[t], norm_scale[t]});
-            if (lane == 0) step_row(p, s);
-        }
+        long_rows([&](i32 p, int t, i64 b, i64 e) {
+            const float s = warp_sum(ew ? row_sum<O, W>(b, e, lane, 32, nbr, lab, sh.group[t], ew,
+                                                        Gathered{xn, 1.f, false})
+                                        : unit_row_sum(b, e, lane, nbr, lab, sh.group[t], xn, sh.scale[t]));
+            if (lane == 0) put(y, xg[cur ^ 1], p, step_value(p, t, deg[p], s));
+        });
+        share(y);
         float* tmp = x; x = y; y = tmp;
+        cur ^= 1;
     }
-    // no shared memory of another block is touched after the last cluster.sync
-    for (i32 p = first; p < n; p += stride) {
-        if (pdt[p] < 0) continue;
-        const int t = pdt[p] & 0xff;
-        const i32 v = pv[p];
-        float a = (x[v] - norm_mean[t]) * norm_scale[t];
+    // no shared memory of another block is touched after the last barrier
+    for (i32 p = rank * kFastThreads + threadIdx.x; p < n; p += blocks * kFastThreads) {
+        const int t = task_of[p];
+        if (t == 255) continue;
+        const i32 v = ord[p];
+        float a = (x[p] - sh.mean[t]) * sh.scale[t];
         if (a == 0.f) a = 0.f;
         if (x_out) x_out[v] = a;
         const u32 bits = __float_as_uint(a);
-        const u32 ord = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
-        key[p] = (static_cast<u64>(ord) << 32) | static_cast<u32>(v);
+        const u32 o = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
+        key[p] = (static_cast<u64>(o) << 32) | static_cast<u32>(v);
     }
 }
 
@@ -463,14 +578,52 @@ __device__ __forceinline__ u64 mul_div_floor(u64 w, u64 num, u64 den) {
     return static_cast<u64>(p / den);
 }
 
-// Weight-prefix split, src/initial_partition_gpu.cu:231-254, block per task.
+// The boundary of one task's split from its inclusive weight prefix
+// (src/initial_partition_gpu.cu:231-254), by one thread; writes the child
+// tasks.
+__device__ inline int split_boundary(const InitTask& tk, InitTask* next, const u64* prefix, u64 capacity, u32* err) {
+    const i32 b = tk.begin, c = tk.count;
+    const int left_parts = tk.parts / 2, right_parts = tk.parts - left_parts;
+    const u64 W_ = tk.weight;
+    const u64 target = mul_div_floor(W_, static_cast<u64>(left_parts), static_cast<u64>(tk.parts));
+    const u64 left_limit = capacity > W_ / left_parts ? W_ : capacity * left_parts;
+    const u64 right_limit = capacity > W_ / right_parts ? W_ : capacity * right_parts;
+    const u64 min_left = W_ > right_limit ? W_ - right_limit : 0;
+    // lower_bound over the inclusive prefix
+    i32 lo = 0, hi = c;
+    while (lo < hi) {
+        const i32 mid = lo + (hi - lo) / 2;
+        if (prefix[mid] < target) lo = mid + 1; else hi = mid;
+    }
+    int boundary = lo + 1;
+    boundary = max(left_parts, min(c - right_parts, boundary));
+    u64 lw = prefix[boundary - 1];
+    if (lw > left_limit && boundary > left_parts) { --boundary; lw = prefix[boundary - 1]; }
+    if (lw < min_left && boundary < c - right_parts) { ++boundary; lw = prefix[boundary - 1]; }
+    if (lw > left_limit || lw < min_left) set_error(err, kErrSplit);
+    const u64 rw = W_ - lw;
+    if (tk.left_child >= 0) {
+        InitTask& L = next[tk.left_child];
+        L.begin = b; L.count = boundary; L.weight = lw;
+    } else if (lw > capacity) {
+        set_error(err, kErrBalance);
+    }
+    if (tk.right_child >= 0) {
+        InitTask& R = next[tk.right_child];
+        R.begin = b + boundary; R.count = c - boundary; R.weight = rw;
+    } else if (rw > capacity) {
+        set_error(err, kErrBalance);
+    }
+    return boundary;
+}
+
+// Weight-prefix split, block per task.
 template <typename W>
 __global__ void __launch_bounds__(kThreads) task_split_kernel(int tasks, const InitTask* task, InitTask* next,
                                                               const i32* order, const W* vw, u64 capacity,
                                                               u64* prefix, i32* labels, u32* err) {
     __shared__ i64 scan_sh[kWarps + 1];
     __shared__ int boundary_sh;
-    __shared__ u64 left_weight_sh;
     const int t = blockIdx.x;
     if (t >= tasks) return;
     const InitTask tk = task[t];
@@ -485,46 +638,116 @@ __global__ void __launch_bounds__(kThreads) task_split_kernel(int tasks, const I
         carry += static_cast<u64>(total);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const int left_parts = tk.parts / 2, right_parts = tk.parts - left_parts;
-        const u64 W_ = tk.weight;
-        const u64 target = mul_div_floor(W_, static_cast<u64>(left_parts), static_cast<u64>(tk.parts));
-        const u64 left_limit = capacity > W_ / left_parts ? W_ : capacity * left_parts;
-        const u64 right_limit = capacity > W_ / right_parts ? W_ : capacity * right_parts;
-        const u64 min_left = W_ > right_limit ? W_ - right_limit : 0;
-        // lower_bound over the inclusive prefix
-        i32 lo = 0, hi = c;
-        while (lo < hi) {
-            const i32 mid = lo + (hi - lo) / 2;
-            if (prefix[b + mid] < target) lo = mid + 1; else hi = mid;
-        }
-        int boundary = lo + 1;
-        boundary = max(left_parts, min(c - right_parts, boundary));
-        u64 lw = prefix[b + boundary - 1];
-        if (lw > left_limit && boundary > left_parts) { --boundary; lw = prefix[b + boundary - 1]; }
-        if (lw < min_left && boundary < c - right_parts) { ++boundary; lw = prefix[b + boundary - 1]; }
-        if (lw > left_limit || lw < min_left) set_error(err, kErrSplit);
-        boundary_sh = boundary;
-        left_weight_sh = lw;
-        const u64 rw = W_ - lw;
-        if (tk.left_child >= 0) {
-            InitTask& L = next[tk.left_child];
-            L.begin = b; L.count = boundary; L.weight = lw;
-        } else if (lw > capacity) {
-            set_error(err, kErrBalance);
-        }
-        if (tk.right_child >= 0) {
-            InitTask& R = next[tk.right_child];
-            R.begin = b + boundary; R.count = c - boundary; R.weight = rw;
-        } else if (rw > capacity) {
-            set_error(err, kErrBalance);
-        }
-    }
+    if (threadIdx.x == 0) boundary_sh = split_boundary(tk, next, prefix + b, capacity, err);
     __syncthreads();
     const int boundary = boundary_sh;
     const int left_parts = tk.parts / 2;
     for (i32 i = threadIdx.x; i < c; i += kThreads)
         labels[order[b + i]] = i < boundary ? tk.first_part : tk.first_part + left_parts;
+}
+
+// Sort and split of tasks of at most kOrderN positions in one launch, block
+// per task: a bitonic sort of the (value, id) keys in shared memory -- the keys
+// differ, so any sort gives the one order -- with the steps of stride below 32
+// in registers, then the weight prefix in the keys' place.  Bound by its ~40
+// barriers; the radix sort and split kernels take 8 passes of 4 barriers.
+constexpr i32 kOrderN = 4096;
+constexpr int kOrderThreads = 1024;
+constexpr int kOrderItems = kOrderN / kOrderThreads;
+
+template <typename W>
+__global__ void __launch_bounds__(kOrderThreads) task_order_kernel(int tasks, const InitTask* task, InitTask* next,
+                                                                   const u64* key, i32* order, const W* vw,
+                                                                   u64 capacity, i32* labels, u32* err) {
+    __shared__ u64 k[kOrderN];
+    __shared__ u64 scan[kOrderThreads / 32];
+    __shared__ int boundary_sh;
+    const int tid = static_cast<int>(threadIdx.x), lane = tid & 31, warp = tid >> 5;
+    const InitTask tk = task[blockIdx.x];
+    const i32 b = tk.begin, c = tk.count;
+    int size2 = 32;
+    while (size2 < c) size2 <<= 1;
+    const int items = (size2 + kOrderThreads - 1) / kOrderThreads;   // per thread, at tid + j * kOrderThreads
+    u64 v[kOrderItems];
+#pragma unroll
+    for (int j = 0; j < kOrderItems; ++j) {
+        const int i = tid + j * kOrderThreads;
+        v[j] = i < c ? key[b + i] : ~0ULL;
+    }
+    // the strides below 32 of one merge size, between lanes
+    auto lanes = [&](int size) {
+#pragma unroll
+        for (int stride = 16; stride; stride >>= 1) {
+            if (stride >= size) continue;
+#pragma unroll
+            for (int j = 0; j < kOrderItems; ++j) {
+                if (j >= items) break;
+                const u64 o = __shfl_xor_sync(0xffffffffu, v[j], stride);
+                const bool up = ((tid + j * kOrderThreads) & size) == 0, lower = (lane & stride) == 0;
+                if ((lower == up) ? o < v[j] : o > v[j]) v[j] = o;
+            }
+        }
+    };
+    for (int size = 2; size <= 32; size <<= 1) lanes(size);
+    for (int size = 64; size <= size2; size <<= 1) {
+#pragma unroll
+        for (int j = 0; j < kOrderItems; ++j)
+            if (tid + j * kOrderThreads < size2) k[tid + j * kOrderThreads] = v[j];
+        __syncthreads();
+        for (int stride = size >> 1; stride >= 32; stride >>= 1) {
+            for (int q = tid; q < size2 >> 1; q += kOrderThreads) {
+                const int i = 2 * q - (q & (stride - 1));
+                const u64 x = k[i], y = k[i + stride];
+                if ((x > y) == ((i & size) == 0)) { k[i] = y; k[i + stride] = x; }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int j = 0; j < kOrderItems; ++j)
+            if (tid + j * kOrderThreads < size2) v[j] = k[tid + j * kOrderThreads];
+        lanes(size);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < kOrderItems; ++j)
+        if (tid + j * kOrderThreads < size2) k[tid + j * kOrderThreads] = v[j];
+    __syncthreads();
+    // neighbouring positions per thread for the prefix
+    i32 id[kOrderItems];
+    u64 w[kOrderItems], sum = 0;
+#pragma unroll
+    for (int j = 0; j < kOrderItems; ++j) {
+        const int i = tid * items + j;
+        id[j] = -1;
+        w[j] = 0;
+        if (j < items && i < c) {
+            id[j] = static_cast<i32>(k[i] & 0xffffffffu);
+            w[j] = static_cast<u64>(weight_at(vw, id[j]));
+            order[b + i] = id[j];
+        }
+        sum += w[j];
+    }
+    const u64 inc = warp_inclusive_sum(sum);
+    if (lane == 31) scan[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        const u64 x = scan[lane];
+        scan[lane] = warp_inclusive_sum(x) - x;
+    }
+    __syncthreads();
+    u64 run = scan[warp] + inc - sum;
+#pragma unroll
+    for (int j = 0; j < kOrderItems; ++j) {
+        run += w[j];
+        if (id[j] >= 0) k[tid * items + j] = run;
+    }
+    __syncthreads();
+    if (tid == 0) boundary_sh = split_boundary(tk, next, k, capacity, err);
+    __syncthreads();
+    const int boundary = boundary_sh, left_parts = tk.parts / 2;
+#pragma unroll
+    for (int j = 0; j < kOrderItems; ++j)
+        if (id[j] >= 0) labels[id[j]] = tid * items + j < boundary ? tk.first_part : tk.first_part + left_parts;
 }
 
 // Part weights + cut terms of the initial partition (part_weights,

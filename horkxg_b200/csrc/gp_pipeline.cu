@@ -1105,73 +1105,87 @@ std::vector<DepthPlan> plan_tasks(int parts) {
     return depths;
 }
 
+// Entries up to which a cluster's 16 SMs walk the rows of the replicated
+// diffusion; above, a cooperative grid does.  Measured us per depth (65 steps),
+// cluster and grid: RGG of 3,001 vertices (29 K entries) 369 and 409; coarsest
+// graphs of RMAT-14 k = 32 (0.7 M) 1,074 and 719, of RMAT-16 k = 16 (0.4 M)
+// 977 and 627.  With diffusion_kernel's grid or the former cluster form:
+// RGG 3,001 810, RMAT-16 2,098, RMAT-20 k = 32 2,278 (now 890).
+constexpr i64 kClusterDiffM = 1 << 18;
+
 template <typename T>
-void launch_diffusion(Device& d, const DGraph<T>& g, int ntasks, const InitTask* tasks, const i32* task_of_pos,
+void launch_diffusion(Device& d, const DGraph<T>& g, int ntasks, const InitTask* tasks, i32* task_of_pos,
                       i32 positions, const i32* order, const i32* labels, u32 seed, int steps, float* deg, float* xa,
-                      float* xb, Moments* contrib, float* x_out, u64* key, u32* bar, i64 max_degree = -1) {
+                      float* xb, Moments* contrib, float* x_out, u64* key, u32* bar, float* exchange = nullptr,
+                      i64 max_degree = -1) {
     using O = typename T::O;
     using W = typename T::W;
-    // Small graphs (max_degree known, every row within a warp's reach): one
-    // thread-block cluster, same values, no grid barriers.
-    if (d.small_diffusion && max_degree >= 0 && max_degree <= kHeavyRow && positions <= kSmallDiffN &&
-        g.m <= kSmallDiffM && positions == g.n) {
-        auto small = diffusion_small_kernel<O, W>;
-        const size_t smem = small_diffusion_smem(positions);
-        // the attribute is shared by every thread of the process (server
-        // slots launch concurrently): always the largest size, never lowered
-        GP_CUDA(cudaFuncSetAttribute(small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(small_diffusion_smem(kSmallDiffN))));
-        // a power of two: one block per 1024 positions and per
-        // kSmallDiffBlockEdges edges
-        int cs = 1;
-        while (cs < kSmallDiffCluster && (cs * kSmallDiffThreads < positions || cs * kSmallDiffBlockEdges < g.m)) cs *= 2;
-        if (cs > 8) GP_CUDA(cudaFuncSetAttribute(small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(cs);
-        cfg.blockDim = dim3(kSmallDiffThreads);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = cs;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        // a cluster that cannot be placed (too few free SMs in a GPC) leaves
-        // the graph to the cooperative kernel, which computes the same values
-        int placeable = 0;
-        GP_CUDA(cudaOccupancyMaxActiveClusters(&placeable, small, &cfg));
-        if (placeable > 0) {
-            launch_cluster(d, "diffusion_small_kernel", small, cs, kSmallDiffThreads, smem, ntasks, tasks, task_of_pos,
-                           positions, order, labels, g.off.get(), g.nbr.get(), g.ewp(), seed, steps, x_out, key);
-            return;
+    auto cooperative = [&](const char* name, void* kernel, int grid, int threads, size_t smem, void** args) {
+        GP_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(u32), d.stream));
+        cudaEvent_t ev0 = nullptr;
+        if (d.prof) { ev0 = d.event(); GP_CUDA(cudaEventRecord(ev0, d.stream)); }
+        GP_CUDA(cudaLaunchCooperativeKernel(kernel, grid, threads, args, smem, d.stream));
+        ++d.launches;
+        if (d.prof) {
+            cudaEvent_t ev1 = d.event();
+            GP_CUDA(cudaEventRecord(ev1, d.stream));
+            auto& e = d.prof_table[name];
+            e.pending.push_back({ev0, ev1});
+            ++e.launches;
         }
-    }
-    auto kernel = diffusion_kernel<O, W>;
-    int per_sm = 0;
-    GP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
-    const int max_grid = std::max(1, per_sm) * d.sms;
-    const int grid = std::max(1, std::min({max_grid, 2 * d.sms, blocks_for(positions, kWarps)}));
-    GP_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(u32), d.stream));
+    };
     const O* off = g.off.get();
     const i32* nbr = g.nbr.get();
     const W* ew = g.ewp();
     u32* bar_counter = bar;
     u32* bar_gen = bar + 1;
     u32* err = d.err;
-    void* args[] = {&ntasks, &tasks, &task_of_pos, &positions, &order, &labels, &off, &nbr, &ew, &seed, &steps,
-                    &deg, &xa, &xb, &contrib, &x_out, &key, &bar_counter, &bar_gen, &err};
-    cudaEvent_t ev0 = nullptr;
-    if (d.prof) { ev0 = d.event(); GP_CUDA(cudaEventRecord(ev0, d.stream)); }
-    GP_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kernel), grid, kThreads, args, 0, d.stream));
-    ++d.launches;
-    if (d.prof) {
-        cudaEvent_t ev1 = d.event();
-        GP_CUDA(cudaEventRecord(ev1, d.stream));
-        auto& e = d.prof_table["diffusion_kernel"];
-        e.pending.push_back({ev0, ev1});
-        ++e.launches;
+    // Every row within a warp's reach and the vectors within shared memory:
+    // replicated vectors, the same values (max_degree < 0: not known).
+    if (d.small_diffusion && max_degree >= 0 && max_degree <= kHeavyRow && positions <= kFastN && positions == g.n) {
+        auto cluster = diffusion_fast_kernel<false, O, W>;
+        // the attribute is shared by every thread of the process (server
+        // slots launch concurrently): always the largest size, never lowered
+        const i32 cluster_n = 16 * kFastBlockRows;
+        GP_CUDA(cudaFuncSetAttribute(cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(fast_diffusion_smem(cluster_n, false))));
+        const int most = wide_cluster_blocks(d, cluster, kFastThreads, fast_diffusion_smem(cluster_n, false));
+        if (g.m <= kClusterDiffM && positions <= most * kFastBlockRows) {
+            // 64 rows a block while there are blocks (RGG of 1,000 vertices,
+            // us per depth: 237, with 128 rows a block 275)
+            int blocks = 1;
+            while (blocks < most && blocks * 64 < positions) blocks *= 2;
+            launch_cluster(d, "diffusion_fast_kernel", cluster, blocks, kFastThreads,
+                           fast_diffusion_smem(positions, false), ntasks, tasks, positions, order, labels, off, nbr,
+                           ew, seed, steps, static_cast<float*>(nullptr), x_out, key, static_cast<u32*>(nullptr),
+                           static_cast<u32*>(nullptr), err);
+            return;
+        }
+        auto grid_kernel = diffusion_fast_kernel<true, O, W>;
+        const size_t smem = fast_diffusion_smem(positions, true);
+        GP_CUDA(cudaFuncSetAttribute(grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(fast_diffusion_smem(kFastN, true))));
+        // a warp per row, one block per SM; the rows of eight lanes need
+        // kFastBlockRows positions per block at most
+        const int grid = std::max((positions + kFastBlockRows - 1) / kFastBlockRows,
+                                  std::min(std::max(d.sms / d.share, 1), blocks_for(positions, kFastWarps)));
+        i32 n = positions;
+        void* args[] = {&ntasks, &tasks, &n, &order, &labels, &off, &nbr, &ew, &seed, &steps,
+                        &exchange, &x_out, &key, &bar_counter, &bar_gen, &err};
+        cooperative("diffusion_fast_kernel", reinterpret_cast<void*>(grid_kernel), grid, kFastThreads, smem, args);
+        return;
     }
+    GP_CUDA(cudaMemsetAsync(task_of_pos, 0xff, static_cast<size_t>(positions) * sizeof(i32), d.stream));
+    launch(d, "task_positions_kernel", task_positions_kernel, ntasks, kThreads, 0, ntasks, tasks, task_of_pos);
+    auto kernel = diffusion_kernel<O, W>;
+    int per_sm = 0;
+    GP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
+    const int max_grid = std::max(1, per_sm) * d.sms;
+    const int grid = std::max(1, std::min({max_grid, 2 * d.sms, blocks_for(positions, kWarps)}));
+    const i32* top = task_of_pos;
+    void* args[] = {&ntasks, &tasks, &top, &positions, &order, &labels, &off, &nbr, &ew, &seed, &steps,
+                    &deg, &xa, &xb, &contrib, &x_out, &key, &bar_counter, &bar_gen, &err};
+    cooperative("diffusion_kernel", reinterpret_cast<void*>(kernel), grid, kThreads, 0, args);
 }
 
 // `trace` (optional, device, depths x n floats): for every recursion depth
@@ -1207,6 +1221,7 @@ void initial_partition(Device& d, const DGraph<T>& g, int parts, double ratio, u
     Buf<i32> order(d, static_cast<size_t>(n)), task_of_pos(d, static_cast<size_t>(n));
     launch(d, "iota_kernel", iota_kernel, blocks_for(n, kThreads), kThreads, 0, n, order.get());
     Buf<float> deg(d, static_cast<size_t>(n)), xa(d, static_cast<size_t>(n)), xb(d, static_cast<size_t>(n));
+    Buf<float> exchange(d, 3 * static_cast<size_t>(n));
     Buf<Moments> contrib(d, static_cast<size_t>(n));
     Buf<u64> key(d, static_cast<size_t>(n)), key_alt(d, static_cast<size_t>(n)), prefix(d, static_cast<size_t>(n));
     Buf<u32> bar(d, 2);
@@ -1220,16 +1235,20 @@ void initial_partition(Device& d, const DGraph<T>& g, int parts, double ratio, u
     }
     for (size_t dpt = 0; dpt < depths.size(); ++dpt) {
         const int nt = static_cast<int>(depths[dpt].tasks.size());
-        GP_CUDA(cudaMemsetAsync(task_of_pos.get(), 0xff, n * sizeof(i32), d.stream));
-        launch(d, "task_positions_kernel", task_positions_kernel, nt, kThreads, 0, nt, dtasks[dpt].get(), task_of_pos.get());
-        GP_LAUNCH();
         float* x_out = trace ? trace + dpt * static_cast<size_t>(n) : nullptr;
         launch_diffusion(d, g, nt, dtasks[dpt].get(), task_of_pos.get(), n, order.get(), labels.get(), seed, 64,
-                         deg.get(), xa.get(), xb.get(), contrib.get(), x_out, key.get(), bar.get(), max_degree);
-        launch(d, "task_sort_kernel", task_sort_kernel, nt, kThreads, 0, nt, dtasks[dpt].get(), key.get(), key_alt.get(), order.get());
+                         deg.get(), xa.get(), xb.get(), contrib.get(), x_out, key.get(), bar.get(), exchange.get(),
+                         max_degree);
         InitTask* next = dpt + 1 < depths.size() ? dtasks[dpt + 1].get() : nullptr;
-        launch(d, "task_split_kernel", task_split_kernel<W>, nt, kThreads, 0, nt, dtasks[dpt].get(), next, order.get(), g.vwp(), capacity,
-                                                           prefix.get(), labels.get(), d.err);
+        if (n <= kOrderN) {
+            launch(d, "task_order_kernel", task_order_kernel<W>, nt, kOrderThreads, 0, nt, dtasks[dpt].get(), next,
+                   key.get(), order.get(), g.vwp(), capacity, labels.get(), d.err);
+        } else {
+            launch(d, "task_sort_kernel", task_sort_kernel, nt, kThreads, 0, nt, dtasks[dpt].get(), key.get(),
+                   key_alt.get(), order.get());
+            launch(d, "task_split_kernel", task_split_kernel<W>, nt, kThreads, 0, nt, dtasks[dpt].get(), next,
+                   order.get(), g.vwp(), capacity, prefix.get(), labels.get(), d.err);
+        }
         GP_LAUNCH();
     }
     d.check_errors();
@@ -1239,7 +1258,7 @@ void initial_partition(Device& d, const DGraph<T>& g, int parts, double ratio, u
     launch(d, "cut_kernel", cut_kernel<typename T::O, W>, stride_grid(d, static_cast<i64>(n) * 32), kThreads, 0, n,
            g.off.get(), g.nbr.get(), g.ewp(), labels.get(), loads.get() + parts);
     {
-        const auto& hubs = hub_index(d, g);
+        const auto& hubs = hub_index(d, g, max_degree > kHubThreshold ? -1 : 0);
         if (hubs.count)
             launch(d, "hub_cut_kernel", hub_cut_kernel<typename T::O, W>, static_cast<int>(hubs.chunks), kThreads, 0,
                    hubs.chunk.get(), g.nbr.get(), g.ewp(), labels.get(), loads.get() + parts);
@@ -2371,8 +2390,6 @@ void initial_partition_static(const gp_graph* gi, int parts, double ratio, u32 s
     for (size_t dpt = 0; dpt < depths.size(); ++dpt) {
         const int nt = static_cast<int>(depths[dpt].tasks.size());
         InitTask* tasks = sc.tasks + dpt * kMaxInitTasks;
-        GP_CUDA(cudaMemsetAsync(sc.task_of_pos, 0xff, static_cast<size_t>(n) * sizeof(i32), stream));
-        launch(d, "task_positions_kernel", task_positions_kernel, nt, kThreads, 0, nt, tasks, sc.task_of_pos);
         launch_diffusion(d, g, nt, tasks, sc.task_of_pos, n, sc.order, labels, seed, 64, sc.deg, sc.xa, sc.xb,
                          sc.contrib, nullptr, sc.key, sc.bar);
         launch(d, "task_sort_kernel", task_sort_kernel, nt, kThreads, 0, nt, tasks, sc.key, sc.key_alt, sc.order);
@@ -2922,15 +2939,12 @@ gp_status gp_diffusion(gp_ctx* ctx, const gp_graph* graph, const int32_t* labels
             gp::Buf<gp::i32> dl(d, static_cast<size_t>(n)), order(d, static_cast<size_t>(n)), top(d, static_cast<size_t>(n));
             gp::to_device(d, dl.get(), labels, static_cast<size_t>(n));
             std::vector<gp::i32> ord(members);
-            std::vector<gp::i32> tp(static_cast<size_t>(n), -1);
-            for (size_t i = 0; i < members.size(); ++i) tp[i] = 0;
             ord.resize(static_cast<size_t>(n), 0);
             gp::to_device(d, order.get(), ord.data(), ord.size());
-            gp::to_device(d, top.get(), tp.data(), tp.size());
             gp::InitTask task{0, static_cast<gp::i32>(members.size()), group, 2, 0, -1, -1};
             gp::Buf<gp::InitTask> dt(d, 1);
             gp::to_device(d, dt.get(), &task, 1);
-            gp::Buf<float> deg(d, n), xa(d, n), xb(d, n), xo(d, n);
+            gp::Buf<float> deg(d, n), xa(d, n), xb(d, n), xo(d, n), exchange(d, 3 * static_cast<size_t>(n));
             gp::Buf<gp::Moments> contrib(d, n);
             gp::Buf<gp::u64> key(d, n);
             gp::Buf<gp::u32> bar(d, 2);
@@ -2943,7 +2957,7 @@ gp_status gp_diffusion(gp_ctx* ctx, const gp_graph* graph, const int32_t* labels
             gp::fetch(d, &max_degree, md.get(), 1);
             gp::launch_diffusion<T>(d, g, 1, dt.get(), top.get(), n, order.get(), dl.get(), seed, steps, deg.get(),
                                     xa.get(), xb.get(), contrib.get(), xo.get(), key.get(), bar.get(),
-                                    static_cast<gp::i64>(max_degree));
+                                    exchange.get(), static_cast<gp::i64>(max_degree));
             d.check_errors();
             gp::to_host(d, x, xo.get(), static_cast<size_t>(n));
             d.sync();

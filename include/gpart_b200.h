@@ -302,10 +302,11 @@ gp_status gp_ctx_set_sync_mode(gp_ctx* ctx, int blocking);
  * device's block slots, so that kernels of other contexts run beside them;
  * results do not depend on it.  The server sets it to its slot count. */
 gp_status gp_ctx_set_device_share(gp_ctx* ctx, int share);
-/* Small coarsest graphs (at most 4096 vertices, 2,097,152 edges and rows of
- * at most 4096 edges) run the spectral diffusion in one thread-block cluster
- * instead of a cooperative grid; both compute the same values.  enable = 0 keeps the
- * grid kernel for every graph (default 1). */
+/* Coarsest graphs of at most 8192 vertices with rows of at most 4096 entries
+ * run the spectral diffusion with every vector replicated in shared memory (one
+ * thread-block cluster, or a cooperative grid for graphs of more than 262,144
+ * entries); the general kernel computes the same values.  enable = 0 keeps the
+ * general kernel for every graph (default 1). */
 gp_status gp_ctx_set_small_diffusion(gp_ctx* ctx, int enable);
 
 /* Hubs (vertices of more than 2048 edges) aggregate their neighbours'
