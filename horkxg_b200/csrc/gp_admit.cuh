@@ -1,0 +1,463 @@
+// Admission of one SCLP round (src/coarsen.cu:600-680,1086-1121,1334-1370).
+// A proposal to a target whose whole demand fits its cap is accepted; the
+// proposals to an over-subscribed target are accepted in the order (gain
+// descending, tie descending, vertex ascending) while their weight fits.
+//
+// The order is needed inside each such target only, so nothing is sorted
+// globally (the reference and an earlier form sorted all of them by target):
+// the proposals are gathered into one segment per target -- counted while
+// they are classified, placed by an atomic allocation, in no particular order
+// -- and a warp ranks a segment of at most 32 by comparing all pairs; a longer
+// one (a hub's cluster) is cut by a block at a threshold, as the rebalance
+// cuts its crossing bucket.  Most segments hold 2 to 5 proposals; on power-law
+// graphs the largest hold 10^5-10^6, of which a cluster admits a few thousand.
+// Those are first narrowed by all blocks in two steps, by a logarithmic code
+// of the gain and by the eight bits that follow in the order (one block streaming a segment of
+// 10^6 six times took longer than the sort: RMAT-24 +70 ms).
+#pragma once
+
+#include "gp_refine.cuh"
+#include "gp_sclp.cuh"
+
+namespace gp {
+
+constexpr u32 kWarpSegment = 32;
+
+// cls: 0 = no move, 1 = accept, 2 = decided by its segment.  slot[v]: the
+// proposal's place in its target's segment.
+__global__ void __launch_bounds__(kThreads) admit_classify_kernel(i64 n, const i32* __restrict__ target,
+                                                                  const u64* __restrict__ demand,
+                                                                  const u64* __restrict__ cw, u64 cap,
+                                                                  unsigned char* cls, u32* crowd, u32* slot, i32* list,
+                                                                  SclpState* state) {
+    if (state->done) return;
+    const i64 v = static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x;
+    bool contested = false;
+    i32 to = -1;
+    if (v < n) {
+        const i32 t = target[v];
+        unsigned char c = 0;
+        if (t != kInvalid) {
+            const u64 base = cw[t];
+            if (base <= cap) {
+                if (demand[t] <= cap - base) {
+                    c = 1;
+                } else {
+                    contested = true;
+                    to = t;
+                }
+            }
+        }
+        cls[v] = c;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, contested);
+    if (!m) return;
+    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+    u32 base = 0;
+    // one atomic per target and warp: a hub's cluster draws many proposals
+    const unsigned peers = __match_any_sync(0xffffffffu, to);
+    const int first = __ffs(peers) - 1;
+    if (contested && lane == first) base = atomicAdd(&crowd[to], static_cast<u32>(__popc(peers)));
+    base = __shfl_sync(0xffffffffu, base, first);
+    if (contested) slot[v] = base + __popc(peers & lanemask_lt());
+    if (lane == leader) base = atomicAdd(&state->contested, static_cast<u32>(__popc(m)));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (contested) list[base + __popc(m & lanemask_lt())] = static_cast<i32>(v);
+}
+
+// The first proposal of every contested target reserves its segment;
+// `demand` of the target then holds the segment's start.
+__global__ void __launch_bounds__(kThreads) admit_reserve_kernel(const i32* __restrict__ list,
+                                                                 const i32* __restrict__ target,
+                                                                 const u32* __restrict__ slot,
+                                                                 const u32* __restrict__ crowd, u64* demand,
+                                                                 i32* segments, SclpState* state) {
+    if (state->done) return;
+    const i64 count = state->contested;
+    for (i64 base = static_cast<i64>(blockIdx.x) * kThreads; base < count; base += static_cast<i64>(gridDim.x) * kThreads) {
+        const i64 i = base + threadIdx.x;
+        i32 t = -1;
+        u32 size = 0;
+        if (i < count) {
+            const i32 v = list[i];
+            if (slot[v] == 0) { t = target[v]; size = crowd[t]; }
+        }
+        // one atomic each per warp: the places and the list entries
+        const u32 inc = warp_inclusive_sum(size);
+        const unsigned m = __ballot_sync(0xffffffffu, t >= 0);
+        if (!m) continue;
+        const int lane = threadIdx.x & 31;
+        u64 place = 0;
+        u32 entry = 0;
+        if (lane == 31) {
+            place = atomic_add_u64(&state->segment_items, inc);
+            entry = atomicAdd(&state->segments, static_cast<u32>(__popc(m)));
+        }
+        place = __shfl_sync(0xffffffffu, place, 31);
+        entry = __shfl_sync(0xffffffffu, entry, 31);
+        if (t >= 0) {
+            demand[t] = place + inc - size;
+            segments[entry + __popc(m & lanemask_lt())] = t;
+        }
+    }
+}
+
+// A proposal in its segment: the gain, then tie (high) and vertex (low).
+__global__ void __launch_bounds__(kThreads) admit_scatter_kernel(const i32* __restrict__ list,
+                                                                 const i32* __restrict__ target,
+                                                                 const u64* __restrict__ gain,
+                                                                 const u32* __restrict__ tie,
+                                                                 const u32* __restrict__ slot,
+                                                                 const u64* __restrict__ demand, u64* seg_gain,
+                                                                 u64* seg_tie, const SclpState* state) {
+    if (state->done) return;
+    const i64 count = state->contested;
+    for (i64 i = static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * kThreads) {
+        const i32 v = list[i];
+        const u64 at = demand[target[v]] + slot[v];
+        seg_gain[at] = gain[v];
+        seg_tie[at] = (static_cast<u64>(~tie[v]) << 32) | static_cast<u32>(v);   // ascending = tie descending, vertex ascending
+    }
+}
+
+// Longer than this, a segment is narrowed by all blocks first.
+constexpr u32 kGiantSegment = 8192;
+// Per giant segment: weights by gain code, weights by fine code inside the
+// crossing one, and the number of proposals left for the block that finishes it.
+constexpr int kGiantRow = 513;
+
+// 0..251, larger for larger gains: exact below 8, then four codes per octave.
+__device__ __forceinline__ u32 gain_code(u64 g) {
+    if (g < 4) return static_cast<u32>(g);
+    const int msb = 63 - __clzll(static_cast<long long>(g));
+    return static_cast<u32>((msb - 1) * 4 + static_cast<int>((g >> (msb - 2)) & 3));
+}
+
+// The order's next eight bits inside one gain code, ascending in (gain
+// descending, tie descending): the gain's bits below the code, then the tie's.
+__device__ __forceinline__ u32 fine_code(u64 g, u64 k) {
+    const int msb = g ? 63 - __clzll(static_cast<long long>(g)) : 0;
+    const int bits = msb > 2 ? msb - 2 : 0;
+    const u64 below = ~g & ((1ULL << bits) - 1);
+    if (bits >= 8) return static_cast<u32>(below >> (bits - 8));
+    return static_cast<u32>((below << (8 - bits)) | (k >> (56 + bits)));
+}
+
+// Warp per segment of at most kWarpSegment proposals; longer ones are listed.
+template <typename W>
+__global__ void __launch_bounds__(kThreads) admit_resolve_kernel(const i32* __restrict__ segments,
+                                                                 const u64* __restrict__ demand,
+                                                                 const u64* __restrict__ seg_gain,
+                                                                 const u64* __restrict__ seg_tie,
+                                                                 const u64* __restrict__ cw, const W* __restrict__ vw,
+                                                                 u64 cap, u32* crowd, unsigned char* cls, i32* big,
+                                                                 i32* giant, u64* giant_rows, SclpState* state) {
+    if (state->done) return;
+    const int lane = threadIdx.x & 31;
+    const i64 count = state->segments;
+    const i64 warps = static_cast<i64>(gridDim.x) * kWarps;
+    for (i64 s = static_cast<i64>(blockIdx.x) * kWarps + (threadIdx.x >> 5); s < count; s += warps) {
+        const i32 t = segments[s];
+        const u32 size = crowd[t];
+        if (size > kGiantSegment) {
+            u32 at = 0;
+            if (lane == 0) giant[at = atomicAdd(&state->giants, 1u)] = t;
+            at = __shfl_sync(0xffffffffu, at, 0);
+            for (int i = lane; i < kGiantRow; i += 32) giant_rows[static_cast<i64>(at) * kGiantRow + i] = 0;
+            continue;
+        }
+        if (size > kWarpSegment) {
+            if (lane == 0) big[atomicAdd(&state->big, 1u)] = t;
+            continue;
+        }
+        const u64 start = demand[t], room = cap - cw[t];
+        u64 g = 0, k = ~0ULL, w = 0, before = 0;
+        if (static_cast<u32>(lane) < size) {
+            g = seg_gain[start + lane];
+            k = seg_tie[start + lane];
+            w = static_cast<u64>(weight_at(vw, static_cast<i64>(k & 0xffffffffu)));
+        }
+        for (u32 j = 0; j < size; ++j) {
+            const u64 gj = __shfl_sync(0xffffffffu, g, static_cast<int>(j));
+            const u64 kj = __shfl_sync(0xffffffffu, k, static_cast<int>(j));
+            const u64 wj = __shfl_sync(0xffffffffu, w, static_cast<int>(j));
+            if (gj > g || (gj == g && kj < k)) before += wj;
+        }
+        if (static_cast<u32>(lane) < size) cls[k & 0xffffffffu] = before + w <= room ? 1 : 0;
+        __syncwarp();
+        if (lane == 0) crowd[t] = 0;   // for the next round
+    }
+}
+
+constexpr int kAdmitThreads = 512;
+
+struct AdmitShared {
+    u64 scan[32];
+    u64 hist[256];
+    u32 members[256];
+    u64 g_and, g_or, k_and, k_or, left;
+    u32 few;
+    int digit;
+    static constexpr u32 kFew = 128;
+    u64 few_g[kFew], few_k[kFew], few_w[kFew];
+};
+
+// The bin of `hist` (256 entries) that crosses the quota `left`, and what is
+// left of the quota in it.  The whole block calls it.
+__device__ __forceinline__ void crossing_bin(const u64* hist, u64 left, AdmitShared& sh) {
+    __syncthreads();
+    const u64 w = threadIdx.x < 256 ? __ldcg(&hist[threadIdx.x]) : 0;
+    const u64 before = select_exclusive_sum(w, sh.scan);
+    if (threadIdx.x < 256 && before <= left && before + w > left) {
+        sh.digit = static_cast<int>(threadIdx.x);
+        sh.left = left - before;
+    }
+    __syncthreads();
+}
+
+// Three passes of all blocks over the giant segments, a chunk of kGiantSegment
+// proposals at a time.  STEP 0 sums weights by gain code; STEP 1 decides the
+// proposals outside the crossing code and sums those in it by fine code; STEP 2
+// decides those outside the crossing fine code and lists the rest.
+template <int STEP, typename W>
+__global__ void __launch_bounds__(kAdmitThreads) admit_giant_kernel(const i32* __restrict__ giant,
+                                                                    const u64* __restrict__ demand,
+                                                                    const u64* __restrict__ seg_gain,
+                                                                    const u64* __restrict__ seg_tie,
+                                                                    const u64* __restrict__ cw,
+                                                                    const W* __restrict__ vw, u64 cap,
+                                                                    const u32* __restrict__ crowd, u64* giant_rows,
+                                                                    u64* rest, unsigned char* cls,
+                                                                    const SclpState* state) {
+    if (state->done) return;
+    __shared__ AdmitShared sh;
+    const u32 giants = state->giants;
+    for (u32 s = 0; s < giants; ++s) {
+        const i32 t = giant[s];
+        const u32 size = crowd[t];
+        if (static_cast<u64>(blockIdx.x) * kGiantSegment >= size) continue;   // uniform over the block
+        u64* row = giant_rows + static_cast<i64>(s) * kGiantRow;
+        const u64 start = demand[t];
+        u32 code = 0, fine = 0;
+        if (STEP >= 1) {
+            crossing_bin(row, cap - cw[t], sh);
+            code = static_cast<u32>(sh.digit);
+        }
+        if (STEP == 2) {
+            const u64 left = sh.left;
+            crossing_bin(row + 256, left, sh);
+            fine = static_cast<u32>(sh.digit);
+        }
+        if (STEP < 2) {
+            __syncthreads();
+            if (threadIdx.x < 256) sh.hist[threadIdx.x] = 0;
+            __syncthreads();
+        }
+        for (u64 c = blockIdx.x; c * kGiantSegment < size; c += gridDim.x) {
+            const u32 end = static_cast<u32>(min(static_cast<u64>(size), (c + 1) * kGiantSegment));
+            for (u32 j0 = static_cast<u32>(c * kGiantSegment); j0 < end; j0 += kAdmitThreads) {
+                const u32 j = j0 + threadIdx.x;
+                u64 k = 0;
+                u32 mine = ~0u;   // bin of this step, ~0: none
+                bool keep = false;
+                if (j < end) {
+                    const u32 gc = 255 - gain_code(seg_gain[start + j]);   // ascending = gain descending
+                    k = seg_tie[start + j];
+                    const u32 fc = fine_code(seg_gain[start + j], k);
+                    if (STEP == 0) mine = gc;
+                    else if (gc != code) { if (STEP == 1) cls[k & 0xffffffffu] = gc < code ? 1 : 0; }
+                    else if (STEP == 1) mine = fc;
+                    else if (fc != fine) cls[k & 0xffffffffu] = fc < fine ? 1 : 0;
+                    else keep = true;
+                }
+                if (STEP < 2) {
+                    // most share a bin (gain 1): one addition per bin and warp
+                    const bool has = mine != ~0u;
+                    const unsigned peers = __match_any_sync(0xffffffffu, mine);
+                    const u64 w = vw ? weight_group_sum(peers, has ? static_cast<u64>(vw[k & 0xffffffffu]) : 0)
+                                     : static_cast<u64>(__popc(peers));
+                    if (has && static_cast<int>(threadIdx.x & 31) == __ffs(peers) - 1) atomic_add_u64(&sh.hist[mine], w);
+                } else {
+                    const u64 at = warp_append(keep, &row[512]);
+                    if (keep) rest[start + at] = j;
+                }
+            }
+        }
+        if (STEP < 2) {
+            __syncthreads();
+            if (threadIdx.x < 256 && sh.hist[threadIdx.x])
+                atomic_add_u64(&row[(STEP == 0 ? 0 : 256) + threadIdx.x], sh.hist[threadIdx.x]);
+        }
+    }
+}
+
+// Block per longer segment: the threshold (gain, then tie and vertex) up to
+// which the proposals fit is built from the high end, eight varying bits a
+// step (see resolve_bucket); at most kFew matching proposals are ranked
+// directly.
+template <typename W>
+__global__ void __launch_bounds__(kAdmitThreads) admit_resolve_big_kernel(
+    const i32* __restrict__ big, const u64* __restrict__ demand, const u64* __restrict__ seg_gain,
+    const u64* __restrict__ seg_tie, const u64* __restrict__ cw, const W* __restrict__ vw, u64 cap, u32* crowd,
+    const i32* __restrict__ giant, const u64* __restrict__ giant_rows, const u64* __restrict__ rest,
+    unsigned char* cls, const SclpState* state) {
+    if (state->done) return;
+    __shared__ AdmitShared sh;
+    const int lane = threadIdx.x & 31;
+    const u32 bigs = state->big, segments = bigs + state->giants;
+    for (u32 s = blockIdx.x; s < segments; s += gridDim.x) {
+        const bool narrowed = s >= bigs;   // a giant segment: what admit_giant_kernel left
+        const i32 t = narrowed ? giant[s - bigs] : big[s];
+        const u64* row = giant_rows + static_cast<i64>(s - bigs) * kGiantRow;
+        const u32 size = narrowed ? static_cast<u32>(row[512]) : crowd[t];
+        const u64* gains = seg_gain + demand[t];
+        const u64* ties = seg_tie + demand[t];
+        const u64* index = rest + demand[t];
+        u64 quota = cap - cw[t];
+        if (narrowed) {
+            crossing_bin(row, quota, sh);
+            quota = sh.left;
+            crossing_bin(row + 256, quota, sh);
+            quota = sh.left;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) {
+            sh.g_and = sh.k_and = ~0ULL;
+            sh.g_or = sh.k_or = 0;
+            sh.few = 0;
+            sh.left = quota;
+        }
+        __syncthreads();
+        auto items = [&](auto f) {   // ascending keys
+            for (u32 j = threadIdx.x; j < size; j += kAdmitThreads) {
+                const u64 i = narrowed ? index[j] : j;
+                f(~gains[i], ties[i]);
+            }
+        };
+        u64 ga = ~0ULL, go = 0, ka = ~0ULL, ko = 0;
+        items([&](u64 g, u64 k) { ga &= g; go |= g; ka &= k; ko |= k; });
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            ga &= __shfl_xor_sync(0xffffffffu, ga, o);
+            go |= __shfl_xor_sync(0xffffffffu, go, o);
+            ka &= __shfl_xor_sync(0xffffffffu, ka, o);
+            ko |= __shfl_xor_sync(0xffffffffu, ko, o);
+        }
+        if (lane == 0) {
+            atomicAnd(reinterpret_cast<unsigned long long*>(&sh.g_and), static_cast<unsigned long long>(ga));
+            atomicOr(reinterpret_cast<unsigned long long*>(&sh.g_or), static_cast<unsigned long long>(go));
+            atomicAnd(reinterpret_cast<unsigned long long*>(&sh.k_and), static_cast<unsigned long long>(ka));
+            atomicOr(reinterpret_cast<unsigned long long*>(&sh.k_or), static_cast<unsigned long long>(ko));
+        }
+        __syncthreads();
+        u64 hi_g = 0, above_g = 0, hi_k = 0, above_k = 0;
+        auto matches = [&](u64 g, u64 k) { return (g & above_g) == hi_g && (k & above_k) == hi_k; };
+        u32 matching = size;
+        auto step = [&](auto digit) {
+            if (threadIdx.x < 256) { sh.hist[threadIdx.x] = 0; sh.members[threadIdx.x] = 0; }
+            if (threadIdx.x == 0) sh.digit = 255;
+            __syncthreads();
+            items([&](u64 g, u64 k) {
+                if (!matches(g, k)) return;
+                const u32 dg = digit(g, k);
+                atomicAdd(&sh.members[dg], 1u);
+                if (vw) atomic_add_u64(&sh.hist[dg], static_cast<u64>(vw[k & 0xffffffffu]));
+            });
+            __syncthreads();
+            u64 w = 0;
+            if (threadIdx.x < 256) w = vw ? sh.hist[threadIdx.x] : static_cast<u64>(sh.members[threadIdx.x]);
+            const u64 before = select_exclusive_sum(w, sh.scan);
+            const u64 left = sh.left;
+            __syncthreads();
+            if (threadIdx.x < 256 && before <= left && before + w > left) {
+                sh.digit = static_cast<int>(threadIdx.x);
+                sh.left = left - before;
+            }
+            __syncthreads();
+            const u32 dg = static_cast<u32>(sh.digit);
+            matching = sh.members[dg];
+            __syncthreads();
+            return dg;
+        };
+        auto narrow = [&](u64 vary, u64& hi, u64& above, auto pick) {
+            while (vary && matching > AdmitShared::kFew) {
+                const int top = 63 - __clzll(static_cast<long long>(vary));
+                const int shift = top > 7 ? top - 7 : 0;
+                const u64 field = 0xffULL >> (7 - (top - shift));
+                const u32 dg = step([&](u64 g, u64 k) { return static_cast<u32>((pick(g, k) >> shift) & field); });
+                above |= field << shift;
+                hi = (hi & ~(field << shift)) | (static_cast<u64>(dg) << shift);
+                vary &= ~(~0ULL << shift);
+            }
+        };
+        // bits in which the proposals agree match from the start
+        if (matching > AdmitShared::kFew) {
+            hi_g = sh.g_and;
+            above_g = ~(sh.g_and ^ sh.g_or);
+            narrow(sh.g_and ^ sh.g_or, hi_g, above_g, [](u64 g, u64) { return g; });
+        }
+        if (matching > AdmitShared::kFew) {
+            hi_k = sh.k_and;
+            above_k = ~(sh.k_and ^ sh.k_or);
+            narrow(sh.k_and ^ sh.k_or, hi_k, above_k, [](u64, u64 k) { return k; });
+        }
+        items([&](u64 g, u64 k) {
+            if (!matches(g, k)) {
+                const u64 a = g & above_g;
+                cls[k & 0xffffffffu] = a < hi_g || (a == hi_g && (k & above_k) < hi_k) ? 1 : 0;
+                return;
+            }
+            const u32 at = atomicAdd(&sh.few, 1u);
+            if (at >= AdmitShared::kFew) return;   // cannot happen: vertices differ
+            sh.few_g[at] = g;
+            sh.few_k[at] = k;
+            sh.few_w[at] = static_cast<u64>(weight_at(vw, static_cast<i64>(k & 0xffffffffu)));
+        });
+        __syncthreads();
+        constexpr u32 kLanes = kAdmitThreads / AdmitShared::kFew;
+        const u32 few = min(sh.few, AdmitShared::kFew), at = threadIdx.x / kLanes;
+        u64 before = 0;
+        if (at < few)
+            for (u32 j = threadIdx.x % kLanes; j < few; j += kLanes)
+                if (sh.few_g[j] < sh.few_g[at] || (sh.few_g[j] == sh.few_g[at] && sh.few_k[j] < sh.few_k[at]))
+                    before += sh.few_w[j];
+        for (int o = kLanes / 2; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+        if (at < few && threadIdx.x % kLanes == 0) {
+            const u64 left = sh.left;
+            cls[sh.few_k[at] & 0xffffffffu] = before <= left && sh.few_w[at] <= left - before ? 1 : 0;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) crowd[t] = 0;   // for the next round
+        __syncthreads();
+    }
+}
+
+// Moves the accepted vertices, clears `demand` for the next round and counts
+// the clusters that became empty (sources are movers' clusters and targets are
+// not, so only one side of a cluster's weight changes in a round).
+template <typename W>
+__global__ void __launch_bounds__(kThreads) sclp_commit_kernel(i64 n, const unsigned char* __restrict__ cls,
+                                                               const i32* __restrict__ target,
+                                                               const W* __restrict__ vw, i32* clusters, u64* cw,
+                                                               u64* demand, int round, SclpState* state) {
+    if (state->done) return;
+    __shared__ long long sh[kWarps + 1];
+    const i64 v = static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x;
+    long long change = 0;
+    if (v < n) {
+        demand[v] = 0;
+        if (cls[v] == 1) {
+            const i32 t = target[v];
+            const i32 s = clusters[v];
+            const u64 w = static_cast<u64>(weight_at(vw, v));
+            const u64 had = atomic_add_u64(&cw[s], 0ULL - w), got = atomic_add_u64(&cw[t], w);
+            clusters[v] = t;
+            if (w) change = (got == 0 ? 1 : 0) - (had == w ? 1 : 0);
+        }
+    }
+    change = block_sum(change, sh);
+    if (round == 0 && blockIdx.x == 0) change -= static_cast<long long>(state->weightless);
+    if (threadIdx.x == 0 && change) atomic_add_u64(&state->clusters, static_cast<u64>(change));
+}
+
+}  // namespace gp

@@ -575,24 +575,76 @@ __global__ void __launch_bounds__(kThreads) giant_place_kernel(const SegChunk* _
 // `bitmap_from`: rows longer than this (up to kGiantSeg) take the bitmap
 // ranking of class 5 whatever their class by length, since on levels with
 // few coarse vertices a bitmap over the id range costs less than sorting.
-__global__ void row_class_kernel(i64 rows, const i64* temp_off, i64 smem_cap, i64 bitmap_from, u64* keys, i32* vals,
-                                 u64* counts) {
-    __shared__ unsigned long long local[2 * kRowClasses];
-    if (threadIdx.x < 2 * kRowClasses) local[threadIdx.x] = 0;
+// Rows are appended to their class's list a tile of 2048 rows at a time, so a
+// list stays nearly in row order; classes 1 and 2 grow from the two ends of
+// one array, 3 and 4 of a second, 5 and 6 of a third (`lists` holds the three,
+// `rows` entries each).  The lists' order does not matter.
+constexpr int kRowItems = 8;
+constexpr int kRowTile = kThreads * kRowItems;
+
+__host__ __device__ inline i64 row_list_at(int k, i64 rows, i64 count) {   // first entry of class k's list
+    const i64 array = static_cast<i64>((k - 1) / 2) * rows;
+    return (k & 1) ? array : array + rows - count;
+}
+
+__global__ void __launch_bounds__(kThreads) row_class_kernel(i64 rows, const i64* __restrict__ temp_off, i64 smem_cap,
+                                                             i64 bitmap_from, i32* lists, u64* counts) {
+    __shared__ u32 warp_count[kWarps][kRowClasses];
+    __shared__ unsigned long long entries[kRowClasses];
+    __shared__ i64 base_sh[kRowClasses];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < kRowClasses) entries[threadIdx.x] = 0;
     __syncthreads();
-    const i64 c = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (c < rows) {
-        const i64 l = temp_off[c + 1] - temp_off[c];
-        const int k = l == 0 ? 0 : l <= 32 ? 1 : l <= kWarpSegCap ? 2 : (l > bitmap_from && l <= kGiantSeg) ? 5
-                    : l <= kMidSegCap ? 3 : l <= smem_cap ? 4 : l <= kGiantSeg ? 5 : 6;
-        keys[c] = static_cast<u64>(k);
-        vals[c] = static_cast<i32>(c);
-        atomicAdd(&local[k], 1ull);
-        atomicAdd(&local[kRowClasses + k], static_cast<unsigned long long>(l));
+    for (i64 base = static_cast<i64>(blockIdx.x) * kRowTile; base < rows; base += static_cast<i64>(gridDim.x) * kRowTile) {
+        int cls[kRowItems];
+        u32 mine = 0;   // lane k: rows of class k in the warp
+        const i64 c0 = base + warp * 32 * kRowItems + lane;
+#pragma unroll
+        for (int j = 0; j < kRowItems; ++j) {
+            const i64 c = c0 + j * 32;
+            i64 l = 0;
+            int k = 0;
+            if (c < rows) {
+                l = temp_off[c + 1] - temp_off[c];
+                k = l == 0 ? 0 : l <= 32 ? 1 : l <= kWarpSegCap ? 2 : (l > bitmap_from && l <= kGiantSeg) ? 5
+                  : l <= kMidSegCap ? 3 : l <= smem_cap ? 4 : l <= kGiantSeg ? 5 : 6;
+            }
+            cls[j] = k;
+#pragma unroll
+            for (int q = 1; q < kRowClasses; ++q) {
+                const unsigned m = __ballot_sync(0xffffffffu, k == q);
+                if (!m) continue;
+                if (lane == q) mine += __popc(m);
+                const i64 sum = warp_sum(k == q ? l : i64{0});
+                if (lane == 0) atomicAdd(&entries[q], static_cast<unsigned long long>(sum));
+            }
+        }
+        if (lane < kRowClasses) warp_count[warp][lane] = mine;
+        __syncthreads();
+        if (threadIdx.x >= 1 && threadIdx.x < kRowClasses) {
+            u32 run = 0;
+            for (int w = 0; w < kWarps; ++w) { const u32 x = warp_count[w][threadIdx.x]; warp_count[w][threadIdx.x] = run; run += x; }
+            base_sh[threadIdx.x] = run ? static_cast<i64>(atomic_add_u64(&counts[threadIdx.x], run)) : 0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 1; q < kRowClasses; ++q) {
+            i64 at = base_sh[q] + warp_count[warp][q];
+            i32* list = lists + static_cast<i64>((q - 1) / 2) * rows;
+#pragma unroll
+            for (int j = 0; j < kRowItems; ++j) {
+                const unsigned m = __ballot_sync(0xffffffffu, cls[j] == q);
+                if (cls[j] == q) {
+                    const i64 i = at + __popc(m & lanemask_lt());
+                    list[(q & 1) ? i : rows - 1 - i] = static_cast<i32>(c0 + j * 32);
+                }
+                at += __popc(m);
+            }
+        }
+        __syncthreads();   // the shared counts are free again
     }
-    __syncthreads();
-    if (threadIdx.x < 2 * kRowClasses && local[threadIdx.x])
-        atomicAdd(reinterpret_cast<unsigned long long*>(&counts[threadIdx.x]), local[threadIdx.x]);
+    if (threadIdx.x >= 1 && threadIdx.x < kRowClasses && entries[threadIdx.x])
+        atomicAdd(reinterpret_cast<unsigned long long*>(&counts[kRowClasses + threadIdx.x]), entries[threadIdx.x]);
 }
 
 template <typename O>

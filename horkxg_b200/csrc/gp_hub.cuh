@@ -147,6 +147,7 @@ template <typename O, typename W, typename S>
 __global__ void __launch_bounds__(kThreads) hub_insert_kernel(
     const Chunk* __restrict__ chunks, const i32* __restrict__ nbr, const W* __restrict__ ew,
     const i32* __restrict__ clusters, RoundParams p, const i64* __restrict__ table_off, S* table, u32* err) {
+    if (!round_ready(p)) return;
     const Chunk ch = chunks[blockIdx.x];
     if (role_blocked(p.identity ? ch.v : clusters[ch.v], p)) return;   // no proposal: nothing to count
     const int lane = threadIdx.x & 31;
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(THREADS) hub_smem_kernel(
     const i32* __restrict__ hub_ids, const O* __restrict__ off, const i32* __restrict__ nbr,
     const W* __restrict__ ew, const W* __restrict__ vw, const i32* __restrict__ clusters,
     const u64* __restrict__ cw, RoundParams p, SclpOut out) {
+    if (!round_ready(p)) return;
     constexpr int kHubSmemWarps = THREADS / 32;
     constexpr int kHubSmemThreads = THREADS;
     extern __shared__ unsigned long long table[];   // hub_smem_slots(degree) entries
@@ -307,6 +309,7 @@ __global__ void hub_extent_kernel(i64 count, const i32* __restrict__ hubs, const
 template <typename O>
 __global__ void role_work_kernel(i64 count, const i32* __restrict__ list, const O* __restrict__ off,
                                  const i32* __restrict__ clusters, RoundParams p, u64* out) {
+    if (!round_ready(p)) return;
     u64 v_n = 0, e_n = 0, s_n = 0;
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
          i += static_cast<i64>(gridDim.x) * blockDim.x) {
@@ -330,6 +333,7 @@ template <typename W, typename S>
 __global__ void __launch_bounds__(kThreads) hub_candidates_kernel(
     i64 hubs, const i32* __restrict__ hub_list, const i64* __restrict__ table_off, S* table,
     const i32* __restrict__ clusters, RoundParams p, HubPartial* partials, i64 tile_base) {
+    if (!round_ready(p)) return;
     __shared__ CandShared red;
     __shared__ int hub_sh;
     const i64 tile = tile_base + blockIdx.x;  // tile_base offsets a launch over a sub-range of tables
@@ -364,6 +368,7 @@ template <typename W>
 __global__ void hub_finalize_kernel(i64 hubs, const i32* __restrict__ hub_list, const i64* __restrict__ table_off,
                                     const HubPartial* __restrict__ partials, const i32* __restrict__ clusters,
                                     const W* __restrict__ vw, const u64* __restrict__ cw, RoundParams p, SclpOut out) {
+    if (!round_ready(p)) return;
     const i64 h = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (h >= hubs) return;
     const i32 v = hub_list[h];
@@ -593,6 +598,7 @@ template <typename O, typename W>
 __global__ void __launch_bounds__(kThreads) affinity_direct_warp_kernel(
     i64 count, const i32* __restrict__ list, const O* __restrict__ off, const i32* __restrict__ nbr,
     const W* __restrict__ ew, const W* __restrict__ vw, const u64* __restrict__ cw, RoundParams p, SclpOut out) {
+    if (!round_ready(p)) return;
     const int lane = threadIdx.x & 31;
     const i64 gid = (static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
     if (gid >= count) return;
@@ -612,6 +618,7 @@ template <typename O, typename W>
 __global__ void __launch_bounds__(kThreads) affinity_direct_block_kernel(
     i64 count, const i32* __restrict__ list, const O* __restrict__ off, const i32* __restrict__ nbr,
     const W* __restrict__ ew, const W* __restrict__ vw, const u64* __restrict__ cw, RoundParams p, SclpOut out) {
+    if (!round_ready(p)) return;
     __shared__ CandShared red;
     const i32 v = list[blockIdx.x];
     if (role_blocked(v, p)) {
@@ -630,6 +637,7 @@ template <typename W>
 __global__ void __launch_bounds__(kThreads) hub_direct_kernel(const Chunk* __restrict__ chunks,
                                                               const i32* __restrict__ nbr, const W* __restrict__ ew,
                                                               RoundParams p, HubPartial* partials) {
+    if (!round_ready(p)) return;
     __shared__ CandShared red;
     const Chunk ch = chunks[blockIdx.x];
     if (role_blocked(ch.v, p)) return;   // the hub's finalisation writes no proposal
@@ -646,6 +654,7 @@ __global__ void hub_chunk_finalize_kernel(i64 hubs, const i32* __restrict__ hub_
                                           const HubPartial* __restrict__ partials, const i32* __restrict__ clusters,
                                           const W* __restrict__ vw, const u64* __restrict__ cw, RoundParams p,
                                           SclpOut out) {
+    if (!round_ready(p)) return;
     const i64 h = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (h >= hubs) return;
     const i32 v = hub_list[h];

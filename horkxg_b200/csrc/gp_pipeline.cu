@@ -27,6 +27,7 @@
 #include "gp_initial.cuh"
 #include "gp_refine.cuh"
 #include "gp_hub.cuh"
+#include "gp_admit.cuh"
 #include "gp_refine_small.cuh"
 #include "gp_analyze.cuh"
 #include "gp_symmetrize.cuh"
@@ -261,39 +262,29 @@ __global__ void iota_kernel(i64 n, i32* a) {
     if (i < n) a[i] = static_cast<i32>(i);
 }
 
+// Sum of m weights as out[0] + out[1] * 2^32: the sums of the weights' low and
+// high halves, which fit 64 bits for fewer than 2^32 weights.  Two additions
+// per block (a saturating compare-and-swap loop on one word made the blocks
+// queue: 250-500 us on levels of 10^5-10^7 entries).
 template <typename W>
-__global__ void widen_weights_kernel(i64 n, const W* vw, u64* out) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = static_cast<u64>(weight_at(vw, i));
+__global__ void __launch_bounds__(kThreads) split_sum_kernel(i64 m, const W* __restrict__ w, u64* out) {
+    __shared__ u64 sh[kWarps + 1];
+    u64 lo = 0, hi = 0;
+    for (i64 i = static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x; i < m; i += static_cast<i64>(gridDim.x) * kThreads) {
+        const u64 x = static_cast<u64>(weight_at(w, i));
+        lo += x & 0xffffffffu;
+        hi += x >> 32;
+    }
+    lo = block_sum(lo, sh);
+    hi = block_sum(hi, sh);
+    if (threadIdx.x == 0 && lo) atomic_add_u64(&out[0], lo);
+    if (threadIdx.x == 0 && hi) atomic_add_u64(&out[1], hi);
 }
 
-template <typename W>
-__global__ void sat_sum_kernel(i64 m, const W* w, u64* out) {
-    __shared__ u64 sh[kWarps];
-    u64 s = 0;
-    for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += static_cast<i64>(gridDim.x) * blockDim.x) {
-        const u64 x = static_cast<u64>(weight_at(w, i));
-        s = ~0ULL - s < x ? ~0ULL : s + x;
-    }
-    for (int o = 16; o; o >>= 1) {
-        const u64 x = __shfl_xor_sync(0xffffffffu, s, o);
-        s = ~0ULL - s < x ? ~0ULL : s + x;
-    }
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s = 0;
-        for (int i = 0; i < kWarps; ++i) s = ~0ULL - s < sh[i] ? ~0ULL : s + sh[i];
-        if (s) {
-            u64 prev = *reinterpret_cast<volatile u64*>(out);
-            while (true) {
-                const u64 next = ~0ULL - prev < s ? ~0ULL : prev + s;
-                const u64 seen = atomic_cas_u64(out, prev, next);
-                if (seen == prev) break;
-                prev = seen;
-            }
-        }
-    }
+// The sum of split_sum_kernel, saturated at 2^64 - 1.
+inline u64 saturated_sum(const u64* parts) {
+    const unsigned __int128 sum = parts[0] + (static_cast<unsigned __int128>(parts[1]) << 32);
+    return sum > ~0ULL ? ~0ULL : static_cast<u64>(sum);
 }
 
 inline int stride_grid(Device& d, i64 items, int per_block = kThreads) {
@@ -314,8 +305,9 @@ struct AggResult {
 template <typename T>
 struct SclpWork {
     Buf<i32> clusters, target, list, list_alt, clist, clist_alt;
-    Buf<u64> cw, gain, demand, keys, keys_alt, excl, ckeys, ckeys_alt;
-    Buf<u32> tie, ccount;
+    Buf<u64> cw, gain, demand, keys, keys_alt, excl;
+    Buf<u32> tie, crowd, slot;
+    Buf<SclpState> state;
     Buf<unsigned char> cls;
     Buf<i64> pos, flags, positions, table_off;
     Buf<HubSlot> table;
@@ -328,8 +320,9 @@ struct SclpWork {
         clusters.ensure(d, s); target.ensure(d, s); list.ensure(d, s); list_alt.ensure(d, s);
         clist.ensure(d, s); clist_alt.ensure(d, s);
         cw.ensure(d, s); gain.ensure(d, s); demand.ensure(d, s); keys.ensure(d, s); keys_alt.ensure(d, s);
-        excl.ensure(d, s); ckeys.ensure(d, s); ckeys_alt.ensure(d, s);
-        tie.ensure(d, s); ccount.ensure(d, 8); cls.ensure(d, s);
+        excl.ensure(d, s);
+        tie.ensure(d, s); crowd.ensure(d, s); slot.ensure(d, s); cls.ensure(d, s);
+        state.ensure(d, 1);
         pos.ensure(d, s); flags.ensure(d, s); positions.ensure(d, s);
         scalars.ensure(d, 16);
     }
@@ -374,33 +367,35 @@ void aggregate(Device& d, const DGraph<T>& g, SclpWork<T>& w, int parts, u32 see
     const W* vw = g.vwp();
     u64* sc = w.scalars.get();
     GP_CUDA(cudaMemsetAsync(sc, 0, 16 * sizeof(u64), d.stream));
-    w.ccount.zero(d);
-    launch(d, "weight_stats_kernel", weight_stats_kernel<W>, stride_grid(d, n), kThreads, 0, n, vw, sc);
+    w.state.zero(d);
+    SclpState* state = w.state.get();
+    i32* clusters = w.clusters.get();
+    u64* cw = w.cw.get();
+    launch(d, "sclp_setup_kernel", sclp_setup_kernel<O, W>, stride_grid(d, n, kSetupTile), kThreads, 0, n, off, vw,
+           w.clist.get(), w.clist_alt.get(), clusters, cw, w.target.get(), w.demand.get(), w.crowd.get(), state);
     GP_LAUNCH();
-    launch(d, "degree_class_kernel", degree_class_kernel<O>, blocks_for(n, kThreads), kThreads, 0, n, off, w.ckeys.get(),
-           w.clist.get(), w.ccount.get(), sc + 8);
-    GP_LAUNCH();
-    radix_sort<u64, i32>(d, w.ckeys.get(), w.clist.get(), w.ckeys_alt.get(), w.clist_alt.get(), n, 0, 8);
     trace().mark(d, "agg.classes_launched", level);
-    u64 stats[16];
-    u32 cnt[kClasses];
-    to_host(d, stats, sc, 16);
-    fetch(d, cnt, w.ccount.get(), kClasses);
-    const u64 total = stats[0], maxw = stats[1];
+    SclpState hs;
+    fetch(d, &hs, state, 1);
+    const u32* cnt = hs.classes;
+    const u64 total = hs.total, maxw = hs.max;
     const u64 denom = static_cast<u64>(beta) * static_cast<u64>(parts);
     const u64 cap = std::max(maxw, total / denom + (total % denom != 0 ? 1 : 0));
-    i64 class_off[kClasses + 1] = {0};
-    for (int c = 0; c < kClasses; ++c) class_off[c + 1] = class_off[c] + cnt[c];
-    const i32* lists = w.clist.get();
-    auto class_list = [&](int c) { return lists + class_off[c]; };
+    // see class_slot; class 5 is the hub index
+    auto class_list = [&](int c) -> const i32* {
+        const i32* l = c <= 2 ? w.clist.get() : w.clist_alt.get();
+        return (c & 1) ? l : l + (n - cnt[c]);
+    };
 
     trace().mark(d, "agg.classes_fetched", level);
     if (!w.edge_total_known) {
         if (ew) {
-            Buf<u64> t(d, 1);
+            Buf<u64> t(d, 2);
             t.zero(d);
-            launch(d, "sat_sum_kernel", sat_sum_kernel<W>, stride_grid(d, g.m), kThreads, 0, g.m, ew, t.get());
-            fetch(d, &w.edge_total, t.get(), 1);
+            launch(d, "split_sum_kernel", split_sum_kernel<W>, stride_grid(d, g.m), kThreads, 0, g.m, ew, t.get());
+            u64 sums[2];
+            fetch(d, sums, t.get(), 2);
+            w.edge_total = saturated_sum(sums);
         } else {
             w.edge_total = static_cast<u64>(g.m);
         }
@@ -437,12 +432,6 @@ void aggregate(Device& d, const DGraph<T>& g, SclpWork<T>& w, int parts, u32 see
     }
 
     trace().mark(d, "agg.hub_tables", level);
-    i32* clusters = w.clusters.get();
-    u64* cw = w.cw.get();
-    launch(d, "iota_kernel", iota_kernel, blocks_for(n, kThreads), kThreads, 0, n, clusters);
-    launch(d, "widen_weights_kernel", widen_weights_kernel<W>, blocks_for(n, kThreads), kThreads, 0, n, vw, cw);
-    launch(d, "fill_i32_kernel", fill_i32_kernel, blocks_for(n, kThreads), kThreads, 0, n, w.target.get(), kInvalid);
-    GP_LAUNCH();
     SclpOut so{w.target.get(), w.gain.get(), w.tie.get(), w.demand.get()};
 
     // Algorithmic bytes of one affinity+decode pass over class c, counting
@@ -465,7 +454,8 @@ void aggregate(Device& d, const DGraph<T>& g, SclpWork<T>& w, int parts, u32 see
             for (int c = 1; c < kClasses; ++c)
                 if (cnt[c])
                     launch(d, "role_work_kernel", role_work_kernel<O>, stride_grid(d, cnt[c]), kThreads, 0,
-                           static_cast<i64>(cnt[c]), class_list(c), off, clusters, p, cw_dev.get() + 3 * c);
+                           static_cast<i64>(cnt[c]), c == 5 ? hubs.list.get() : class_list(c), off, clusters, p,
+                           cw_dev.get() + 3 * c);
             fetch(d, &work[0][0], cw_dev.get(), 3 * kClasses);
             if (chip && gcount) {
                 Buf<u64> gw(d, 3);
@@ -588,60 +578,77 @@ void aggregate(Device& d, const DGraph<T>& g, SclpWork<T>& w, int parts, u32 see
         fetch(d, &c, sc + 5, 1);
         return static_cast<i64>(c);
     };
-    auto sorted_weight_prefix = [&](i64 count) {
-        exclusive_scan<u64>(d, SortedWeight<W>{w.list.get(), vw}, w.excl.get(), count);
-    };
-
     i64 cluster_count = n;
     const i64 desired = (n + 1) / 2;
-    int rounds = 0;
+    // Small levels run all rounds without a round trip (a round that does not
+    // run costs its launches, about 2 us each, a round trip about 10); large
+    // ones return after each, since an empty launch over 10^7 vertices costs
+    // more.  The kernels decide on the device either way.
+    const bool stop_early = n > (1 << 18) || d.prof;
+    // A segment of more than kGiantSegment proposals needs as many vertices.
+    const i64 giant_cap = n / kGiantSegment;
+    Buf<u64> giant_rows(d, static_cast<size_t>(std::max<i64>(giant_cap, 1)) * kGiantRow);
     for (int round = 0; round < 4; ++round) {
-        if (static_cast<double>(cluster_count) <= 0.60 * n) break;
-        const i64 removable = std::max<i64>(0, cluster_count - desired);
-        const double fraction = std::min(0.50, static_cast<double>(removable) / static_cast<double>(cluster_count));
-        const auto threshold = static_cast<u32>(fraction * 4294967296.0);
-        RoundParams p = make_round(seed, level, round, true, threshold);
+        RoundParams p = make_round(seed, level, round, true, 0);
         p.sum32 = sum32;
-        w.demand.zero(d);
+        p.state = state;
+        launch(d, "round_begin_kernel", round_begin_kernel, 1, 1, 0, n, round, state);
         affinity(p);
-        GP_CUDA(cudaMemsetAsync(sc + 3, 0, sizeof(u64), d.stream));
-        launch(d, "admission_classify_kernel", admission_classify_kernel, blocks_for(n, kThreads), kThreads, 0, 
-            n, w.target.get(), w.demand.get(), cw, cap, w.gain.get(), w.cls.get(), sc + 3);
-        GP_LAUNCH();
-        i64 contested = 0;
-        u64 gmax = 0;
-        compact_contested(contested, gmax);
-        if (contested > 0) {
-            order_proposals(d, w, n, contested, gmax);
-            sorted_weight_prefix(contested);
-            launch(d, "segment_heads_kernel", segment_heads_kernel, blocks_for(contested, kThreads), kThreads, 0, 
-                contested, w.list.get(), w.target.get(), w.excl.get(), w.demand.get(), 0);
-            launch(d, "contested_accept_kernel", contested_accept_kernel<W>, blocks_for(contested, kThreads), kThreads, 0, 
-                contested, w.list.get(), w.target.get(), w.excl.get(), w.demand.get(), cw, vw, cap, w.cls.get());
-            GP_LAUNCH();
+        launch(d, "admit_classify_kernel", admit_classify_kernel, blocks_for(n, kThreads), kThreads, 0, n,
+               w.target.get(), w.demand.get(), cw, cap, w.cls.get(), w.crowd.get(), w.slot.get(), w.list.get(), state);
+        launch(d, "admit_reserve_kernel", admit_reserve_kernel, stride_grid(d, n), kThreads, 0, w.list.get(),
+               w.target.get(), w.slot.get(), w.crowd.get(), w.demand.get(), w.list_alt.get(), state);
+        launch(d, "admit_scatter_kernel", admit_scatter_kernel, stride_grid(d, n), kThreads, 0, w.list.get(),
+               w.target.get(), w.gain.get(), w.tie.get(), w.slot.get(), w.demand.get(), w.keys.get(), w.keys_alt.get(),
+               state);
+        i32* big = reinterpret_cast<i32*>(w.slot.get());   // the slots are used up: big segments from
+        i32* giant = big + n / 2;                           // the front (at most n / 33), giants from the middle
+        launch(d, "admit_resolve_kernel", admit_resolve_kernel<W>, stride_grid(d, n * 8), kThreads, 0,
+               w.list_alt.get(), w.demand.get(), w.keys.get(), w.keys_alt.get(), cw, vw, cap, w.crowd.get(),
+               w.cls.get(), big, giant, giant_rows.get(), state);
+        if (giant_cap) {
+            const int grid = static_cast<int>(std::min<i64>((n + kGiantSegment - 1) / kGiantSegment, d.grid_limit(4)));
+            auto narrow = [&](auto kernel) {
+                launch(d, "admit_giant_kernel", kernel, grid, kAdmitThreads, 0, giant, w.demand.get(), w.keys.get(),
+                       w.keys_alt.get(), cw, vw, cap, w.crowd.get(), giant_rows.get(), w.excl.get(), w.cls.get(), state);
+            };
+            narrow(admit_giant_kernel<0, W>);
+            narrow(admit_giant_kernel<1, W>);
+            narrow(admit_giant_kernel<2, W>);
         }
-        launch(d, "sclp_commit_kernel", sclp_commit_kernel<W>, blocks_for(n, kThreads), kThreads, 0, n, w.cls.get(), w.target.get(), vw,
-                                                                                 clusters, cw);
+        launch(d, "admit_resolve_big_kernel", admit_resolve_big_kernel<W>,
+               static_cast<int>(std::min<i64>(n / (kWarpSegment + 1) + 1, d.grid_limit(2))), kAdmitThreads, 0, big,
+               w.demand.get(), w.keys.get(), w.keys_alt.get(), cw, vw, cap, w.crowd.get(), giant, giant_rows.get(),
+               w.excl.get(), w.cls.get(), state);
+        launch(d, "sclp_commit_kernel", sclp_commit_kernel<W>, blocks_for(n, kThreads), kThreads, 0, n, w.cls.get(),
+               w.target.get(), vw, clusters, cw, w.demand.get(), round, state);
         GP_LAUNCH();
-        cluster_count = count_clusters();
         trace().mark(d, "agg.round", round);
-        ++rounds;
-        if (log.on)
-            log.out << "ml_gpu_sclp_round level=" << level << " round=" << round << " mover_fraction=" << fraction
-                    << " clusters=" << cluster_count
-                    << " contraction_ratio=" << static_cast<double>(cluster_count) / static_cast<double>(n) << '\n';
-        if (static_cast<double>(cluster_count) <= 0.60 * n) break;
+        if (stop_early || round == 3 || log.on) {
+            fetch(d, &hs, state, 1);
+            if (log.on && hs.rounds == round + 1)
+                log.out << "ml_gpu_sclp_round level=" << level << " round=" << round
+                        << " mover_fraction=" << hs.fraction[round] << " clusters=" << hs.clusters
+                        << " contraction_ratio=" << static_cast<double>(hs.clusters) / static_cast<double>(n) << '\n';
+            if (static_cast<double>(hs.clusters) <= 0.60 * static_cast<double>(n)) break;
+        }
     }
+    cluster_count = static_cast<i64>(hs.clusters);
+    const int rounds = hs.rounds;
 
     if (pack && cnt[0] > 1) {
         const i64 iso = cnt[0];
-        exclusive_scan<u64>(d, SortedWeight<W>{class_list(0), vw}, w.excl.get(), iso);
+        i32* isolated = w.list.get();   // in vertex order
+        exclusive_scan<i64>(d, IsIsolated{off, sizeof(O) == 8 ? 1 : 0}, w.pos.get(), n);
+        launch(d, "compact_isolated_kernel", compact_isolated_kernel<O>, blocks_for(n, kThreads), kThreads, 0, n, off,
+               w.pos.get(), isolated);
+        exclusive_scan<u64>(d, SortedWeight<W>{isolated, vw}, w.excl.get(), iso);
         launch(d, "fill_i32_kernel", fill_i32_kernel, blocks_for(iso + 1, kThreads), kThreads, 0, iso + 1, w.list_alt.get(),
                                                                                    std::numeric_limits<i32>::max());
-        launch(d, "isolated_rep_kernel", isolated_rep_kernel<W>, blocks_for(iso, kThreads), kThreads, 0, iso, class_list(0), w.excl.get(),
+        launch(d, "isolated_rep_kernel", isolated_rep_kernel<W>, blocks_for(iso, kThreads), kThreads, 0, iso, isolated, w.excl.get(),
                                                                                     vw, cap, w.list_alt.get());
         launch(d, "isolated_commit_kernel", isolated_commit_kernel<W>, blocks_for(iso, kThreads), kThreads, 0, 
-            iso, class_list(0), w.excl.get(), vw, cap, w.list_alt.get(), clusters, cw);
+            iso, isolated, w.excl.get(), vw, cap, w.list_alt.get(), clusters, cw);
         GP_LAUNCH();
         cluster_count = count_clusters();
     }
@@ -677,11 +684,10 @@ void aggregate(Device& d, const DGraph<T>& g, SclpWork<T>& w, int parts, u32 see
     }
 
     trace().mark(d, "agg.isolated_two_hop", level);
-    // compaction
+    // compaction: the non-empty clusters in id order
     Buf<i32> compact(d, static_cast<size_t>(n));
-    exclusive_scan<i32>(d, NonEmpty{cw}, compact.get(), n, reinterpret_cast<i32*>(sc + 6));
-    i32 coarse_n = 0;
-    fetch(d, &coarse_n, reinterpret_cast<i32*>(sc + 6), 1);
+    exclusive_scan<i32>(d, NonEmpty{cw}, compact.get(), n);
+    const i32 coarse_n = static_cast<i32>(cluster_count);
     out.map = Buf<i32>(d, static_cast<size_t>(n));
     out.cvw = Buf<W>(d, static_cast<size_t>(std::max<i32>(coarse_n, 1)));
     out.cvw.zero(d);
@@ -708,15 +714,18 @@ void contract(Device& d, const DGraph<T>& g, const i32* map, i64 coarse_n, Buf<t
     using O = typename T::O;
     using W = typename T::W;
     const i64 n = g.n, m = g.m;
-    Buf<i64> fdeg(d, static_cast<size_t>(coarse_n) + 1);
-    Buf<i64> temp_off(d, static_cast<size_t>(coarse_n) + 1);
-    Buf<i64> cursor(d, static_cast<size_t>(coarse_n) + 1);
+    // fine degrees, cursors and lengths of the coarse rows, cleared together
+    const size_t row_count = static_cast<size_t>(coarse_n) + 1;
+    Buf<i64> row_state(d, 3 * row_count);
+    i64* fdeg = row_state.get();
+    i64* cursor = fdeg + row_count;
+    i64* row_len = cursor + row_count;
+    Buf<i64> temp_off(d, row_count);
     Buf<i64> scal(d, 4);
-    fdeg.zero(d);
-    cursor.zero(d);
-    launch(d, "row_fine_degree_kernel", row_fine_degree_kernel<O>, blocks_for(n, kThreads), kThreads, 0, n, g.off.get(), map, fdeg.get());
+    row_state.zero(d);
+    launch(d, "row_fine_degree_kernel", row_fine_degree_kernel<O>, blocks_for(n, kThreads), kThreads, 0, n, g.off.get(), map, fdeg);
     GP_LAUNCH();
-    exclusive_scan_array<i64>(d, fdeg.get(), temp_off.get(), coarse_n + 1);
+    exclusive_scan_array<i64>(d, fdeg, temp_off.get(), coarse_n + 1);
     const u32 sentinel = static_cast<u32>(coarse_n);
     trace().mark(d, "contract.rows", coarse_n);
     Buf<u32> tgt(d, static_cast<size_t>(std::max<i64>(m, 1)));
@@ -725,20 +734,19 @@ void contract(Device& d, const DGraph<T>& g, const i32* map, i64 coarse_n, Buf<t
     d.prof_bytes("scatter_edges_kernel", static_cast<double>(n + 1) * sizeof(O) + n * (4.0 + 8 + 8) +
                                              static_cast<double>(m) * (4 + 4 + 4 + (g.ewp() ? sizeof(W) : 0) + sizeof(W)));
     launch(d, "scatter_edges_kernel", scatter_edges_kernel<O, W>, blocks_for(warps * 32, kThreads), kThreads, 0, n,
-           g.off.get(), g.nbr.get(), g.ewp(), map, temp_off.get(), cursor.get(), sentinel, tgt.get(), wt.get());
+           g.off.get(), g.nbr.get(), g.ewp(), map, temp_off.get(), cursor, sentinel, tgt.get(), wt.get());
     const auto& hubs = hub_index(d, g);
     if (hubs.count) {
         Buf<i64> hub_dst(d, static_cast<size_t>(hubs.count));
         launch(d, "hub_reserve_kernel", hub_reserve_kernel<O>, blocks_for(hubs.count, kThreads), kThreads, 0,
-               hubs.count, hubs.list.get(), g.off.get(), map, temp_off.get(), cursor.get(), hub_dst.get());
+               hubs.count, hubs.list.get(), g.off.get(), map, temp_off.get(), cursor, hub_dst.get());
         launch(d, "hub_scatter_kernel", hub_scatter_kernel<O, W>, static_cast<int>(hubs.chunks), kThreads, 0,
                hubs.chunk.get(), g.off.get(), g.nbr.get(), g.ewp(), map, hub_dst.get(), sentinel, tgt.get(), wt.get());
     }
     GP_LAUNCH();
     trace().mark(d, "contract.scatter", m);
     // row classes
-    Buf<u64> rk(d, static_cast<size_t>(coarse_n)), rk_alt(d, static_cast<size_t>(coarse_n));
-    Buf<i32> rl(d, static_cast<size_t>(coarse_n)), rl_alt(d, static_cast<size_t>(coarse_n));
+    Buf<i32> lists(d, 3 * static_cast<size_t>(coarse_n));
     Buf<u64> rc(d, 2 * kRowClasses);
     rc.zero(d);
     // A row is ranked by the bitmap of segment_bitmap_kernel instead of a
@@ -746,15 +754,13 @@ void contract(Device& d, const DGraph<T>& g, const i32* map, i64 coarse_n, Buf<t
     // costs about coarse_n / 32 words per window plus two passes over the row,
     // the sort three passes with barriers; both give the same row.
     const i64 bitmap_from = std::max<i64>(kWarpSegCap, coarse_n / 64);
-    launch(d, "row_class_kernel", row_class_kernel, blocks_for(coarse_n, kThreads), kThreads, 0, coarse_n,
-           temp_off.get(), static_cast<i64>(seg_smem_capacity<W>()), bitmap_from, rk.get(), rl.get(), rc.get());
+    launch(d, "row_class_kernel", row_class_kernel, stride_grid(d, coarse_n, kRowTile), kThreads, 0, coarse_n,
+           temp_off.get(), static_cast<i64>(seg_smem_capacity<W>()), bitmap_from, lists.get(), rc.get());
     GP_LAUNCH();
-    radix_sort<u64, i32>(d, rk.get(), rl.get(), rk_alt.get(), rl_alt.get(), coarse_n, 0, 8);
     u64 rcnt[2 * kRowClasses];
     fetch(d, rcnt, rc.get(), 2 * kRowClasses);
     const u64* rent = rcnt + kRowClasses;   // entries per class
-    i64 cstart[kRowClasses + 1] = {0};
-    for (int k = 0; k < kRowClasses; ++k) cstart[k + 1] = cstart[k] + static_cast<i64>(rcnt[k]);
+    auto row_list = [&](int k) { return lists.get() + row_list_at(k, coarse_n, static_cast<i64>(rcnt[k])); };
     // segment kernels read and write each scattered entry once (target + weight)
     auto seg_bytes = [&](int k) { return 2.0 * static_cast<double>(rent[k]) * (4 + sizeof(W)); };
     d.prof_bytes("segment_warp_kernel", seg_bytes(1));
@@ -763,21 +769,19 @@ void contract(Device& d, const DGraph<T>& g, const i32* map, i64 coarse_n, Buf<t
     const bool sort_big = (coarse_n + kBitmapWindow - 1) / kBitmapWindow > kSortWindows;
     d.prof_bytes(sort_big ? "segment_sort_kernel" : "segment_bitmap_kernel", seg_bytes(5));
     d.prof_bytes("giant_place_kernel", seg_bytes(6));
-    Buf<i64> row_len(d, static_cast<size_t>(coarse_n) + 1);
-    row_len.zero(d);
     const int key_bits = std::max(1, bit_width_u64(static_cast<u64>(coarse_n)));
     if (rcnt[1])
         launch(d, "segment_warp_kernel", segment_warp_kernel<W>, blocks_for(static_cast<i64>(rcnt[1]) * 32, kThreads),
-               kThreads, 0, rcnt[1], rl.get() + cstart[1], temp_off.get(), sentinel, tgt.get(), wt.get(),
-               row_len.get());
+               kThreads, 0, rcnt[1], row_list(1), temp_off.get(), sentinel, tgt.get(), wt.get(),
+               row_len);
     if (rcnt[2]) {
         const size_t smem = static_cast<size_t>(kWarps) * (2 * kWarpSegCap * sizeof(W) +
                                                           (2 * kWarpSegCap + kRadix) * sizeof(u32));
         GP_CUDA(cudaFuncSetAttribute(segment_warp_radix_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(smem)));
         launch(d, "segment_warp_radix_kernel", segment_warp_radix_kernel<W>,
-               blocks_for(static_cast<i64>(rcnt[2]) * 32, kThreads), kThreads, smem, rcnt[2], rl.get() + cstart[2],
-               temp_off.get(), sentinel, key_bits, tgt.get(), wt.get(), row_len.get());
+               blocks_for(static_cast<i64>(rcnt[2]) * 32, kThreads), kThreads, smem, rcnt[2], row_list(2),
+               temp_off.get(), sentinel, key_bits, tgt.get(), wt.get(), row_len);
     }
     for (int k = 3; k <= 4; ++k) {
         if (!rcnt[k]) continue;
@@ -787,19 +791,25 @@ void contract(Device& d, const DGraph<T>& g, const i32* map, i64 coarse_n, Buf<t
                                      static_cast<int>(2 * static_cast<size_t>(seg_smem_capacity<W>()) *
                                                       (sizeof(u32) + sizeof(W)))));
         launch(d, "segment_smem_kernel", segment_smem_kernel<W>, static_cast<int>(rcnt[k]), kThreads, smem, rcnt[k],
-               rl.get() + cstart[k], temp_off.get(), sentinel, key_bits, cap, tgt.get(), wt.get(), row_len.get());
+               row_list(k), temp_off.get(), sentinel, key_bits, cap, tgt.get(), wt.get(), row_len);
     }
     GP_LAUNCH();
-    // rows above seg_smem_capacity (classes 5 and 6, contiguous in the class
-    // order) are written to alternate buffers
-    const i64 c3 = cstart[5];
+    // rows above seg_smem_capacity (classes 5 and 6, put into one list) are
+    // written to alternate buffers
     const i64 big = static_cast<i64>(rcnt[5] + rcnt[6]);
+    Buf<i32> big_list;
+    if (big) {
+        big_list = Buf<i32>(d, static_cast<size_t>(big));
+        GP_CUDA(cudaMemcpyAsync(big_list.get(), row_list(5), rcnt[5] * sizeof(i32), cudaMemcpyDeviceToDevice, d.stream));
+        GP_CUDA(cudaMemcpyAsync(big_list.get() + rcnt[5], row_list(6), rcnt[6] * sizeof(i32), cudaMemcpyDeviceToDevice,
+                                d.stream));
+    }
     Buf<i64> alt_off;
     Buf<u32> ak;
     Buf<W> aw;
     if (big) {
         alt_off = Buf<i64>(d, static_cast<size_t>(big) + 1);
-        exclusive_scan<i64>(d, BigRowLen{rl.get() + c3, temp_off.get(), big}, alt_off.get(), big + 1,
+        exclusive_scan<i64>(d, BigRowLen{big_list.get(), temp_off.get(), big}, alt_off.get(), big + 1,
                             scal.get());
         i64 alt_total = 0;
         fetch(d, &alt_total, scal.get(), 1);
@@ -808,21 +818,21 @@ void contract(Device& d, const DGraph<T>& g, const i32* map, i64 coarse_n, Buf<t
     }
     if (rcnt[5] && sort_big) {
         launch(d, "segment_sort_kernel", segment_sort_kernel<W>, static_cast<int>(rcnt[5]), kThreads, 0,
-               static_cast<i64>(rcnt[5]), rl.get() + c3, temp_off.get(), alt_off.get(), sentinel, key_bits, tgt.get(),
-               wt.get(), ak.get(), aw.get(), row_len.get());
+               static_cast<i64>(rcnt[5]), big_list.get(), temp_off.get(), alt_off.get(), sentinel, key_bits, tgt.get(),
+               wt.get(), ak.get(), aw.get(), row_len);
         GP_LAUNCH();
     } else if (rcnt[5]) {
         const size_t smem = (static_cast<size_t>(kBitmapWords) + kBitmapGroups) * sizeof(u32);
         GP_CUDA(cudaFuncSetAttribute(segment_bitmap_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(smem)));
         launch(d, "segment_bitmap_kernel", segment_bitmap_kernel<W>, static_cast<int>(rcnt[5]), kThreads, smem,
-               static_cast<i64>(rcnt[5]), rl.get() + c3, temp_off.get(), alt_off.get(), sentinel, coarse_n, tgt.get(),
-               wt.get(), ak.get(), aw.get(), row_len.get());
+               static_cast<i64>(rcnt[5]), big_list.get(), temp_off.get(), alt_off.get(), sentinel, coarse_n, tgt.get(),
+               wt.get(), ak.get(), aw.get(), row_len);
         GP_LAUNCH();
     }
     if (rcnt[6]) {
         const i64 giants = static_cast<i64>(rcnt[6]);
-        const i32* glist = rl.get() + cstart[6];
+        const i32* glist = big_list.get() + rcnt[5];
         const i64* galt = alt_off.get() + rcnt[5];
         Buf<i64> chunk_off(d, static_cast<size_t>(giants) + 1);
         exclusive_scan<i64>(d, GiantChunkCount{glist, temp_off.get(), giants}, chunk_off.get(), giants + 1,
@@ -843,7 +853,7 @@ void contract(Device& d, const DGraph<T>& g, const i32* map, i64 coarse_n, Buf<t
         launch(d, "giant_mark_kernel", giant_mark_kernel, static_cast<int>(chunks_total), kThreads, 0, chunks.get(),
                tgt.get(), sentinel, wpr, gbits.get());
         launch(d, "giant_scan_kernel", giant_scan_kernel, static_cast<int>(giants), kThreads, 0, glist, wpr,
-               gbits.get(), gpre.get(), row_len.get());
+               gbits.get(), gpre.get(), row_len);
         launch(d, "giant_place_kernel", giant_place_kernel<W>, static_cast<int>(chunks_total), kThreads, 0,
                chunks.get(), tgt.get(), wt.get(), sentinel, wpr, gbits.get(), gpre.get(), galt, ak.get(), aw.get());
         GP_LAUNCH();
@@ -851,7 +861,7 @@ void contract(Device& d, const DGraph<T>& g, const i32* map, i64 coarse_n, Buf<t
     trace().mark(d, "contract.segments", static_cast<long long>(rcnt[5]), static_cast<long long>(rcnt[6]));
     out.n = coarse_n;
     out.off = Buf<O>(d, static_cast<size_t>(coarse_n) + 1);
-    exclusive_scan<O>(d, RowLenToO<O>{row_len.get()}, out.off.get(), coarse_n + 1, reinterpret_cast<O*>(scal.get() + 1));
+    exclusive_scan<O>(d, RowLenToO<O>{row_len}, out.off.get(), coarse_n + 1, reinterpret_cast<O*>(scal.get() + 1));
     O cm = 0;
     fetch(d, &cm, reinterpret_cast<O*>(scal.get() + 1), 1);
     out.m = static_cast<i64>(cm);
@@ -864,7 +874,7 @@ void contract(Device& d, const DGraph<T>& g, const i32* map, i64 coarse_n, Buf<t
                kThreads, 0, coarse_n, temp_off.get(), out.off.get(), tgt.get(), wt.get(), out.nbr.get(), out.ew.get());
         if (big)
             launch(d, "copy_big_rows_kernel", copy_big_rows_kernel<O, W>, static_cast<int>(big), kThreads, 0,
-                   rl.get() + c3, alt_off.get(), out.off.get(), ak.get(), aw.get(), out.nbr.get(), out.ew.get());
+                   big_list.get(), alt_off.get(), out.off.get(), ak.get(), aw.get(), out.nbr.get(), out.ew.get());
         GP_LAUNCH();
     }
     out.vw = std::move(cvw);
@@ -1203,14 +1213,14 @@ void initial_partition(Device& d, const DGraph<T>& g, int parts, double ratio, u
     Buf<u64> sc(d, 8);
     sc.zero(d);
     launch(d, "weight_stats_kernel", weight_stats_kernel<W>, stride_grid(d, n), kThreads, 0, n, g.vwp(), sc.get());
-    launch(d, "sat_sum_kernel", sat_sum_kernel<W>, stride_grid(d, g.m), kThreads, 0, g.m, g.ewp(), sc.get() + 2);
+    launch(d, "split_sum_kernel", split_sum_kernel<W>, stride_grid(d, g.m), kThreads, 0, g.m, g.ewp(), sc.get() + 2);
     launch(d, "max_degree_kernel", max_degree_kernel<typename T::O>, stride_grid(d, n), kThreads, 0, n64, g.off.get(),
-           sc.get() + 3);
+           sc.get() + 4);
     GP_LAUNCH();
-    u64 st[4];
-    fetch(d, st, sc.get(), 4);
-    const u64 total = st[0], maxw = st[1], edge_total = st[2];
-    const i64 max_degree = static_cast<i64>(st[3]);
+    u64 st[5];
+    fetch(d, st, sc.get(), 5);
+    const u64 total = st[0], maxw = st[1], edge_total = saturated_sum(st + 2);
+    const i64 max_degree = static_cast<i64>(st[4]);
     if (!total || total == ~0ULL || edge_total == ~0ULL)
         fail(GP_EOVERFLOW, "GPU initializer weight accumulation overflow");
     const u64 capacity = partition_capacity(total, parts, ratio);
@@ -1825,13 +1835,14 @@ gp_refine_stats refine_level(Device& d, const DGraph<T>& g, RefineWork& w, i32* 
 template <typename T>
 u64 directed_total(Device& d, const DGraph<T>& g) {
     if (!g.ewp()) return static_cast<u64>(g.m);
-    Buf<u64> s(d, 1);
+    Buf<u64> s(d, 2);
     s.zero(d);
-    launch(d, "sat_sum_kernel", sat_sum_kernel<typename T::W>, stride_grid(d, g.m), kThreads, 0, g.m, g.ewp(), s.get());
+    launch(d, "split_sum_kernel", split_sum_kernel<typename T::W>, stride_grid(d, g.m), kThreads, 0, g.m, g.ewp(),
+           s.get());
     GP_LAUNCH();
-    u64 total = 0;
-    fetch(d, &total, s.get(), 1);
-    return total;
+    u64 sums[2];
+    fetch(d, sums, s.get(), 2);
+    return saturated_sum(sums);
 }
 
 // The affinity cache can hold 32-bit sums when the level's total directed
@@ -2370,10 +2381,10 @@ void initial_partition_static(const gp_graph* gi, int parts, double ratio, u32 s
         fail(GP_EINVAL, "weighted CSR shape is invalid (offsets not monotone from 0 to m or neighbor out of range)");
 
     launch(d, "weight_stats_kernel", weight_stats_kernel<W>, stride_grid(d, n), kThreads, 0, n, g.vwp(), sc.stats);
-    launch(d, "sat_sum_kernel", sat_sum_kernel<W>, stride_grid(d, g.m), kThreads, 0, g.m, g.ewp(), sc.stats + 2);
-    u64 st[3];
+    launch(d, "split_sum_kernel", split_sum_kernel<W>, stride_grid(d, g.m), kThreads, 0, g.m, g.ewp(), sc.stats + 2);
+    u64 st[4];
     read(st, sc.stats, sizeof(st));
-    const u64 total = st[0], maxw = st[1], edge_total = st[2];
+    const u64 total = st[0], maxw = st[1], edge_total = saturated_sum(st + 2);
     if (!total || total == ~0ULL || edge_total == ~0ULL)
         fail(GP_EOVERFLOW, "GPU initializer weight accumulation overflow");
     const u64 capacity = partition_capacity(total, parts, ratio);

@@ -7,11 +7,11 @@
 //   for deg <= 2048, and a block with an L2-resident global hash table for
 //   hubs above that; the four u64 affinity arrays of the reference never hit
 //   HBM;
-// * admission without a global sort: every target's proposed weight
-//   ("demand") is summed during the affinity pass; a proposal to a target
-//   whose whole demand fits is accepted directly, and only proposals to
-//   over-subscribed targets are ordered by (target, gain desc, tie desc,
-//   vertex) with a stable LSD radix sort over the compacted list;
+// * admission without a sort: every target's proposed weight ("demand") is
+//   summed during the affinity pass; a proposal to a target whose whole
+//   demand fits is accepted directly, and the proposals to each over-
+//   subscribed target are gathered and ranked among themselves
+//   (gp_admit.cuh);
 // * isolated packing, two-hop pairing and compaction as in the reference.
 //
 // The result (cluster map, coarse weights) is bit-identical to the
@@ -28,7 +28,24 @@ constexpr int kMediumSlots = 512;        // warp hash, deg 33..256
 constexpr int kLargeSlots = 4096;        // block hash, deg 257..2048
 constexpr int kHubDegree = 2048;         // above: global hash
 
+// A level's rounds, kept on the device so that consecutive rounds need no
+// round trip: the number of non-empty clusters decides whether a round runs
+// and its mover threshold (src/coarsen.cu:1305-1330).
+struct SclpState {
+    u64 clusters;         // non-empty clusters
+    u64 total, max;       // vertex weight of the level
+    u64 weightless;       // vertices of weight 0: singletons that count as empty
+    u32 classes[8];       // vertices per degree class
+    u32 threshold;
+    i32 done;
+    i32 rounds;           // rounds run
+    u32 contested, segments, big, giants;   // admission lists of the round
+    u64 segment_items;
+    double fraction[4];   // mover fraction of each round, for the log
+};
+
 struct RoundParams {
+    const SclpState* state;   // null: threshold as given, the round always runs
     u32 role_salt;
     u32 tie_salt;
     u32 mover_threshold;
@@ -41,6 +58,7 @@ struct RoundParams {
 // Salts of src/coarsen.cu:1152-1157.
 inline RoundParams make_round(u32 seed, int level, int round, bool filter, u32 mover_threshold) {
     RoundParams p;
+    p.state = nullptr;
     p.role_salt = seed ^ (static_cast<u32>(level) * 0x9e3779b9U) ^ (static_cast<u32>(round) * 0x85ebca6bU) ^ 0x27d4eb2dU;
     p.tie_salt = seed ^ (static_cast<u32>(level) * 0xc2b2ae35U) ^ (static_cast<u32>(round) * 0x165667b1U) ^ 0xd3a2646cU;
     p.mover_threshold = mover_threshold;
@@ -49,6 +67,14 @@ inline RoundParams make_round(u32 seed, int level, int round, bool filter, u32 m
     p.two_hop = 0;
     p.sum32 = 0;
     return p;
+}
+
+// False when the round does not run; fills in the threshold of the device's
+// round state.  Every kernel of a round calls it first.
+__device__ __forceinline__ bool round_ready(RoundParams& p) {
+    if (!p.state) return true;
+    p.mover_threshold = p.state->threshold;
+    return !p.state->done;
 }
 
 __device__ __forceinline__ bool is_mover(i32 c, const RoundParams& p) {
@@ -121,6 +147,7 @@ __global__ void __launch_bounds__(kThreads) affinity_small_kernel(
     i64 count, const i32* __restrict__ list, const O* __restrict__ off, const i32* __restrict__ nbr,
     const W* __restrict__ ew, const W* __restrict__ vw, const i32* __restrict__ clusters,
     const u64* __restrict__ cw, RoundParams p, SclpOut out) {
+    if (!round_ready(p)) return;
     const int lane = threadIdx.x & 31;
     const int lig = lane & (G - 1);
     const unsigned mask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
@@ -228,6 +255,7 @@ __global__ void __launch_bounds__(kThreads) affinity_warp_hash_kernel(
     i64 count, const i32* __restrict__ list, const O* __restrict__ off, const i32* __restrict__ nbr,
     const W* __restrict__ ew, const W* __restrict__ vw, const i32* __restrict__ clusters,
     const u64* __restrict__ cw, RoundParams p, SclpOut out, u32* err) {
+    if (!round_ready(p)) return;
     constexpr int kSlotBytes = PACKED ? 8 : 12;
     __shared__ __align__(16) unsigned char table_all[kWarps][kMediumSlots * kSlotBytes];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -292,6 +320,7 @@ __global__ void __launch_bounds__(kThreads) affinity_block_hash_kernel(
     i64 count, const i32* __restrict__ list, const O* __restrict__ off, const i32* __restrict__ nbr,
     const W* __restrict__ ew, const W* __restrict__ vw, const i32* __restrict__ clusters,
     const u64* __restrict__ cw, RoundParams p, SclpOut out, u32* err) {
+    if (!round_ready(p)) return;
     extern __shared__ unsigned char smem_raw[];
     auto* slots = reinterpret_cast<unsigned long long*>(smem_raw);   // PACKED
     u64* vals = reinterpret_cast<u64*>(smem_raw);                     // !PACKED
@@ -341,30 +370,130 @@ __global__ void __launch_bounds__(kThreads) affinity_block_hash_kernel(
 // ---------------------------------------------------------------------------
 constexpr int kClasses = 6;
 
-// counts[c] (u32) and edges[c] (u64, sum of degrees) per class.
-template <typename O>
-__global__ void degree_class_kernel(i64 n, const O* off, u64* keys, i32* vals, u32* counts, u64* edges) {
-    __shared__ u32 local[kClasses];
-    __shared__ unsigned long long local_edges[kClasses];
-    if (threadIdx.x < kClasses) { local[threadIdx.x] = 0; local_edges[threadIdx.x] = 0; }
-    __syncthreads();
-    const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (v < n) {
-        const i64 d = static_cast<i64>(off[v + 1]) - off[v];
-        const int c = d == 0 ? 0 : d <= 8 ? 1 : d <= 32 ? 2 : d <= 256 ? 3 : d <= kHubDegree ? 4 : 5;
-        keys[v] = static_cast<u64>(c);
-        vals[v] = static_cast<i32>(v);
-        atomicAdd(&local[c], 1u);
-        atomicAdd(&local_edges[c], static_cast<unsigned long long>(d));
-    }
-    __syncthreads();
-    if (threadIdx.x < kClasses && local[threadIdx.x]) {
-        atomicAdd(&counts[threadIdx.x], local[threadIdx.x]);
-        atomic_add_u64(&edges[threadIdx.x], local_edges[threadIdx.x]);
-    }
+__device__ __forceinline__ int degree_class(i64 d) {
+    return d == 0 ? 0 : d <= 8 ? 1 : d <= 32 ? 2 : d <= 256 ? 3 : d <= kHubDegree ? 4 : 5;
 }
 
+// Where a level's class lists lie: classes 1 and 2 grow from the two ends of
+// one array of n entries, 3 and 4 from the ends of another (0, the isolated
+// vertices, is compacted in vertex order when it is packed; 5 is the hub
+// index).  The lists' order does not matter: every vertex of a list is
+// handled by itself.
+__device__ __forceinline__ i32* class_slot(int c, i64 n, i32* a, i32* b, i64 i) {
+    i32* l = c <= 2 ? a : b;
+    return (c & 1) ? l + i : l + (n - 1 - i);
+}
 
+constexpr int kSetupItems = 8;
+constexpr int kSetupTile = kThreads * kSetupItems;
+
+// Everything a level's aggregation starts from in one pass over its vertices:
+// the degree-class lists (tiles of 2048 consecutive vertices are appended at
+// once, so a list stays nearly in vertex order), singleton clusters and their
+// weights, empty proposals, the total and the largest vertex weight.  It
+// replaced a class sort and five passes (RMAT-20: 10 launches).
+template <typename O, typename W>
+__global__ void __launch_bounds__(kThreads) sclp_setup_kernel(i64 n, const O* __restrict__ off,
+                                                              const W* __restrict__ vw, i32* a, i32* b, i32* clusters,
+                                                              u64* cw, i32* target, u64* demand, u32* crowd,
+                                                              SclpState* state) {
+    __shared__ u32 warp_count[kWarps][kClasses];
+    __shared__ u32 base_sh[kClasses];
+    __shared__ u64 sum_sh[kWarps + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    u64 sum = 0, mx = 0, weightless = 0;
+    for (i64 base = static_cast<i64>(blockIdx.x) * kSetupTile; base < n; base += static_cast<i64>(gridDim.x) * kSetupTile) {
+        int cls[kSetupItems];
+        u32 mine[kClasses] = {};   // of the warp
+        const i64 v0 = base + warp * 32 * kSetupItems + lane;
+#pragma unroll
+        for (int j = 0; j < kSetupItems; ++j) {
+            const i64 v = v0 + j * 32;
+            cls[j] = -1;
+            if (v < n) {
+                cls[j] = degree_class(static_cast<i64>(off[v + 1]) - static_cast<i64>(off[v]));
+                const u64 w = static_cast<u64>(weight_at(vw, v));
+                clusters[v] = static_cast<i32>(v);
+                cw[v] = w;
+                target[v] = kInvalid;
+                demand[v] = 0;
+                crowd[v] = 0;
+                sum += w;
+                mx = w > mx ? w : mx;
+                weightless += w == 0 ? 1 : 0;
+            }
+#pragma unroll
+            for (int c = 0; c < kClasses; ++c) mine[c] += __popc(__ballot_sync(0xffffffffu, cls[j] == c));
+        }
+        if (lane < kClasses) {
+            u32 x = 0;
+#pragma unroll
+            for (int c = 0; c < kClasses; ++c) if (lane == c) x = mine[c];
+            warp_count[warp][lane] = x;
+        }
+        __syncthreads();
+        if (threadIdx.x < kClasses) {
+            u32 run = 0;
+            for (int w = 0; w < kWarps; ++w) { const u32 c = warp_count[w][threadIdx.x]; warp_count[w][threadIdx.x] = run; run += c; }
+            base_sh[threadIdx.x] = run ? atomicAdd(&state->classes[threadIdx.x], run) : 0;
+        }
+        __syncthreads();
+        u32 at[kClasses];
+#pragma unroll
+        for (int c = 0; c < kClasses; ++c) at[c] = base_sh[c] + warp_count[warp][c];
+#pragma unroll
+        for (int j = 0; j < kSetupItems; ++j) {
+#pragma unroll
+            for (int c = 1; c <= 4; ++c) {
+                const unsigned m = __ballot_sync(0xffffffffu, cls[j] == c);
+                if (cls[j] == c)
+                    *class_slot(c, n, a, b, static_cast<i64>(at[c]) + __popc(m & lanemask_lt())) =
+                        static_cast<i32>(v0 + j * 32);
+                at[c] += __popc(m);
+            }
+        }
+        __syncthreads();   // the shared counts are free again
+    }
+    sum = block_sum(sum, sum_sh);
+    mx = warp_max(mx);
+    if (lane == 0 && mx) atomic_max_u64(&state->max, mx);
+    if (threadIdx.x == 0 && sum) atomic_add_u64(&state->total, sum);
+    weightless = warp_sum(weightless);
+    if (lane == 0 && weightless) atomic_add_u64(&state->weightless, weightless);
+}
+
+// The next round's threshold, or the end of the rounds
+// (src/coarsen.cu:1305-1330); one thread.
+__global__ void round_begin_kernel(i64 n, int round, SclpState* s) {
+    if (round == 0) { s->clusters = static_cast<u64>(n); s->done = 0; s->rounds = 0; }
+    if (s->done) return;
+    const i64 clusters = static_cast<i64>(s->clusters);
+    if (static_cast<double>(clusters) <= 0.60 * static_cast<double>(n)) { s->done = 1; return; }
+    const i64 desired = (n + 1) / 2;
+    const i64 removable = clusters > desired ? clusters - desired : 0;
+    const double fraction = fmin(0.50, static_cast<double>(removable) / static_cast<double>(clusters));
+    s->threshold = static_cast<u32>(fraction * 4294967296.0);
+    s->fraction[round] = fraction;
+    s->rounds = round + 1;
+    s->contested = s->segments = s->big = s->giants = 0;
+    s->segment_items = 0;
+}
+
+struct IsIsolated {
+    const void* off;
+    int wide;
+    __device__ i64 operator()(i64 v) const {
+        if (wide) { const i64* o = static_cast<const i64*>(off); return o[v + 1] == o[v] ? 1 : 0; }
+        const i32* o = static_cast<const i32*>(off);
+        return o[v + 1] == o[v] ? 1 : 0;
+    }
+};
+
+template <typename O>
+__global__ void compact_isolated_kernel(i64 n, const O* __restrict__ off, const i64* __restrict__ pos, i32* list) {
+    const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (v < n && off[v + 1] == off[v]) list[pos[v]] = static_cast<i32>(v);
+}
 
 // Level statistics: total / maximum vertex weight and degree-class counts.
 template <typename W>
@@ -386,33 +515,21 @@ __global__ void weight_stats_kernel(i64 n, const W* vw, u64* out /* [0]=sum [1]=
 // Admission (src/coarsen.cu:1086-1121,1334-1370,652-680)
 // cls: 0 = no move, 1 = accept, 2 = contested (target over-subscribed)
 // ---------------------------------------------------------------------------
-__global__ void admission_classify_kernel(i64 n, const i32* target, const u64* demand, const u64* cw, u64 cap,
-                                          const u64* gain, unsigned char* cls, u64* gmax) {
-    const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    const i32 t = target[v];
-    unsigned char c = 0;
-    if (t != kInvalid) {
-        const u64 base = cw[t];
-        if (base <= cap) {
-            if (demand[t] <= cap - base) {
-                c = 1;
-            } else {
-                c = 2;
-                atomic_max_u64(gmax, gain[v]);
-            }
-        }
-    }
-    cls[v] = c;
-}
-
 // Two-hop candidates: every valid favourite is "contested" (needs order).
 __global__ void favorite_classify_kernel(i64 n, const i32* target, const u64* gain, unsigned char* cls, u64* gmax) {
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v >= n) return;
     const bool ok = target[v] != kInvalid;
     cls[v] = ok ? 2 : 0;
-    if (ok) atomic_max_u64(gmax, gain[v]);
+    // one atomic per warp (all lanes of a full warp are here or none but the last warp's)
+    u64 g = ok ? gain[v] : 0;
+    const unsigned m = __activemask();
+    if (m == 0xffffffffu) {
+        g = warp_max(g);
+        if ((threadIdx.x & 31) == 0 && g) atomic_max_u64(gmax, g);
+    } else if (g) {
+        atomic_max_u64(gmax, g);
+    }
 }
 
 struct IsClass2 {
@@ -462,32 +579,6 @@ __global__ void segment_heads_kernel(i64 count, const i32* list, const i32* targ
     if (i >= count) return;
     const i32 t = target[list[i]];
     if (i == 0 || target[list[i - 1]] != t) segbase[t] = store_index ? static_cast<u64>(i) : excl[i];
-}
-
-template <typename W>
-__global__ void contested_accept_kernel(i64 count, const i32* list, const i32* target, const u64* excl,
-                                        const u64* segbase, const u64* cw, const W* vw, u64 cap, unsigned char* cls) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const i32 v = list[i];
-    const i32 t = target[v];
-    const u64 w = static_cast<u64>(weight_at(vw, v));
-    const u64 prefix = excl[i] + w - segbase[t];
-    const u64 base = cw[t];
-    cls[v] = (base <= cap && prefix <= cap - base) ? 1 : 0;
-}
-
-template <typename W>
-__global__ void sclp_commit_kernel(i64 n, const unsigned char* cls, const i32* target, const W* vw, i32* clusters,
-                                   u64* cw) {
-    const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (v >= n || cls[v] != 1) return;
-    const i32 t = target[v];
-    const i32 s = clusters[v];
-    const u64 w = static_cast<u64>(weight_at(vw, v));
-    atomic_add_u64(&cw[s], 0ULL - w);
-    atomic_add_u64(&cw[t], w);
-    clusters[v] = t;
 }
 
 __global__ void count_nonzero_kernel(i64 n, const u64* cw, u64* out) {

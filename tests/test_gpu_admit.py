@@ -1,0 +1,52 @@
+"""Admission to over-subscribed clusters against the oracle: segments of every
+size class (a warp's, a block's, and those narrowed by all blocks first), with
+equal and with varied gains and vertex weights, and vertices of weight zero."""
+import numpy as np
+import pytest
+
+import horkxg_b200 as hb
+import pyoracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def stars(hubs, leaves, weighted, seed):
+    """`hubs` hubs in a ring, each with `leaves` leaves; leaves also form
+    sparse pairs, so that not every gain is the hub's edge."""
+    rng = np.random.default_rng(seed)
+    n = hubs * (leaves + 1)
+    centre = np.arange(hubs) * (leaves + 1)
+    leaf = np.setdiff1d(np.arange(n), centre)
+    a = np.concatenate([centre, leaf, leaf[:-1:7]])
+    b = np.concatenate([np.roll(centre, 1), np.repeat(centre, leaves), leaf[1::7][:len(leaf[:-1:7])]])
+    keep = a != b
+    a, b = a[keep], b[keep]
+    key = np.unique(np.minimum(a, b) * n + np.maximum(a, b))
+    a, b = key // n, key % n
+    w = rng.integers(1, 40, len(a)) if weighted else np.ones(len(a), np.int64)
+    src, dst, ew = np.concatenate([a, b]), np.concatenate([b, a]), np.concatenate([w, w])
+    order = np.lexsort((dst, src))
+    off = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(src, minlength=n), out=off[1:])
+    vw = rng.integers(1, 5, n).astype(np.uint64) if weighted else None
+    return off, dst[order], (ew[order].astype(np.uint64) if weighted else None), vw
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("hubs,leaves", [(50, 12), (40, 70), (20, 400), (6, 9000), (2, 20000), (1, 30000)])
+def test_admission_matches_oracle(ctx, hubs, leaves, weighted):
+    off, nbr, ew, vw = stars(hubs, leaves, weighted, hubs + leaves)
+    g, og = hb.HostGraph(off, nbr, ew, vw, index64=True), O.Graph(off, nbr, ew, vw)
+    for parts, beta, seed, level in ((2, 2, 0, 0), (4, 8, 3, 1), (2, 64, 1, 0)):
+        mp, cn, cap = ctx.aggregate(g, parts, seed, level, beta, True)
+        omp, ocn, ocap = O.aggregate(og, parts, seed, level, beta, True)
+        assert (cn, cap) == (ocn, ocap) and np.array_equal(mp, omp)
+
+
+def test_whole_coarsening_with_stars(ctx):
+    off, nbr, _, _ = stars(2, 20000, False, 5)
+    levels = ctx.coarsen(hb.HostGraph(off, nbr, index64=True), parts=4)
+    olevels, omaps = O.coarsen(O.Graph(off, nbr), 4, 0, -1, True)
+    assert len(levels) == len(olevels)
+    for (coff, cnbr, cew, cvw, cmap), og in zip(levels, olevels):
+        assert np.array_equal(coff, og.off) and np.array_equal(cnbr, og.nbr) and np.array_equal(cew, og.ew)
