@@ -28,33 +28,53 @@ __device__ __forceinline__ bool is_hub(const O* off, i64 v) {
     return static_cast<i64>(off[v + 1]) - static_cast<i64>(off[v]) > kHubThreshold;
 }
 
+// Counts the hubs into *count and, with `ids`, lists them in any order.
 template <typename O>
-struct HubFlag {
-    const O* off;
-    __device__ i64 operator()(i64 v) const { return is_hub(off, v) ? 1 : 0; }
-};
+__global__ void hub_collect_kernel(i64 n, const O* __restrict__ off, u64* ids, i64* count) {
+    u64 found = 0;
+    const i64 end = (n + 31) / 32 * 32;   // whole warps for the append
+    for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < end;
+         v += static_cast<i64>(gridDim.x) * blockDim.x) {
+        const bool hub = v < n && is_hub(off, v);
+        if (ids) {
+            const u64 slot = warp_append(hub, reinterpret_cast<u64*>(count));
+            if (hub) ids[slot] = static_cast<u64>(v);
+        } else {
+            found += hub ? 1 : 0;
+        }
+    }
+    if (ids) return;
+    found = warp_sum(found);
+    if ((threadIdx.x & 31) == 0 && found) atomic_add_u64(reinterpret_cast<u64*>(count), found);
+}
 
+// Chunks of the hubs in list order.
 template <typename O>
 struct HubChunkCount {
+    const u64* ids;
     const O* off;
-    __device__ i64 operator()(i64 v) const {
-        const i64 d = static_cast<i64>(off[v + 1]) - static_cast<i64>(off[v]);
-        return d > kHubThreshold ? (d + kChunkEdges - 1) / kChunkEdges : 0;
+    i64 count;
+    __device__ i64 operator()(i64 i) const {
+        if (i >= count) return 0;
+        const i64 v = static_cast<i64>(ids[i]);
+        return (static_cast<i64>(off[v + 1]) - static_cast<i64>(off[v]) + kChunkEdges - 1) / kChunkEdges;
     }
 };
 
+// A warp per hub.
 template <typename O>
-__global__ void hub_fill_kernel(i64 n, const O* off, const i64* hub_pos, const i64* chunk_pos, i32* hubs,
-                                Chunk* chunks, i64* chunk_begin) {
-    const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (v >= n || !is_hub(off, v)) return;
-    const i64 h = hub_pos[v];
-    hubs[h] = static_cast<i32>(v);
-    chunk_begin[h] = chunk_pos[v];
-    const i64 b = off[v], e = off[v + 1];
-    i64 c = chunk_pos[v];
-    for (i64 s = b; s < e; s += kChunkEdges, ++c)
-        chunks[c] = {static_cast<i32>(v), static_cast<i32>(h), s, s + kChunkEdges < e ? s + kChunkEdges : e};
+__global__ void hub_fill_kernel(i64 count, const u64* __restrict__ ids, const O* __restrict__ off,
+                                const i64* __restrict__ chunk_begin, i32* hubs, Chunk* chunks) {
+    for (i64 h = blockIdx.x; h < count; h += gridDim.x) {
+        const i64 v = static_cast<i64>(ids[h]);
+        if (threadIdx.x == 0) hubs[h] = static_cast<i32>(v);
+        const i64 b = off[v], e = off[v + 1];
+        for (i64 c = threadIdx.x; b + c * kChunkEdges < e; c += blockDim.x) {
+            const i64 s = b + c * kChunkEdges;
+            chunks[chunk_begin[h] + c] = {static_cast<i32>(v), static_cast<i32>(h), s,
+                                          s + kChunkEdges < e ? s + kChunkEdges : e};
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------

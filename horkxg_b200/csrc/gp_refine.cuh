@@ -67,22 +67,46 @@ struct alignas(16) PropRec {
 __device__ __forceinline__ void cache_add(u32* p, u64 v) { atomicAdd(p, static_cast<u32>(v)); }
 __device__ __forceinline__ void cache_add(u64* p, u64 v) { atomic_add_u64(p, v); }
 
-// Exact directed cut, warp per vertex, one atomic per block
-// (refine_cut_kernel, src/refine.cu:52-87).
+// Exact directed cut, one atomic per block (refine_cut_kernel,
+// src/refine.cu:52-87).  A warp takes four consecutive rows at a time: rows of
+// at most 32 entries are walked by 8 lanes each, longer ones (up to the hub
+// degree) by the whole warp one after the other.  Bound by the label gathers;
+// with a warp per row a mesh's rows of 4-7 entries left most lanes idle
+// (grid of 10^6 vertices 128 -> 45 us, 320^3 grid 606 -> 378 us a launch).
 template <typename O, typename W>
 __global__ void __launch_bounds__(kThreads) cut_kernel(i64 n, const O* __restrict__ off, const i32* __restrict__ nbr,
                                                        const W* __restrict__ ew, const i32* __restrict__ labels,
                                                        u64* out) {
     __shared__ u64 sh[kWarps + 1];
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, grp = lane >> 3, gl = lane & 7;
     u64 local = 0;
     const i64 warps_total = static_cast<i64>(gridDim.x) * kWarps;
-    for (i64 v = static_cast<i64>(blockIdx.x) * kWarps + (threadIdx.x >> 5); v < n; v += warps_total) {
-        const i64 b = off[v], end = off[v + 1];
-        if (end - b > kHubDegree) continue;   // hub rows: chunked kernel
-        const i32 s = labels[v];
-        for (i64 e = b + lane; e < end; e += 32)
-            if (labels[nbr[e]] != s) local += static_cast<u64>(weight_at(ew, e));
+    for (i64 q = static_cast<i64>(blockIdx.x) * kWarps + (threadIdx.x >> 5); q * 4 < n; q += warps_total) {
+        const i64 v = q * 4 + grp;
+        i64 b = 0, deg = 0;
+        i32 s = 0;
+        if (v < n) {
+            b = static_cast<i64>(off[v]);
+            deg = static_cast<i64>(off[v + 1]) - b;
+            s = labels[v];
+        }
+        if (deg <= 32) {
+            i32 u[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) u[r] = gl + 8 * r < deg ? nbr[b + gl + 8 * r] : -1;
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (u[r] >= 0 && labels[u[r]] != s) local += static_cast<u64>(weight_at(ew, b + gl + 8 * r));
+        }
+        unsigned longs = __ballot_sync(0xffffffffu, gl == 0 && deg > 32 && deg <= kHubDegree);
+        while (longs) {
+            const int src = __ffs(longs) - 1;
+            longs &= longs - 1;
+            const i64 lb = __shfl_sync(0xffffffffu, b, src), ld = __shfl_sync(0xffffffffu, deg, src);
+            const i32 ls = __shfl_sync(0xffffffffu, s, src);
+            for (i64 e = lb + lane; e < lb + ld; e += 32)
+                if (labels[nbr[e]] != ls) local += static_cast<u64>(weight_at(ew, e));
+        }
     }
     local = block_sum(local, sh);
     if (threadIdx.x == 0 && local) atomic_add_u64(out, local);
