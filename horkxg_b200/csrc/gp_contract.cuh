@@ -296,6 +296,128 @@ __global__ void __launch_bounds__(kThreads) segment_warp_radix_kernel(i64 rows, 
     if (lane == 0) row_len[c] = u;
 }
 
+// Sorts `len` (<= 16 * kThreads) entries of (k0, w0) by key into (k1, w1),
+// leaving the sentinels out; returns the entries kept, or -1 when the keys
+// crowd so much that the caller should radix sort them.  The keys' range is
+// cut into about as many equal buckets as there are entries: placing an entry
+// takes two shared atomics, and a bucket then holds one or two entries, which
+// one thread orders (a crowded bucket is ranked by a warp).  A radix sort
+// takes three or four passes of ten barriers with a match per key.  `cnt`
+// holds kBuckets + 1 words.
+constexpr int kBuckets = 2048;
+constexpr int kBucketThread = 12;      // ordered by one thread
+constexpr int kBucketWarp = 512;       // ranked by one warp
+
+struct BucketShared {
+    u32 lo, hi, crowded, largest;
+    i64 scan_tmp[kWarps + 1];
+    u32 list[64];
+};
+
+template <typename W>
+__device__ int block_bucket_sort(const u32* k0, const W* w0, u32* k1, W* w1, int len, u32 sentinel, u32* cnt,
+                                 BucketShared& sh) {
+    constexpr int kItems = 16;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int buckets = 64;
+    while (buckets < len && buckets < kBuckets) buckets <<= 1;
+    if (threadIdx.x == 0) { sh.lo = ~0u; sh.hi = 0; sh.crowded = 0; sh.largest = 0; }
+    for (int b = threadIdx.x; b <= buckets; b += kThreads) cnt[b] = 0;
+    __syncthreads();
+    u32 lo = ~0u, hi = 0;
+    for (int i = threadIdx.x; i < len; i += kThreads) {
+        const u32 k = k0[i];
+        if (k != sentinel) { lo = min(lo, k); hi = max(hi, k); }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0 && lo <= hi) { atomicMin(&sh.lo, lo); atomicMax(&sh.hi, hi); }
+    __syncthreads();
+    lo = sh.lo;
+    hi = sh.hi;
+    if (lo > hi) return 0;   // sentinels only; uniform over the block
+    const u64 scale = (static_cast<u64>(buckets) << 32) / (static_cast<u64>(hi - lo) + 1);
+    auto bucket_of = [&](u32 k) { return static_cast<int>((static_cast<u64>(k - lo) * scale) >> 32); };
+    u32 place[kItems];
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+        const int i = threadIdx.x + j * kThreads;
+        if (i >= len) break;
+        const u32 k = k0[i];
+        place[j] = k != sentinel ? atomicAdd(&cnt[bucket_of(k)], 1u) : ~0u;
+    }
+    __syncthreads();
+    // bucket starts, each thread over neighbouring buckets
+    const int per = (buckets + kThreads - 1) / kThreads;
+    u32 sum = 0;
+    for (int q = 0; q < per; ++q) {
+        const int b = threadIdx.x * per + q;
+        if (b < buckets) sum += cnt[b];
+    }
+    i64 total;
+    u32 run = static_cast<u32>(block_exclusive_sum<i64>(sum, sh.scan_tmp, &total));
+    for (int q = 0; q < per; ++q) {
+        const int b = threadIdx.x * per + q;
+        if (b >= buckets) break;
+        const u32 c = cnt[b];
+        cnt[b] = run;
+        run += c;
+        if (c > kBucketThread) {
+            const u32 at = atomicAdd(&sh.crowded, 1u);
+            if (at < 64) sh.list[at] = static_cast<u32>(b);
+            atomicMax(&sh.largest, c);
+        }
+    }
+    if (threadIdx.x == 0) cnt[buckets] = static_cast<u32>(total);
+    __syncthreads();
+    if (sh.crowded > 64 || sh.largest > kBucketWarp) return -1;
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+        const int i = threadIdx.x + j * kThreads;
+        if (i >= len) break;
+        if (place[j] == ~0u) continue;
+        const u32 k = k0[i];
+        const u32 at = cnt[bucket_of(k)] + place[j];
+        k1[at] = k;
+        w1[at] = w0[i];
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < buckets; b += kThreads) {
+        const u32 s = cnt[b], e = cnt[b + 1];
+        if (e - s < 2 || e - s > kBucketThread) continue;
+        for (u32 i = s + 1; i < e; ++i) {
+            const u32 k = k1[i];
+            const W w = w1[i];
+            u32 x = i;
+            for (; x > s && k1[x - 1] > k; --x) { k1[x] = k1[x - 1]; w1[x] = w1[x - 1]; }
+            k1[x] = k;
+            w1[x] = w;
+        }
+    }
+    // crowded buckets: each entry's rank by comparison with the others, through
+    // the source buffers, whose entries are all placed
+    u32* kt = const_cast<u32*>(k0);
+    W* wt = const_cast<W*>(w0);
+    const u32 crowded = sh.crowded;
+    for (u32 q = warp; q < crowded; q += kWarps) {
+        const u32 b = sh.list[q], s = cnt[b], e = cnt[b + 1];
+        for (u32 i = s + lane; i < e; i += 32) {
+            const u32 k = k1[i];
+            u32 rank = s;
+            for (u32 x = s; x < e; ++x) {
+                const u32 o = k1[x];
+                rank += o < k || (o == k && x < i) ? 1 : 0;
+            }
+            kt[rank] = k;
+            wt[rank] = w1[i];
+        }
+        __syncwarp();
+        for (u32 i = s + lane; i < e; i += 32) { k1[i] = kt[i]; w1[i] = wt[i]; }
+    }
+    __syncthreads();
+    return static_cast<int>(total);
+}
+
 // Rows with kWarpSegCap+1..seg_smem_capacity entries: block per row, radix
 // sort in a shared-memory buffer of `cap` entries (the class's bound).
 template <typename W>
@@ -307,8 +429,10 @@ __global__ void __launch_bounds__(kThreads) segment_smem_kernel(i64 rows, const 
     W* w1 = w0 + cap;
     u32* k0 = reinterpret_cast<u32*>(w1 + cap);
     u32* k1 = k0 + cap;
-    __shared__ RankShared rank_sh;
+    __shared__ RankShared rank_sh;   // or the bucket counts
     __shared__ RunShared<W> run_sh;
+    __shared__ BucketShared bucket_sh;
+    static_assert(sizeof(RankShared) >= (kBuckets + 1) * sizeof(u32), "the bucket counts share the ranking scratch");
     const i64 r = blockIdx.x;
     if (r >= rows) return;
     const i32 c = list[r];
@@ -338,8 +462,16 @@ __global__ void __launch_bounds__(kThreads) segment_smem_kernel(i64 rows, const 
     }
     for (i64 i = head + 4 * groups + threadIdx.x; i < len; i += kThreads) { k0[i] = src_k[i]; w0[i] = src_w[i]; }
     __syncthreads();
-    block_radix_sort_segment(k0, w0, k1, w1, len, 0, key_bits, rank_sh);
-    const i64 u = block_reduce_runs(k0, w0, len, sentinel, tgt + s, wt + s, run_sh);
+    const int kept = block_bucket_sort(k0, w0, k1, w1, static_cast<int>(len), sentinel,
+                                       reinterpret_cast<u32*>(&rank_sh), bucket_sh);
+    i64 u;
+    if (kept >= 0) {
+        u = block_reduce_runs(k1, w1, static_cast<i64>(kept), sentinel, tgt + s, wt + s, run_sh);
+    } else {
+        __syncthreads();
+        block_radix_sort_segment(k0, w0, k1, w1, len, 0, key_bits, rank_sh);
+        u = block_reduce_runs(k0, w0, len, sentinel, tgt + s, wt + s, run_sh);
+    }
     if (threadIdx.x == 0) row_len[c] = u;
 }
 

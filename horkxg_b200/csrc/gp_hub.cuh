@@ -169,7 +169,8 @@ __global__ void __launch_bounds__(kThreads) hub_insert_kernel(
     const i32* __restrict__ clusters, RoundParams p, const i64* __restrict__ table_off, S* table, u32* err) {
     if (!round_ready(p)) return;
     const Chunk ch = chunks[blockIdx.x];
-    if (role_blocked(p.identity ? ch.v : clusters[ch.v], p)) return;   // no proposal: nothing to count
+    const i32 source = p.identity ? ch.v : clusters[ch.v];
+    if (role_blocked(source, p)) return;   // no proposal: nothing to count
     const int lane = threadIdx.x & 31;
     const i64 t0 = table_off[ch.hub];
     const u32 size = static_cast<u32>(table_off[ch.hub + 1] - t0);
@@ -184,6 +185,7 @@ __global__ void __launch_bounds__(kThreads) hub_insert_kernel(
             if (u != ch.v) {
                 c = p.identity ? u : clusters[u];
                 w = static_cast<u64>(weight_at(ew, e));
+                if (!may_count(c, source, p)) c = -1;
             }
         }
     };
@@ -267,6 +269,7 @@ __global__ void __launch_bounds__(THREADS) hub_smem_kernel(
             if (u != v) {
                 c = clusters[u];
                 w = static_cast<u64>(weight_at(ew, e));
+                if (!may_count(c, source, p)) c = -1;
             }
         }
         // Every lane inserts its own edge: the 32 neighbours of one step

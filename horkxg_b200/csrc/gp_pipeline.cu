@@ -1536,8 +1536,8 @@ gp_refine_stats refine_level(Device& d, const DGraph<T>& g, RefineWork& w, i32* 
                       static_cast<double>(n - hubs.count) * k * sizeof(C);
         d.prof_bytes("build_cache_kernel", build_bytes);
     }
-    launch(d, "build_cache_kernel", build_cache_kernel<O, W, C>, stride_grid(d, n * 8), kThreads, 0, n, off, nbr, ew,
-           labels, k, cache);
+    launch(d, "build_cache_kernel", build_cache_kernel<false, O, W, C>, stride_grid(d, n * 8), kThreads, 0, n, off, nbr,
+           ew, labels, k, cache, static_cast<u64*>(nullptr));
     Buf<long long> hub_corr;
     if (hubs.count) {
         launch(d, "zero_hub_rows_kernel", zero_hub_rows_kernel<C>, blocks_for(hubs.count * k, kThreads), kThreads, 0,
@@ -1568,24 +1568,30 @@ gp_refine_stats refine_level(Device& d, const DGraph<T>& g, RefineWork& w, i32* 
         GP_LAUNCH();
         max_edge_weight = w.scratch.get() + 7;
     }
-    struct Stats { RefineCounters c; u64 pw[32]; };
+    struct Stats { RefineCounters c; u64 pw[32]; u64 cut; };
     static_assert(sizeof(Stats) <= Device::kPinnedBytes, "stats fit the pinned staging buffer");
+    // rebuilds the cache and counts the cut (directed, into w.scratch[0]) from it
     auto build_cache = [&]() {
         d.prof_bytes("build_cache_kernel", build_bytes);
-        launch(d, "build_cache_kernel", build_cache_kernel<O, W, C>, stride_grid(d, n * 8), kThreads, 0, n, off, nbr,
-               ew, labels, k, cache);
+        u64* cut = w.scratch.get();
+        GP_CUDA(cudaMemsetAsync(cut, 0, sizeof(u64), d.stream));
+        launch(d, "build_cache_kernel", build_cache_kernel<true, O, W, C>, stride_grid(d, n * 8), kThreads, 0, n, off,
+               nbr, ew, labels, k, cache, cut);
         if (hubs.count) {
             launch(d, "zero_hub_rows_kernel", zero_hub_rows_kernel<C>, blocks_for(hubs.count * k, kThreads), kThreads,
                    0, hubs.count, hubs.list.get(), k, cache);
             launch(d, "hub_build_cache_kernel", hub_build_cache_kernel<W, C>, static_cast<int>(hubs.chunks), kThreads,
                    0, hubs.chunk.get(), nbr, ew, labels, k, cache);
+            launch(d, "hub_cache_cut_kernel", hub_cache_cut_kernel<C>, stride_grid(d, hubs.count * k), kThreads, 0,
+                   hubs.count, hubs.list.get(), labels, k, cache, cut);
         }
     };
     // Applies the listed movers.  When the LP movers' edges outnumber m/8,
     // updating the affinity cache edge by edge (two random atomics per edge)
-    // costs more than rebuilding it with one streaming pass, and the cut is
-    // then recounted exactly instead of being updated by the per-edge deltas;
-    // both routes give the same cache and the same cut.  (Rebalance moves
+    // costs more than rebuilding it with one streaming pass, which also counts
+    // the cut exactly (its rows hold the connections to other parts) instead
+    // of updating it by the per-edge deltas; both routes give the same cache
+    // and the same cut.  (Rebalance moves
     // stay edge by edge: measured, the rebuild plus recount does not pay
     // there.)  The kernels read the mover count from the device, so a
     // rebalance apply needs no round trip before its launch: its grids are
@@ -1639,6 +1645,8 @@ gp_refine_stats refine_level(Device& d, const DGraph<T>& g, RefineWork& w, i32* 
         Stats h;
         {
             auto* staged = reinterpret_cast<Stats*>(d.pinned);
+            if (rebuild)
+                GP_CUDA(cudaMemcpyAsync(&staged->cut, w.scratch.get(), sizeof(u64), cudaMemcpyDeviceToHost, d.stream));
             GP_CUDA(cudaMemcpyAsync(&staged->c, ctr, sizeof(RefineCounters), cudaMemcpyDeviceToHost, d.stream));
             GP_CUDA(cudaMemcpyAsync(staged->pw, pw, k * sizeof(u64), cudaMemcpyDeviceToHost, d.stream));
             d.sync();
@@ -1660,8 +1668,12 @@ gp_refine_stats refine_level(Device& d, const DGraph<T>& g, RefineWork& w, i32* 
                                                      static_cast<double>(h.c.hub_chunks) * 8 +
                                                      static_cast<double>(h.c.hub_edges) * per_edge);
         }
-        if (rebuild) current_cut = undirected_cut(d, g, labels, w.scratch.get());
-        else apply_delta(h.c.delta);
+        if (rebuild) {
+            if (h.cut & 1ULL) fail(GP_ERUNTIME, "refinement cut is not symmetric");
+            current_cut = h.cut / 2;
+        } else {
+            apply_delta(h.c.delta);
+        }
         std::copy(h.pw, h.pw + k, host_pw.begin());
         st.accepted += static_cast<u64>(h.c.movers);
         if (verify) {

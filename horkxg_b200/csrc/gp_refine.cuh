@@ -181,11 +181,14 @@ __device__ __forceinline__ void load_row(const C* row, int k, C (&vals)[32]) {
 // The four cache rows, consecutive in memory, are then stored by the whole
 // warp in one coalesced pass.  Hub rows are left to the chunked kernel
 // (zero_hub_rows_kernel clears them after this one).
-// `rows`: one accumulator per warp of the block.
-template <typename O, typename W, typename C>
-__device__ __forceinline__ void build_cache_rows(i64 n, const O* __restrict__ off, const i32* __restrict__ nbr,
-                                                 const W* __restrict__ ew, const i32* labels, int k, C* cache,
-                                                 u64 (*rows)[4][32]) {
+// `rows`: one accumulator per warp of the block.  With CUT every lane's share
+// of the rows' connections to other parts is returned: summed over all rows
+// the directed cut, without a pass of its own over the edges.
+template <bool CUT, typename O, typename W, typename C>
+__device__ __forceinline__ u64 build_cache_rows(i64 n, const O* __restrict__ off, const i32* __restrict__ nbr,
+                                                const W* __restrict__ ew, const i32* labels, int k, C* cache,
+                                                u64 (*rows)[4][32]) {
+    u64 cut = 0;
     u32 (*rows32)[4][32] = reinterpret_cast<u32 (*)[4][32]>(&rows[0][0][0]);   // C = u32: 32-bit accumulators
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane >> 3, gl = lane & 7;
     const int block_warps = static_cast<int>(blockDim.x >> 5);
@@ -253,23 +256,52 @@ __device__ __forceinline__ void build_cache_rows(i64 n, const O* __restrict__ of
         const int nrows = static_cast<int>(n - first < 4 ? n - first : 4);
         const unsigned hub_rows = __ballot_sync(0xffffffffu, gl == 0 && deg > kHubDegree);
         C* dst = cache + first * k;
-        for (int i = lane; i < nrows * k; i += 32) {
+        const i32 own = CUT && v < n ? labels[v] : 0;
+        for (int i0 = 0; i0 < nrows * k; i0 += 32) {
+            const int i = i0 + lane;
             const int row = i / k;
-            if (!(hub_rows & (1u << (row * 8)))) {
-                if constexpr (sizeof(C) == 4) dst[i] = static_cast<C>(rows32[warp][row][i - row * k]);
-                else dst[i] = static_cast<C>(rows[warp][row][i - row * k]);
+            i32 part = 0;
+            if constexpr (CUT) part = __shfl_sync(0xffffffffu, own, (row & 3) * 8);
+            if (i < nrows * k && !(hub_rows & (1u << (row * 8)))) {
+                C value;
+                if constexpr (sizeof(C) == 4) value = static_cast<C>(rows32[warp][row][i - row * k]);
+                else value = static_cast<C>(rows[warp][row][i - row * k]);
+                dst[i] = value;
+                if (CUT && i - row * k != part) cut += static_cast<u64>(value);
             }
         }
         __syncwarp();
     }
+    return cut;
 }
 
-template <typename O, typename W, typename C>
+template <bool CUT, typename O, typename W, typename C>
 __global__ void __launch_bounds__(kThreads) build_cache_kernel(i64 n, const O* __restrict__ off,
                                                                const i32* __restrict__ nbr, const W* __restrict__ ew,
-                                                               const i32* __restrict__ labels, int k, C* cache) {
+                                                               const i32* __restrict__ labels, int k, C* cache,
+                                                               u64* directed_cut) {
     __shared__ u64 rows[kWarps][4][32];
-    build_cache_rows(n, off, nbr, ew, labels, k, cache, rows);
+    u64 cut = build_cache_rows<CUT>(n, off, nbr, ew, labels, k, cache, rows);
+    if constexpr (CUT) {
+        cut = warp_sum(cut);
+        if ((threadIdx.x & 31) == 0 && cut) atomic_add_u64(directed_cut, cut);
+    }
+}
+
+// The hub rows' share of the directed cut, from their finished cache rows.
+template <typename C>
+__global__ void __launch_bounds__(kThreads) hub_cache_cut_kernel(i64 hubs, const i32* __restrict__ hub_list,
+                                                                 const i32* __restrict__ labels, int k,
+                                                                 const C* __restrict__ cache, u64* directed_cut) {
+    u64 cut = 0;
+    for (i64 i = static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x; i < hubs * k; i += static_cast<i64>(gridDim.x) * kThreads) {
+        const i64 h = i / k;
+        const int p = static_cast<int>(i - h * k);
+        const i64 v = hub_list[h];
+        if (p != labels[v]) cut += static_cast<u64>(cache[v * k + p]);
+    }
+    cut = warp_sum(cut);
+    if ((threadIdx.x & 31) == 0 && cut) atomic_add_u64(directed_cut, cut);
 }
 
 // The LP filter of refine_incremental.cuh:332-333, from the level's maximum

@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kSmallThreads) refine_small_kernel(const Small
     if (!a.resume) {
         for (i64 v = tid; v < n; v += threads) { a.locks[v] = 0; a.flags[v] = 0; }
         for (i64 i = tid; i < static_cast<i64>(k) * kBalWidth; i += threads) a.counts[i] = 0;
-        build_cache_rows(n, a.off, a.nbr, a.ew, a.labels, k, a.cache, sh.rows);
+        build_cache_rows<false>(n, a.off, a.nbr, a.ew, a.labels, k, a.cache, sh.rows);
         if (a.ew) {
             u64 mx = 0;
             for (i64 e = tid; e < a.m; e += threads) {

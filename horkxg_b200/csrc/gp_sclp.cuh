@@ -88,6 +88,15 @@ __device__ __forceinline__ bool role_blocked(i32 source, const RoundParams& p) {
     return p.filter && !is_mover(source, p);
 }
 
+// Whether an edge into cluster c can matter to a vertex of cluster `source`:
+// with role filtering a mover's cluster is never a candidate, so its sum is
+// needed only when it is the vertex's own.  Between a third and a half of the
+// clusters are movers in a round; leaving their edges out of the hash tables
+// saves the inserts and shortens the probes.
+__device__ __forceinline__ bool may_count(i32 c, i32 source, const RoundParams& p) {
+    return !p.filter || c == source || !is_mover(c, p);
+}
+
 // sclp_better_candidate, src/coarsen.cu:224-229
 __device__ __forceinline__ bool better(u64 a, u64 ta, u64 b, u64 tb) {
     return a > b || (a == b && a != 0 && ta > tb);
@@ -240,9 +249,8 @@ __device__ __forceinline__ void slot_candidate(i32 key, u64 conn, u32 v, i32 sou
     if (key < 0) return;
     if (key == source) { current = conn; return; }
     // a sum below the running best (or zero) never wins, whatever its tie
-    // key: skip the mover test and the tie hash for it
+    // key: skip the tie hash for it (movers' clusters are not in the table)
     if (conn < best || conn == 0) return;
-    if (p.filter && is_mover(key, p)) return;
     const u64 t = tie_key(v, key, p.tie_salt);
     if (better(conn, t, best, tie)) { best = conn; tie = t; }
 }
@@ -279,6 +287,7 @@ __global__ void __launch_bounds__(kThreads) affinity_warp_hash_kernel(
         const i32 u = nbr[e];
         if (u == v) continue;
         const i32 c = p.identity ? u : clusters[u];
+        if (!may_count(c, source, p)) continue;
         const u64 w = static_cast<u64>(weight_at(ew, e));
         if constexpr (PACKED) packed_insert(slots, kMediumSlots - 1, c, w, err);
         else table_insert(keys, vals, kMediumSlots - 1, c, w, err);
@@ -345,6 +354,7 @@ __global__ void __launch_bounds__(kThreads) affinity_block_hash_kernel(
         const i32 u = nbr[e];
         if (u == v) continue;
         const i32 c = p.identity ? u : clusters[u];
+        if (!may_count(c, source, p)) continue;
         const u64 w = static_cast<u64>(weight_at(ew, e));
         if constexpr (PACKED) packed_insert(slots, static_cast<u32>(nslots - 1), c, w, err);
         else table_insert(keys, vals, static_cast<u32>(nslots - 1), c, w, err);
