@@ -16,6 +16,8 @@
 // 10^6 six times took longer than the sort: RMAT-24 +70 ms).
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "gp_refine.cuh"
 #include "gp_sclp.cuh"
 
@@ -25,13 +27,10 @@ constexpr u32 kWarpSegment = 32;
 
 // cls: 0 = no move, 1 = accept, 2 = decided by its segment.  slot[v]: the
 // proposal's place in its target's segment.
-__global__ void __launch_bounds__(kThreads) admit_classify_kernel(i64 n, const i32* __restrict__ target,
-                                                                  const u64* __restrict__ demand,
-                                                                  const u64* __restrict__ cw, u64 cap,
-                                                                  unsigned char* cls, u32* crowd, u32* slot, i32* list,
-                                                                  SclpState* state) {
-    if (state->done) return;
-    const i64 v = static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x;
+// One vertex per lane, all 32 lanes of a warp.
+__device__ __forceinline__ void admit_classify(i64 v, i64 n, const i32* target, const u64* demand, const u64* cw,
+                                               u64 cap, unsigned char* cls, u32* crowd, u32* slot, i32* list,
+                                               SclpState* state) {
     bool contested = false;
     i32 to = -1;
     if (v < n) {
@@ -65,16 +64,21 @@ __global__ void __launch_bounds__(kThreads) admit_classify_kernel(i64 n, const i
     if (contested) list[base + __popc(m & lanemask_lt())] = static_cast<i32>(v);
 }
 
+__global__ void __launch_bounds__(kThreads) admit_classify_kernel(i64 n, const i32* __restrict__ target,
+                                                                  const u64* __restrict__ demand,
+                                                                  const u64* __restrict__ cw, u64 cap,
+                                                                  unsigned char* cls, u32* crowd, u32* slot, i32* list,
+                                                                  SclpState* state) {
+    if (state->done) return;
+    admit_classify(static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x, n, target, demand, cw, cap, cls, crowd, slot,
+                   list, state);
+}
+
 // The first proposal of every contested target reserves its segment;
 // `demand` of the target then holds the segment's start.
-__global__ void __launch_bounds__(kThreads) admit_reserve_kernel(const i32* __restrict__ list,
-                                                                 const i32* __restrict__ target,
-                                                                 const u32* __restrict__ slot,
-                                                                 const u32* __restrict__ crowd, u64* demand,
-                                                                 i32* segments, SclpState* state) {
-    if (state->done) return;
-    const i64 count = state->contested;
-    for (i64 base = static_cast<i64>(blockIdx.x) * kThreads; base < count; base += static_cast<i64>(gridDim.x) * kThreads) {
+__device__ __forceinline__ void admit_reserve(const i32* list, i64 count, const i32* target, const u32* slot,
+                                              const u32* crowd, u64* demand, i32* segments, SclpState* state) {
+    for (i64 base = static_cast<i64>(blockIdx.x) * blockDim.x; base < count; base += static_cast<i64>(gridDim.x) * blockDim.x) {
         const i64 i = base + threadIdx.x;
         i32 t = -1;
         u32 size = 0;
@@ -102,7 +106,27 @@ __global__ void __launch_bounds__(kThreads) admit_reserve_kernel(const i32* __re
     }
 }
 
+__global__ void __launch_bounds__(kThreads) admit_reserve_kernel(const i32* __restrict__ list,
+                                                                 const i32* __restrict__ target,
+                                                                 const u32* __restrict__ slot,
+                                                                 const u32* __restrict__ crowd, u64* demand,
+                                                                 i32* segments, SclpState* state) {
+    if (state->done) return;
+    admit_reserve(list, state->contested, target, slot, crowd, demand, segments, state);
+}
+
 // A proposal in its segment: the gain, then tie (high) and vertex (low).
+__device__ __forceinline__ void admit_scatter(const i32* list, i64 count, const i32* target, const u64* gain,
+                                              const u32* tie, const u32* slot, const u64* demand, u64* seg_gain,
+                                              u64* seg_tie) {
+    for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * blockDim.x) {
+        const i32 v = list[i];
+        const u64 at = demand[target[v]] + slot[v];
+        seg_gain[at] = gain[v];
+        seg_tie[at] = (static_cast<u64>(~tie[v]) << 32) | static_cast<u32>(v);   // ascending = tie descending, vertex ascending
+    }
+}
+
 __global__ void __launch_bounds__(kThreads) admit_scatter_kernel(const i32* __restrict__ list,
                                                                  const i32* __restrict__ target,
                                                                  const u64* __restrict__ gain,
@@ -111,13 +135,7 @@ __global__ void __launch_bounds__(kThreads) admit_scatter_kernel(const i32* __re
                                                                  const u64* __restrict__ demand, u64* seg_gain,
                                                                  u64* seg_tie, const SclpState* state) {
     if (state->done) return;
-    const i64 count = state->contested;
-    for (i64 i = static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * kThreads) {
-        const i32 v = list[i];
-        const u64 at = demand[target[v]] + slot[v];
-        seg_gain[at] = gain[v];
-        seg_tie[at] = (static_cast<u64>(~tie[v]) << 32) | static_cast<u32>(v);   // ascending = tie descending, vertex ascending
-    }
+    admit_scatter(list, state->contested, target, gain, tie, slot, demand, seg_gain, seg_tie);
 }
 
 // Longer than this, a segment is narrowed by all blocks first.
@@ -144,22 +162,19 @@ __device__ __forceinline__ u32 fine_code(u64 g, u64 k) {
 }
 
 // Warp per segment of at most kWarpSegment proposals; longer ones are listed.
-template <typename W>
-__global__ void __launch_bounds__(kThreads) admit_resolve_kernel(const i32* __restrict__ segments,
-                                                                 const u64* __restrict__ demand,
-                                                                 const u64* __restrict__ seg_gain,
-                                                                 const u64* __restrict__ seg_tie,
-                                                                 const u64* __restrict__ cw, const W* __restrict__ vw,
-                                                                 u64 cap, u32* crowd, unsigned char* cls, i32* big,
-                                                                 i32* giant, u64* giant_rows, SclpState* state) {
-    if (state->done) return;
+// GIANTS: those above kGiantSegment are listed by themselves.
+template <bool GIANTS, typename W>
+__device__ __forceinline__ void admit_resolve(const i32* segments, i64 count, const u64* demand, const u64* seg_gain,
+                                              const u64* seg_tie, const u64* cw, const W* __restrict__ vw, u64 cap,
+                                              u32* crowd, unsigned char* cls, i32* big, i32* giant, u64* giant_rows,
+                                              SclpState* state) {
     const int lane = threadIdx.x & 31;
-    const i64 count = state->segments;
-    const i64 warps = static_cast<i64>(gridDim.x) * kWarps;
-    for (i64 s = static_cast<i64>(blockIdx.x) * kWarps + (threadIdx.x >> 5); s < count; s += warps) {
+    const int block_warps = static_cast<int>(blockDim.x >> 5);
+    const i64 warps = static_cast<i64>(gridDim.x) * block_warps;
+    for (i64 s = static_cast<i64>(blockIdx.x) * block_warps + (threadIdx.x >> 5); s < count; s += warps) {
         const i32 t = segments[s];
         const u32 size = crowd[t];
-        if (size > kGiantSegment) {
+        if (GIANTS && size > kGiantSegment) {
             u32 at = 0;
             if (lane == 0) giant[at = atomicAdd(&state->giants, 1u)] = t;
             at = __shfl_sync(0xffffffffu, at, 0);
@@ -187,6 +202,19 @@ __global__ void __launch_bounds__(kThreads) admit_resolve_kernel(const i32* __re
         __syncwarp();
         if (lane == 0) crowd[t] = 0;   // for the next round
     }
+}
+
+template <typename W>
+__global__ void __launch_bounds__(kThreads) admit_resolve_kernel(const i32* __restrict__ segments,
+                                                                 const u64* __restrict__ demand,
+                                                                 const u64* __restrict__ seg_gain,
+                                                                 const u64* __restrict__ seg_tie,
+                                                                 const u64* __restrict__ cw, const W* __restrict__ vw,
+                                                                 u64 cap, u32* crowd, unsigned char* cls, i32* big,
+                                                                 i32* giant, u64* giant_rows, SclpState* state) {
+    if (state->done) return;
+    admit_resolve<true>(segments, state->segments, demand, seg_gain, seg_tie, cw, vw, cap, crowd, cls, big, giant,
+                        giant_rows, state);
 }
 
 constexpr int kAdmitThreads = 512;
@@ -296,15 +324,12 @@ __global__ void __launch_bounds__(kAdmitThreads) admit_giant_kernel(const i32* _
 // step (see resolve_bucket); at most kFew matching proposals are ranked
 // directly.
 template <typename W>
-__global__ void __launch_bounds__(kAdmitThreads) admit_resolve_big_kernel(
-    const i32* __restrict__ big, const u64* __restrict__ demand, const u64* __restrict__ seg_gain,
-    const u64* __restrict__ seg_tie, const u64* __restrict__ cw, const W* __restrict__ vw, u64 cap, u32* crowd,
-    const i32* __restrict__ giant, const u64* __restrict__ giant_rows, const u64* __restrict__ rest,
-    unsigned char* cls, const SclpState* state) {
-    if (state->done) return;
-    __shared__ AdmitShared sh;
+__device__ __forceinline__ void admit_resolve_big(const i32* big, u32 bigs, const u64* demand, const u64* seg_gain,
+                                                  const u64* seg_tie, const u64* cw, const W* __restrict__ vw, u64 cap,
+                                                  u32* crowd, const i32* giant, u32 giants, const u64* giant_rows,
+                                                  const u64* rest, unsigned char* cls, AdmitShared& sh) {
     const int lane = threadIdx.x & 31;
-    const u32 bigs = state->big, segments = bigs + state->giants;
+    const u32 segments = bigs + giants;
     for (u32 s = blockIdx.x; s < segments; s += gridDim.x) {
         const bool narrowed = s >= bigs;   // a giant segment: what admit_giant_kernel left
         const i32 t = narrowed ? giant[s - bigs] : big[s];
@@ -432,9 +457,35 @@ __global__ void __launch_bounds__(kAdmitThreads) admit_resolve_big_kernel(
     }
 }
 
-// Moves the accepted vertices, clears `demand` for the next round and counts
-// the clusters that became empty (sources are movers' clusters and targets are
-// not, so only one side of a cluster's weight changes in a round).
+template <typename W>
+__global__ void __launch_bounds__(kAdmitThreads) admit_resolve_big_kernel(
+    const i32* __restrict__ big, const u64* __restrict__ demand, const u64* __restrict__ seg_gain,
+    const u64* __restrict__ seg_tie, const u64* __restrict__ cw, const W* __restrict__ vw, u64 cap, u32* crowd,
+    const i32* __restrict__ giant, const u64* __restrict__ giant_rows, const u64* __restrict__ rest,
+    unsigned char* cls, const SclpState* state) {
+    if (state->done) return;
+    __shared__ AdmitShared sh;
+    admit_resolve_big(big, state->big, demand, seg_gain, seg_tie, cw, vw, cap, crowd, giant, state->giants, giant_rows,
+                      rest, cls, sh);
+}
+
+// Moves vertex v if it was accepted and clears `demand` for the next round;
+// returns the change in the number of non-empty clusters (sources are movers'
+// clusters and targets are not, so only one side of a cluster's weight changes
+// in a round).
+template <typename W>
+__device__ __forceinline__ long long sclp_commit(i64 v, const unsigned char* cls, const i32* target,
+                                                 const W* __restrict__ vw, i32* clusters, u64* cw, u64* demand) {
+    demand[v] = 0;
+    if (cls[v] != 1) return 0;
+    const i32 t = target[v];
+    const i32 s = clusters[v];
+    const u64 w = static_cast<u64>(weight_at(vw, v));
+    const u64 had = atomic_add_u64(&cw[s], 0ULL - w), got = atomic_add_u64(&cw[t], w);
+    clusters[v] = t;
+    return w ? (got == 0 ? 1 : 0) - (had == w ? 1 : 0) : 0;
+}
+
 template <typename W>
 __global__ void __launch_bounds__(kThreads) sclp_commit_kernel(i64 n, const unsigned char* __restrict__ cls,
                                                                const i32* __restrict__ target,
@@ -443,21 +494,117 @@ __global__ void __launch_bounds__(kThreads) sclp_commit_kernel(i64 n, const unsi
     if (state->done) return;
     __shared__ long long sh[kWarps + 1];
     const i64 v = static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x;
-    long long change = 0;
-    if (v < n) {
-        demand[v] = 0;
-        if (cls[v] == 1) {
-            const i32 t = target[v];
-            const i32 s = clusters[v];
-            const u64 w = static_cast<u64>(weight_at(vw, v));
-            const u64 had = atomic_add_u64(&cw[s], 0ULL - w), got = atomic_add_u64(&cw[t], w);
-            clusters[v] = t;
-            if (w) change = (got == 0 ? 1 : 0) - (had == w ? 1 : 0);
-        }
-    }
+    long long change = v < n ? sclp_commit(v, cls, target, vw, clusters, cw, demand) : 0;
     change = block_sum(change, sh);
     if (round == 0 && blockIdx.x == 0) change -= static_cast<long long>(state->weightless);
     if (threadIdx.x == 0 && change) atomic_add_u64(&state->clusters, static_cast<u64>(change));
+}
+
+// ---------------------------------------------------------------------------
+// All rounds of a small level in one launch: a thread-block cluster runs the
+// affinity passes and the admission with the cluster barrier between the
+// steps (a round is about ten launches otherwise).  For levels without
+// vertices of more than 256 edges; the steps are the functions above.
+// ---------------------------------------------------------------------------
+template <typename O, typename W>
+struct SmallRoundsArgs {
+    i64 n;
+    u64 cap;
+    int sum32;
+    i64 count[3];             // vertices of degree classes 1, 2 and 3
+    const i32* lists[3];
+    const O* off;
+    const i32* nbr;
+    const W* ew;
+    const W* vw;
+    i32* clusters;
+    u64* cw;
+    SclpOut out;
+    unsigned char* cls;
+    u32 *crowd, *slot;
+    i32 *list, *segments, *big;
+    u64 *seg_gain, *seg_tie;
+    RoundParams rounds[4];
+    SclpState* state;
+    u32* err;
+};
+
+inline size_t small_rounds_smem(bool sum32) {
+    return static_cast<size_t>(kAdmitThreads / 32) * kMediumSlots * (sum32 ? 8 : 12);
+}
+
+template <typename T>
+__device__ __forceinline__ T read_state(const T* p) { return *reinterpret_cast<const volatile T*>(p); }
+
+template <typename O, typename W>
+__global__ void __launch_bounds__(kAdmitThreads) sclp_rounds_small_kernel(const SmallRoundsArgs<O, W> a) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ __align__(16) unsigned char tables[];
+    __shared__ AdmitShared sh;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const i64 n = a.n;
+    const i64 tid = static_cast<i64>(blockIdx.x) * kAdmitThreads + threadIdx.x;
+    const i64 threads = static_cast<i64>(gridDim.x) * kAdmitThreads;
+    const i64 warp_id = tid >> 5, warps = threads >> 5;
+    const bool first = tid == 0;
+    SclpState* st = a.state;
+    i64 clusters = n;   // non-empty ones, the same in every thread
+    for (int round = 0; round < 4; ++round) {
+        // round_begin_kernel's decisions
+        if (static_cast<double>(clusters) <= 0.60 * static_cast<double>(n)) break;
+        const i64 desired = (n + 1) / 2;
+        const i64 removable = clusters > desired ? clusters - desired : 0;
+        const double fraction = fmin(0.50, static_cast<double>(removable) / static_cast<double>(clusters));
+        RoundParams p = a.rounds[round];
+        p.mover_threshold = static_cast<u32>(fraction * 4294967296.0);
+        if (first) {
+            if (round == 0) st->clusters = static_cast<u64>(n);
+            st->rounds = round + 1;
+            st->contested = st->segments = st->big = 0;
+            st->segment_items = 0;
+        }
+        for (i64 w = warp_id; w * 4 < a.count[0]; w += warps)
+            affinity_small<8>(w * 4, a.count[0], a.lists[0], a.off, a.nbr, a.ew, a.vw, a.clusters, a.cw, p, a.out);
+        for (i64 w = warp_id; w < a.count[1]; w += warps)
+            affinity_small<32>(w, a.count[1], a.lists[1], a.off, a.nbr, a.ew, a.vw, a.clusters, a.cw, p, a.out);
+        for (i64 w = warp_id; w < a.count[2]; w += warps) {
+            if (a.sum32)
+                affinity_warp_hash<true>(a.lists[2][w], a.off, a.nbr, a.ew, a.vw, a.clusters, a.cw, p, a.out,
+                                         tables + warp * kMediumSlots * 8, a.err);
+            else
+                affinity_warp_hash<false>(a.lists[2][w], a.off, a.nbr, a.ew, a.vw, a.clusters, a.cw, p, a.out,
+                                          tables + warp * kMediumSlots * 12, a.err);
+        }
+        cluster.sync();
+        for (i64 base = tid - lane; base < n; base += threads)
+            admit_classify(base + lane, n, a.out.target, a.out.demand, a.cw, a.cap, a.cls, a.crowd, a.slot, a.list, st);
+        cluster.sync();
+        const i64 contested = read_state(&st->contested);
+        if (contested) {   // the same in every thread
+            admit_reserve(a.list, contested, a.out.target, a.slot, a.crowd, a.out.demand, a.segments, st);
+            cluster.sync();
+            admit_scatter(a.list, contested, a.out.target, a.out.gain, a.out.tie, a.slot, a.out.demand, a.seg_gain,
+                          a.seg_tie);
+            cluster.sync();
+            admit_resolve<false>(a.segments, static_cast<i64>(read_state(&st->segments)), a.out.demand, a.seg_gain,
+                                 a.seg_tie, a.cw, a.vw, a.cap, a.crowd, a.cls, a.big, static_cast<i32*>(nullptr),
+                                 static_cast<u64*>(nullptr), st);
+            cluster.sync();
+            admit_resolve_big(a.big, read_state(&st->big), a.out.demand, a.seg_gain, a.seg_tie, a.cw, a.vw, a.cap,
+                              a.crowd, static_cast<const i32*>(nullptr), 0u, static_cast<const u64*>(nullptr),
+                              static_cast<const u64*>(nullptr), a.cls, sh);
+            cluster.sync();
+        }
+        long long change = first && round == 0 ? -static_cast<long long>(read_state(&st->weightless)) : 0;
+        for (i64 v = tid; v < n; v += threads)
+            change += sclp_commit(v, a.cls, a.out.target, a.vw, a.clusters, a.cw, a.out.demand);
+        change = warp_sum(change);
+        if (lane == 0 && change) atomic_add_u64(&st->clusters, static_cast<u64>(change));
+        cluster.sync();
+        clusters = static_cast<i64>(read_state(&st->clusters));
+        cluster.sync();   // read before block 0 starts the next round
+    }
 }
 
 }  // namespace gp

@@ -304,6 +304,16 @@ inline u64 saturated_sum(const u64* parts) {
     return sum > ~0ULL ? ~0ULL : static_cast<u64>(sum);
 }
 
+// Levels refined by one cluster (refine_small_kernel): no hub rows (their
+// chunked kernels are not part of it) and at most this many vertices and
+// entries.  One cluster is 16 of the 148 SMs, so it wins while launches and
+// round trips, not bandwidth, are the time.  Measured with the line at 32 K,
+// 128 K, 256 K and 1 M vertices, ms per partition: RGG 150,000 k = 8 11.8,
+// 11.1, 11.0, 11.0; RGG 300,000 k = 32 15.0, 14.7, 14.7, 15.8; grid 700x701
+// k = 16 28.1, 25.7, 25.1, 29.8.
+constexpr i64 kSmallRefineN = 131072;
+constexpr i64 kSmallRefineM = 1 << 21;
+
 // ---------------------------------------------------------------------------
 // SCLP aggregation (src/coarsen.cu:937-1659)
 // ---------------------------------------------------------------------------
@@ -601,7 +611,36 @@ void aggregate(Device& d, const DGraph<T>& g, SclpWork<T>& w, int parts, u32 see
     // A segment of more than kGiantSegment proposals needs as many vertices.
     const i64 giant_cap = n / kGiantSegment;
     Buf<u64> giant_rows(d, static_cast<size_t>(std::max<i64>(giant_cap, 1)) * kGiantRow);
-    for (int round = 0; round < 4; ++round) {
+    // Small levels without long rows run their rounds in one cluster launch
+    // (the same limits as the one-launch refinement).
+    const bool one_launch = !log.on && !trace().on && n <= kSmallRefineN && g.m <= kSmallRefineM && cnt[4] == 0 &&
+                            cnt[5] == 0;
+    if (one_launch) {
+        SmallRoundsArgs<O, W> a{};
+        a.n = n; a.cap = cap; a.sum32 = sum32;
+        for (int c = 1; c <= 3; ++c) { a.count[c - 1] = cnt[c]; a.lists[c - 1] = class_list(c); }
+        a.off = off; a.nbr = nbr; a.ew = ew; a.vw = vw;
+        a.clusters = clusters; a.cw = cw; a.out = so; a.cls = w.cls.get();
+        a.crowd = w.crowd.get(); a.slot = w.slot.get();
+        a.list = w.list.get(); a.segments = w.list_alt.get();
+        a.big = reinterpret_cast<i32*>(w.slot.get());   // the slots are used up by then
+        a.seg_gain = w.keys.get(); a.seg_tie = w.keys_alt.get();
+        for (int round = 0; round < 4; ++round) {
+            a.rounds[round] = make_round(seed, level, round, true, 0);
+            a.rounds[round].sum32 = sum32;
+        }
+        a.state = state; a.err = d.err;
+        auto kernel = sclp_rounds_small_kernel<O, W>;
+        GP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(small_rounds_smem(false))));
+        const int most = wide_cluster_blocks(d, kernel, kAdmitThreads, small_rounds_smem(false));
+        int blocks = 1;
+        while (blocks < most && (blocks * kAdmitThreads < n || static_cast<i64>(blocks) * 4096 < g.m)) blocks *= 2;
+        launch_cluster(d, "sclp_rounds_small_kernel", kernel, blocks, kAdmitThreads,
+                       cnt[3] ? small_rounds_smem(sum32 != 0) : 0, a);
+        fetch(d, &hs, state, 1);
+    }
+    for (int round = 0; round < 4 && !one_launch; ++round) {
         RoundParams p = make_round(seed, level, round, true, 0);
         p.sum32 = sum32;
         p.state = state;
@@ -1417,16 +1456,6 @@ struct RefineWork {
 // known_cut: the cut of `labels` when the caller has it (a projection keeps
 // the cut of the coarser level's result), else kUnknownCut.
 constexpr u64 kUnknownCut = ~0ULL;
-
-// Levels refined by one cluster (refine_small_kernel): no hub rows (their
-// chunked kernels are not part of it) and at most this many vertices and
-// entries.  One cluster is 16 of the 148 SMs, so it wins while launches and
-// round trips, not bandwidth, are the time.  Measured with the line at 32 K,
-// 128 K, 256 K and 1 M vertices, ms per partition: RGG 150,000 k = 8 11.8,
-// 11.1, 11.0, 11.0; RGG 300,000 k = 32 15.0, 14.7, 14.7, 15.8; grid 700x701
-// k = 16 28.1, 25.7, 25.1, 29.8.
-constexpr i64 kSmallRefineN = 131072;
-constexpr i64 kSmallRefineM = 1 << 21;
 
 template <typename T>
 bool refine_is_small(Device& d, const DGraph<T>& g) {

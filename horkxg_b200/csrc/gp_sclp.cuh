@@ -151,16 +151,16 @@ __device__ __forceinline__ void group_reduce(u64& current, u64& best, u64& tie, 
 
 // deg <= G: one lane per edge, G lanes per vertex, equal clusters grouped by
 // __match_any_sync (cf. sclp_affinity_low_match_kernel, :332-403).
+// One warp step: 32 / G list entries from `first` on.
 template <int G, typename O, typename W>
-__global__ void __launch_bounds__(kThreads) affinity_small_kernel(
-    i64 count, const i32* __restrict__ list, const O* __restrict__ off, const i32* __restrict__ nbr,
-    const W* __restrict__ ew, const W* __restrict__ vw, const i32* __restrict__ clusters,
-    const u64* __restrict__ cw, RoundParams p, SclpOut out) {
-    if (!round_ready(p)) return;
+__device__ __forceinline__ void affinity_small(i64 first, i64 count, const i32* list, const O* __restrict__ off,
+                                               const i32* __restrict__ nbr, const W* __restrict__ ew,
+                                               const W* __restrict__ vw, const i32* clusters, const u64* cw,
+                                               const RoundParams& p, const SclpOut& out) {
     const int lane = threadIdx.x & 31;
     const int lig = lane & (G - 1);
     const unsigned mask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
-    const i64 gid = (static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x) / G;
+    const i64 gid = first + lane / G;
     const bool has_vertex = gid < count;
     const i32 v = has_vertex ? list[gid] : -1;
     const i32 source = has_vertex ? (p.identity ? v : clusters[v]) : -1;
@@ -204,6 +204,16 @@ __global__ void __launch_bounds__(kThreads) affinity_small_kernel(
     }
     group_reduce(current, best, tie, G, mask);
     if (has_vertex && lig == 0) decode_and_write(v, source, current, best, tie, p, vw, cw, out);
+}
+
+template <int G, typename O, typename W>
+__global__ void __launch_bounds__(kThreads) affinity_small_kernel(
+    i64 count, const i32* __restrict__ list, const O* __restrict__ off, const i32* __restrict__ nbr,
+    const W* __restrict__ ew, const W* __restrict__ vw, const i32* __restrict__ clusters,
+    const u64* __restrict__ cw, RoundParams p, SclpOut out) {
+    if (!round_ready(p)) return;
+    const i64 warp = (static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
+    affinity_small<G>(warp * (32 / G), count, list, off, nbr, ew, vw, clusters, cw, p, out);
 }
 
 // Shared/global open-addressing table insert (linear probing, key = cluster).
@@ -258,25 +268,20 @@ __device__ __forceinline__ void slot_candidate(i32 key, u64 conn, u32 v, i32 sou
 // Warp per vertex, shared hash of kMediumSlots per warp (cf.
 // sclp_affinity_medium_hash_kernel, :405-476).
 // PACKED: 8-byte slots (packed_insert), for levels with p.sum32.
+// One vertex by one warp; `table` holds kMediumSlots slots of 8 or 12 bytes.
 template <bool PACKED, typename O, typename W>
-__global__ void __launch_bounds__(kThreads) affinity_warp_hash_kernel(
-    i64 count, const i32* __restrict__ list, const O* __restrict__ off, const i32* __restrict__ nbr,
-    const W* __restrict__ ew, const W* __restrict__ vw, const i32* __restrict__ clusters,
-    const u64* __restrict__ cw, RoundParams p, SclpOut out, u32* err) {
-    if (!round_ready(p)) return;
-    constexpr int kSlotBytes = PACKED ? 8 : 12;
-    __shared__ __align__(16) unsigned char table_all[kWarps][kMediumSlots * kSlotBytes];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const i64 gid = static_cast<i64>(blockIdx.x) * kWarps + warp;
-    if (gid >= count) return;
-    const i32 v = list[gid];
+__device__ __forceinline__ void affinity_warp_hash(i32 v, const O* __restrict__ off, const i32* __restrict__ nbr,
+                                                   const W* __restrict__ ew, const W* __restrict__ vw,
+                                                   const i32* clusters, const u64* cw, const RoundParams& p,
+                                                   const SclpOut& out, unsigned char* table, u32* err) {
+    const int lane = threadIdx.x & 31;
     const i32 source = p.identity ? v : clusters[v];
     if (role_blocked(source, p)) {
         if (lane == 0) out.target[v] = kInvalid;
         return;
     }
-    auto* slots = reinterpret_cast<unsigned long long*>(table_all[warp]);   // PACKED
-    u64* vals = reinterpret_cast<u64*>(table_all[warp]);                     // !PACKED
+    auto* slots = reinterpret_cast<unsigned long long*>(table);   // PACKED
+    u64* vals = reinterpret_cast<u64*>(table);                     // !PACKED
     i32* keys = reinterpret_cast<i32*>(vals + kMediumSlots);
     for (int s = lane; s < kMediumSlots; s += 32) {
         if constexpr (PACKED) { slots[s] = 0ULL; } else { keys[s] = -1; vals[s] = 0; }
@@ -305,6 +310,20 @@ __global__ void __launch_bounds__(kThreads) affinity_warp_hash_kernel(
     }
     group_reduce(current, best, tie, 32, 0xffffffffu);
     if (lane == 0) decode_and_write(v, source, current, best, tie, p, vw, cw, out);
+    __syncwarp();   // the table is free again
+}
+
+template <bool PACKED, typename O, typename W>
+__global__ void __launch_bounds__(kThreads) affinity_warp_hash_kernel(
+    i64 count, const i32* __restrict__ list, const O* __restrict__ off, const i32* __restrict__ nbr,
+    const W* __restrict__ ew, const W* __restrict__ vw, const i32* __restrict__ clusters,
+    const u64* __restrict__ cw, RoundParams p, SclpOut out, u32* err) {
+    if (!round_ready(p)) return;
+    __shared__ __align__(16) unsigned char table[kWarps][kMediumSlots * (PACKED ? 8 : 12)];
+    const int warp = threadIdx.x >> 5;
+    const i64 gid = static_cast<i64>(blockIdx.x) * kWarps + warp;
+    if (gid >= count) return;
+    affinity_warp_hash<PACKED>(list[gid], off, nbr, ew, vw, clusters, cw, p, out, table[warp], err);
 }
 
 // Block-wide reduction of (current, best, tie); result valid in thread 0.
