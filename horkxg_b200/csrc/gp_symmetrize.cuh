@@ -5,8 +5,10 @@
 // distinct edge, rows ascending by neighbour.
 //
 // The reference sorts (min, max) keys in disk runs, merges them, counts
-// degrees and sorts again for the reverse direction.  Here the whole job is
-// one device radix sort: each entry writes its two directed keys
+// degrees and sorts again for the reverse direction.  Graphs of up to 2^22
+// vertices are symmetrised row by row with the contraction's row sorts (see
+// symmetrize_rows); above, and for generated graphs, the whole job is one
+// device radix sort: each entry writes its two directed keys
 // (v << b | u) and (u << b | v), b = bits of the vertex range, into slots 2e
 // and 2e + 1 (a self loop writes two all-ones sentinels, which sort last);
 // after the sort equal neighbours are adjacent, a flag-and-scan compaction
@@ -14,6 +16,7 @@
 // aggregated counts of the sources.
 #pragma once
 
+#include "gp_contract.cuh"
 #include "gp_prim.cuh"
 
 namespace gp {
@@ -109,6 +112,111 @@ __global__ void sym_compact_kernel(i64 valid, const u64* __restrict__ keys, cons
         if (head && (threadIdx.x & 31) == __ffs(peers) - 1)
             atomicAdd(reinterpret_cast<unsigned long long*>(&degree[src]), static_cast<unsigned long long>(__popc(peers)));
     }
+}
+
+// ---------------------------------------------------------------------------
+// Row by row.  A block takes a tile of consecutive entries, so hub rows are
+// spread like any others; an entry's row is found by bisection among the rows
+// of the tile.
+// ---------------------------------------------------------------------------
+constexpr int kSymItems = 8;
+constexpr i64 kSymTile = kThreads * kSymItems;
+
+// Last row r in [lo, hi] with off[r] <= e.
+template <typename O>
+__device__ __forceinline__ i64 row_of_entry(const O* __restrict__ off, i64 lo, i64 hi, i64 e) {
+    while (lo < hi) {
+        const i64 mid = (lo + hi + 1) >> 1;
+        if (static_cast<i64>(off[mid]) <= e) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+// f(entry, row) for the block's tile.
+template <typename O, typename F>
+__device__ __forceinline__ void for_tile_entries(i64 n, i64 m, const O* __restrict__ off, F f) {
+    __shared__ i64 range[2];
+    const i64 begin = static_cast<i64>(blockIdx.x) * kSymTile;
+    const i64 end = begin + kSymTile < m ? begin + kSymTile : m;
+    if (begin >= end) return;   // uniform over the block
+    if (threadIdx.x < 2) range[threadIdx.x] = row_of_entry(off, 0, n - 1, threadIdx.x ? end - 1 : begin);
+    __syncthreads();
+    const i64 lo = range[0], hi = range[1];
+#pragma unroll 2
+    for (i64 e = begin + threadIdx.x; e < end; e += kThreads) f(e, row_of_entry(off, lo, hi, e));
+}
+
+// Arrivals of reversed entries per vertex; place[e] is entry e's number among
+// its target's.
+template <typename O>
+__global__ void __launch_bounds__(kThreads) sym_count_kernel(i64 n, i64 m, const O* __restrict__ off,
+                                                             const i32* __restrict__ nbr, u32* arrivals, u32* place,
+                                                             u64* self_loops) {
+    u64 loops = 0;
+    for_tile_entries(n, m, off, [&](i64 e, i64 v) {
+        const i32 u = nbr[e];
+        if (u == v) ++loops;
+        else place[e] = atomicAdd(&arrivals[u], 1u);
+    });
+    loops = warp_sum(loops);
+    if ((threadIdx.x & 31) == 0 && loops) atomic_add_u64(self_loops, loops);
+}
+
+// Entries of a vertex's row before deduplication: its own, then the arrivals.
+template <typename O>
+struct SymRowTotal {
+    const O* off;
+    const u32* arrivals;
+    i64 n;
+    __device__ i64 operator()(i64 v) const {
+        return v < n ? static_cast<i64>(off[v + 1]) - static_cast<i64>(off[v]) + arrivals[v] : 0;
+    }
+};
+
+// Self loops become the sentinel n.
+template <typename O>
+__global__ void __launch_bounds__(kThreads) sym_scatter_kernel(i64 n, i64 m, const O* __restrict__ off,
+                                                               const i32* __restrict__ nbr,
+                                                               const u32* __restrict__ place,
+                                                               const i64* __restrict__ temp_off, u32* __restrict__ tgt) {
+    for_tile_entries(n, m, off, [&](i64 e, i64 v) {
+        const i32 u = nbr[e];
+        tgt[temp_off[v] + (e - static_cast<i64>(off[v]))] = u == v ? static_cast<u32>(n) : static_cast<u32>(u);
+        if (u != v)
+            tgt[temp_off[u] + (static_cast<i64>(off[u + 1]) - static_cast<i64>(off[u])) + place[e]] = static_cast<u32>(v);
+    });
+}
+
+// The unique neighbours of the rows sorted in place, a warp per 32 rows.
+template <typename N>
+__global__ void __launch_bounds__(kThreads) sym_copy_rows_kernel(i64 rows, const i64* __restrict__ temp_off,
+                                                                 const i64* __restrict__ off,
+                                                                 const u32* __restrict__ tgt, N* __restrict__ nbr) {
+    const int lane = threadIdx.x & 31;
+    const i64 r0 = ((static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x) >> 5) * 32;
+    if (r0 >= rows) return;
+    const i64 r = r0 + lane;
+    i64 to = 0, len = 0, from = 0;
+    if (r < rows) {
+        to = off[r];
+        len = off[r + 1] - to;
+        from = temp_off[r];
+        if (temp_off[r + 1] - from > seg_smem_capacity<u32>()) len = 0;   // sym_copy_big_rows_kernel
+    }
+    warp_edge_walk(from, len, [&](bool valid, int owner, i64 i) {
+        const i64 shift = __shfl_sync(0xffffffffu, to - from, owner);
+        if (valid) nbr[i + shift] = static_cast<N>(tgt[i]);
+    });
+}
+
+template <typename N>
+__global__ void __launch_bounds__(kThreads) sym_copy_big_rows_kernel(const i32* __restrict__ list,
+                                                                     const i64* __restrict__ alt_off,
+                                                                     const i64* __restrict__ off,
+                                                                     const u32* __restrict__ keys, N* __restrict__ nbr) {
+    const i32 r = list[blockIdx.x];
+    const i64 to = off[r], len = off[r + 1] - to, from = alt_off[blockIdx.x];
+    for (i64 i = threadIdx.x; i < len; i += kThreads) nbr[to + i] = static_cast<N>(keys[from + i]);
 }
 
 }  // namespace gp
