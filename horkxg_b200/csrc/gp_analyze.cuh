@@ -57,12 +57,13 @@ __device__ __forceinline__ AnalyzeShared analyze_shared(unsigned char* raw, int 
     return s;
 }
 
-// One entry from source part `sp`; false when its neighbour's label is out of
-// range.
+constexpr int kAnalyzeBatch = 4;
+
+// One entry from source part `sp` to a neighbour of part `q`; false when that
+// label is out of range.
 template <typename W>
-__device__ __forceinline__ bool analyze_entry(i64 e, int sp, const i32* __restrict__ nbr, const W* __restrict__ ew,
-                                              const i32* __restrict__ labels, int parts, const AnalyzeShared& s) {
-    const int q = labels[nbr[e]];
+__device__ __forceinline__ bool analyze_entry(i64 e, int q, int sp, const W* __restrict__ ew, int parts,
+                                              const AnalyzeShared& s) {
     if (q < 0 || q >= parts) return false;
     const int slot = 2 * q + (q == sp ? 1 : 0);
     atomicAdd(&s.entries[slot], 1u);
@@ -120,10 +121,37 @@ __global__ void __launch_bounds__(kThreads) analyze_rows_kernel(i64 n, const O* 
                 if (deg) atomic_add_u64(&s.row_length[sp], static_cast<u64>(deg));
             }
         }
-        warp_edge_walk(b, deg, [&](bool valid, int owner, i64 e) {
-            const int from = __shfl_sync(0xffffffffu, sp, owner);
-            if (valid && !analyze_entry(e, from, nbr, ew, labels, parts, s)) bad = true;
-        });
+        // warp_edge_walk kAnalyzeBatch steps at a time: the batch's neighbours
+        // are loaded, then their labels, before any counter is touched
+        const i64 inc = warp_inclusive_sum(deg);
+        const i64 pre = inc - deg;
+        const i64 total = __shfl_sync(0xffffffffu, inc, 31);
+        for (i64 base = 0; base < total; base += kAnalyzeBatch * 32) {
+            int from[kAnalyzeBatch], q[kAnalyzeBatch];
+            i32 u[kAnalyzeBatch];
+            i64 e[kAnalyzeBatch];
+#pragma unroll
+            for (int j = 0; j < kAnalyzeBatch; ++j) {
+                const i64 at = base + j * 32 + lane;
+                int lo = 0;
+#pragma unroll
+                for (int step = 16; step; step >>= 1) {
+                    const i64 probe = __shfl_sync(0xffffffffu, pre, lo + step);
+                    if (probe <= at) lo += step;
+                }
+                const i64 my_pre = __shfl_sync(0xffffffffu, pre, lo);
+                e[j] = __shfl_sync(0xffffffffu, b, lo) + (at - my_pre);
+                from[j] = __shfl_sync(0xffffffffu, sp, lo);
+                u[j] = at < total ? nbr[e[j]] : -1;
+            }
+#pragma unroll
+            for (int j = 0; j < kAnalyzeBatch; ++j) q[j] = u[j] >= 0 ? labels[u[j]] : -1;
+#pragma unroll
+            for (int j = 0; j < kAnalyzeBatch; ++j) {
+                if (u[j] < 0) continue;
+                if (!analyze_entry(e[j], q[j], from[j], ew, parts, s)) bad = true;
+            }
+        }
     }
     if (bad) set_error(err, kErrBadInput);
     analyze_flush(s, parts, ew != nullptr, out);
@@ -148,7 +176,7 @@ __global__ void __launch_bounds__(kThreads) analyze_hub_kernel(i64 count, const 
         }
         if (threadIdx.x == 0) atomic_add_u64(&s.row_length[sp], static_cast<u64>(ch.end - ch.begin));
         for (i64 e = ch.begin + threadIdx.x; e < ch.end; e += kThreads)
-            if (!analyze_entry(e, sp, nbr, ew, labels, parts, s)) bad = true;
+            if (!analyze_entry(e, labels[nbr[e]], sp, ew, parts, s)) bad = true;
     }
     if (bad) set_error(err, kErrBadInput);
     analyze_flush(s, parts, ew != nullptr, out);

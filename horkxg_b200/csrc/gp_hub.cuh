@@ -696,15 +696,16 @@ __global__ void hub_chunk_finalize_kernel(i64 hubs, const i32* __restrict__ hub_
 template <typename O>
 __global__ void __launch_bounds__(kThreads) unsorted_rows_kernel(i64 n, const O* __restrict__ off,
                                                                  const i32* __restrict__ nbr, u32* flag) {
-    const int lane = threadIdx.x & 31;
-    const i64 warps_total = static_cast<i64>(gridDim.x) * kWarps;
+    // 8 lanes per row (the grid of 320^3 took 4.1 ms with a warp per row)
+    const int gl = threadIdx.x & 7;
+    const i64 groups = static_cast<i64>(gridDim.x) * (kThreads / 8);
     bool bad = false;
-    for (i64 v = static_cast<i64>(blockIdx.x) * kWarps + (threadIdx.x >> 5); v < n; v += warps_total) {
+    for (i64 v = static_cast<i64>(blockIdx.x) * (kThreads / 8) + (threadIdx.x >> 3); v < n; v += groups) {
         const i64 b = off[v], e1 = off[v + 1];
         if (e1 - b > kHubDegree) continue;
-        for (i64 e = b + 1 + lane; e < e1; e += 32) bad |= nbr[e] <= nbr[e - 1];
+        for (i64 e = b + 1 + gl; e < e1; e += 8) bad |= nbr[e] <= nbr[e - 1];
     }
-    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(flag, 1u);
+    if (bad) atomicOr(flag, 1u);
 }
 
 template <typename O>

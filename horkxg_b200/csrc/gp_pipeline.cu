@@ -238,7 +238,7 @@ bool unique_rows(Device& d, const DGraph<T>& g) {
     using O = typename T::O;
     Buf<u32> flag(d, 1);
     flag.zero(d);
-    launch(d, "unsorted_rows_kernel", unsorted_rows_kernel<O>, stride_grid(d, g.n * 32), kThreads, 0, g.n, g.off.get(),
+    launch(d, "unsorted_rows_kernel", unsorted_rows_kernel<O>, stride_grid(d, g.n * 8), kThreads, 0, g.n, g.off.get(),
            g.nbr.get(), flag.get());
     const auto& hubs = hub_index(d, g);
     if (hubs.count)
