@@ -564,10 +564,10 @@ __global__ void __launch_bounds__(kAdmitThreads) sclp_rounds_small_kernel(const 
             st->contested = st->segments = st->big = 0;
             st->segment_items = 0;
         }
-        for (i64 w = warp_id; w * 4 < a.count[0]; w += warps)
-            affinity_small<8>(w * 4, a.count[0], a.lists[0], a.off, a.nbr, a.ew, a.vw, a.clusters, a.cw, p, a.out);
+        for (i64 i = tid; i < a.count[0]; i += threads)
+            affinity_tiny(a.lists[0][i], a.off, a.nbr, a.ew, a.vw, a.clusters, a.cw, p, a.out);
         for (i64 w = warp_id; w < a.count[1]; w += warps)
-            affinity_small<32>(w, a.count[1], a.lists[1], a.off, a.nbr, a.ew, a.vw, a.clusters, a.cw, p, a.out);
+            affinity_small(a.lists[1][w], a.off, a.nbr, a.ew, a.vw, a.clusters, a.cw, p, a.out);
         for (i64 w = warp_id; w < a.count[2]; w += warps) {
             if (a.sum32)
                 affinity_warp_hash<true>(a.lists[2][w], a.off, a.nbr, a.ew, a.vw, a.clusters, a.cw, p, a.out,

@@ -489,17 +489,18 @@ void aggregate(Device& d, const DGraph<T>& g, SclpWork<T>& w, int parts, u32 see
             } else {
                 for (int j = 0; j < 3; ++j) gwork[j] = work[5][j];
             }
-            d.prof_bytes("affinity_small_kernel", affinity_bytes(1, p.identity) + affinity_bytes(2, p.identity));
+            d.prof_bytes("affinity_tiny_kernel", affinity_bytes(1, p.identity));
+            d.prof_bytes("affinity_small_kernel", affinity_bytes(2, p.identity));
             if (!(p.identity && direct_ok)) {   // the direct kernels of identity rounds carry no model
                 d.prof_bytes("affinity_warp_hash_kernel", affinity_bytes(3, p.identity));
                 d.prof_bytes("affinity_block_hash_kernel", affinity_bytes(4, p.identity));
             }
         }
         if (cnt[1])
-            launch(d, "affinity_small_kernel", affinity_small_kernel<8, O, W>, blocks_for(static_cast<i64>(cnt[1]) * 8, kThreads), kThreads, 0, 
+            launch(d, "affinity_tiny_kernel", affinity_tiny_kernel<O, W>, blocks_for(cnt[1], kThreads), kThreads, 0,
                 cnt[1], class_list(1), off, nbr, ew, vw, clusters, cw, p, so);
         if (cnt[2])
-            launch(d, "affinity_small_kernel", affinity_small_kernel<32, O, W>, blocks_for(static_cast<i64>(cnt[2]) * 32, kThreads), kThreads, 0, 
+            launch(d, "affinity_small_kernel", affinity_small_kernel<O, W>, blocks_for(static_cast<i64>(cnt[2]) * 32, kThreads), kThreads, 0, 
                 cnt[2], class_list(2), off, nbr, ew, vw, clusters, cw, p, so);
         const bool direct = p.identity && direct_ok;
         if (cnt[3] && direct)

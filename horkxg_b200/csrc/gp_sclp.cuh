@@ -1,8 +1,8 @@
 // SCLP aggregation (size-constrained label propagation), the first stage of
 // the partitioner.  Restates src/coarsen.cu:937-1659 with a B200 layout:
 //
-// * affinity + gain decode fused in one pass per degree class: 8-lane groups
-//   (__match_any_sync) for deg <= 8, a warp for deg <= 32, a warp with a
+// * affinity + gain decode fused in one pass per degree class: a thread for
+//   deg <= 8, a warp (__match_any_sync) for deg <= 32, a warp with a
 //   512-slot shared hash for deg <= 256, a block with a 4096-slot shared hash
 //   for deg <= 2048, and a block with an L2-resident global hash table for
 //   hubs above that; the four u64 affinity arrays of the reference never hit
@@ -149,29 +149,84 @@ __device__ __forceinline__ void group_reduce(u64& current, u64& best, u64& tie, 
     }
 }
 
-// deg <= G: one lane per edge, G lanes per vertex, equal clusters grouped by
+// deg <= 8: one thread per vertex with all of its neighbours in registers; equal
+// clusters are found by comparing all pairs.  Eight gathers are in flight per
+// thread, and a vertex costs a few warp instructions instead of the ~15 of a
+// group of eight lanes with a match and three reductions.
+template <typename O, typename W>
+__device__ __forceinline__ void affinity_tiny(i32 v, const O* __restrict__ off, const i32* __restrict__ nbr,
+                                              const W* __restrict__ ew, const W* __restrict__ vw, const i32* clusters,
+                                              const u64* cw, const RoundParams& p, const SclpOut& out) {
+    const i32 source = p.identity ? v : clusters[v];
+    if (role_blocked(source, p)) {
+        out.target[v] = kInvalid;
+        return;
+    }
+    const i64 b = off[v];
+    const int deg = static_cast<int>(static_cast<i64>(off[v + 1]) - b);
+    i32 c[8];
+    u64 w[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) c[j] = j < deg ? nbr[b + j] : v;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const bool other = c[j] != v;
+        w[j] = other ? static_cast<u64>(weight_at(ew, b + j)) : 0;
+        c[j] = !other ? -1 : (p.identity ? c[j] : clusters[c[j]]);
+    }
+    u64 current = 0, best = 0, tie = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (c[j] < 0) continue;
+        u64 conn = w[j];
+        bool leader = true;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (i == j || c[i] != c[j]) continue;
+            if (i < j) leader = false;
+            conn += w[i];
+        }
+        if (!leader) continue;
+        if (c[j] == source) current = conn;
+        else if (conn >= best && conn != 0 && (!p.filter || !is_mover(c[j], p))) {
+            const u64 t = tie_key(static_cast<u32>(v), c[j], p.tie_salt);
+            if (better(conn, t, best, tie)) { best = conn; tie = t; }
+        }
+    }
+    decode_and_write(v, source, current, best, tie, p, vw, cw, out);
+}
+
+template <typename O, typename W>
+__global__ void __launch_bounds__(kThreads) affinity_tiny_kernel(
+    i64 count, const i32* __restrict__ list, const O* __restrict__ off, const i32* __restrict__ nbr,
+    const W* __restrict__ ew, const W* __restrict__ vw, const i32* __restrict__ clusters,
+    const u64* __restrict__ cw, RoundParams p, SclpOut out) {
+    if (!round_ready(p)) return;
+    const i64 i = static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x;
+    if (i < count) affinity_tiny(list[i], off, nbr, ew, vw, clusters, cw, p, out);
+}
+
+// deg <= 32: one lane per edge, a warp per vertex, equal clusters grouped by
 // __match_any_sync (cf. sclp_affinity_low_match_kernel, :332-403).
-// One warp step: 32 / G list entries from `first` on.
-template <int G, typename O, typename W>
-__device__ __forceinline__ void affinity_small(i64 first, i64 count, const i32* list, const O* __restrict__ off,
-                                               const i32* __restrict__ nbr, const W* __restrict__ ew,
-                                               const W* __restrict__ vw, const i32* clusters, const u64* cw,
-                                               const RoundParams& p, const SclpOut& out) {
+template <typename O, typename W>
+__device__ __forceinline__ void affinity_small(i32 v, const O* __restrict__ off, const i32* __restrict__ nbr,
+                                               const W* __restrict__ ew, const W* __restrict__ vw,
+                                               const i32* clusters, const u64* cw, const RoundParams& p,
+                                               const SclpOut& out) {
     const int lane = threadIdx.x & 31;
-    const int lig = lane & (G - 1);
-    const unsigned mask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
-    const i64 gid = first + lane / G;
-    const bool has_vertex = gid < count;
-    const i32 v = has_vertex ? list[gid] : -1;
-    const i32 source = has_vertex ? (p.identity ? v : clusters[v]) : -1;
+    const i32 source = p.identity ? v : clusters[v];
+    if (role_blocked(source, p)) {
+        if (lane == 0) out.target[v] = kInvalid;
+        return;
+    }
     bool valid = false;
     i32 c = -1;
     u64 w = 0;
-    if (has_vertex && !role_blocked(source, p)) {
+    {
         const i64 begin = off[v];
         const i64 deg = static_cast<i64>(off[v + 1]) - begin;
-        if (lig < deg) {
-            const i64 e = begin + lig;
+        if (lane < deg) {
+            const i64 e = begin + lane;
             const i32 u = nbr[e];
             if (u != v) {
                 valid = true;
@@ -180,16 +235,15 @@ __device__ __forceinline__ void affinity_small(i64 first, i64 count, const i32* 
             }
         }
     }
-    const unsigned peers = __match_any_sync(mask, valid ? c : -1);
+    const unsigned peers = __match_any_sync(0xffffffffu, valid ? c : -1);
     u64 conn = 0;
     if (p.sum32) {
         conn = __reduce_add_sync(peers, static_cast<u32>(w));
     } else {
-        const int base = lane & ~(G - 1);
 #pragma unroll
-        for (int s = 0; s < G; ++s) {
-            const u64 pw = __shfl_sync(mask, w, base + s);
-            if (peers & (1u << (base + s))) conn += pw;
+        for (int s = 0; s < 32; ++s) {
+            const u64 pw = __shfl_sync(0xffffffffu, w, s);
+            if (peers & (1u << s)) conn += pw;
         }
     }
     const bool leader = valid && lane == __ffs(peers) - 1;
@@ -202,18 +256,18 @@ __device__ __forceinline__ void affinity_small(i64 first, i64 count, const i32* 
             tie = tie_key(static_cast<u32>(v), c, p.tie_salt);
         }
     }
-    group_reduce(current, best, tie, G, mask);
-    if (has_vertex && lig == 0) decode_and_write(v, source, current, best, tie, p, vw, cw, out);
+    group_reduce(current, best, tie, 32, 0xffffffffu);
+    if (lane == 0) decode_and_write(v, source, current, best, tie, p, vw, cw, out);
 }
 
-template <int G, typename O, typename W>
+template <typename O, typename W>
 __global__ void __launch_bounds__(kThreads) affinity_small_kernel(
     i64 count, const i32* __restrict__ list, const O* __restrict__ off, const i32* __restrict__ nbr,
     const W* __restrict__ ew, const W* __restrict__ vw, const i32* __restrict__ clusters,
     const u64* __restrict__ cw, RoundParams p, SclpOut out) {
     if (!round_ready(p)) return;
-    const i64 warp = (static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
-    affinity_small<G>(warp * (32 / G), count, list, off, nbr, ew, vw, clusters, cw, p, out);
+    const i64 i = (static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
+    if (i < count) affinity_small(list[i], off, nbr, ew, vw, clusters, cw, p, out);
 }
 
 // Shared/global open-addressing table insert (linear probing, key = cluster).
