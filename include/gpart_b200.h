@@ -328,8 +328,12 @@ gp_status gp_ctx_set_hub_tables(gp_ctx* ctx, int on_chip);
  * one B200 the graph saves host round trips but not consistently time: RMAT-20
  * partitions ran 3-8% faster, RMAT-24 within run-to-run noise, graphs of
  * 10^4-10^5 vertices 4-6% slower (their rebalances end after one or two
- * iterations, so building the graph does not pay).  The deterministic mode
- * and profiling always use the host loop. */
+ * iterations, so building the graph does not pay; measured before such levels
+ * got a launch of their own).  The deterministic mode
+ * and profiling always use the host loop.  Levels of at most 131,072 vertices
+ * and 2^21 entries without hub rows run their whole refinement in one launch
+ * whatever the mode; in mode 0 that launch returns to the host after every
+ * four LP rounds. */
 gp_status gp_ctx_set_graph_loops(gp_ctx* ctx, int mode);
 
 /* Spectral initial partition that allocates no device memory.
