@@ -172,38 +172,75 @@ __device__ i64 block_reduce_runs(const u32* keys, const W* vals, i64 count, u32 
     return unique_carry;
 }
 
-// Rows with <= 32 entries: one warp per row, bitonic sort in registers.
+// One row of at most G entries by a group of G lanes: bitonic sort in
+// registers, then the sums of equal targets.  All lanes of the warp call it.
+template <int G, typename W>
+__device__ __forceinline__ void segment_group(bool has, i32 c, i64 s, int len, u32 sentinel, u32* tgt, W* wt,
+                                              i64* row_len) {
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+    u32 k = gl < len ? tgt[s + gl] : 0xffffffffu;
+    W w = gl < len ? wt[s + gl] : W(0);
+#pragma unroll
+    for (int size = 2; size <= G; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            const u32 ok = __shfl_xor_sync(0xffffffffu, k, stride);
+            const W ow = __shfl_xor_sync(0xffffffffu, w, stride);
+            const bool up = (gl & size) == 0, lower = (gl & stride) == 0;
+            if ((lower == up) ? (ok < k) : (ok > k)) { k = ok; w = ow; }
+        }
+    }
+    const u32 prev = __shfl_up_sync(0xffffffffu, k, 1, G);
+    const bool valid = gl < len && k != sentinel;
+    const bool head = valid && (gl == 0 || prev != k);
+    // segmented inclusive sum over runs (runs are contiguous after sorting)
+    W sum = w;
+#pragma unroll
+    for (int d = 1; d < G; d <<= 1) {
+        const W o = __shfl_up_sync(0xffffffffu, sum, d, G);
+        const u32 ok = __shfl_up_sync(0xffffffffu, k, d, G);
+        if (gl >= d && ok == k) sum += o;
+    }
+    const u32 next = __shfl_down_sync(0xffffffffu, k, 1, G);
+    const bool end = valid && (gl == G - 1 || next != k);
+    const unsigned heads = __ballot_sync(0xffffffffu, head) & (G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (lane & ~(G - 1)));
+    const int u = __popc(heads & lanemask_lt()) + (head ? 0 : -1);   // index of this lane's run
+    __syncwarp();
+    if (end) { tgt[s + u] = k; wt[s + u] = sum; }
+    if (has && gl == 0) row_len[c] = __popc(heads);
+}
+
+// Rows of at most 32 entries, two per warp: side by side in half a warp each
+// when both have at most 16 entries (10 exchange steps instead of 2 x 15; the
+// rows of a mesh's coarse levels hold about 12), else one after the other.
+// Grid of 320^3: 13.3 ms with a warp per row, 10.4 so.  A warp per row gains
+// nothing for longer rows either (a symmetrised graph's 17..32 entries: 0.29
+// to 0.33 ms against 0.31, and 0.32 with both rows loaded before the first
+// sort).  Bounded by the exchange steps' issue.
 template <typename W>
 __global__ void __launch_bounds__(kThreads) segment_warp_kernel(i64 rows, const i32* __restrict__ list,
                                                                 const i64* __restrict__ temp_off, u32 sentinel,
                                                                 u32* tgt, W* wt, i64* row_len) {
     const int lane = threadIdx.x & 31;
-    const i64 r = (static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
-    if (r >= rows) return;
-    const i32 c = list[r];
-    const i64 s = temp_off[c];
-    const int len = static_cast<int>(temp_off[c + 1] - s);
-    u32 k = lane < len ? tgt[s + lane] : 0xffffffffu;
-    W w = lane < len ? wt[s + lane] : W(0);
-    warp_bitonic_sort(k, w);
-    const u32 prev = __shfl_up_sync(0xffffffffu, k, 1);
-    const bool valid = lane < len && k != sentinel;
-    const bool head = valid && (lane == 0 || prev != k);
-    // segmented inclusive sum over runs (runs are contiguous after sorting)
-    W sum = w;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const W o = __shfl_up_sync(0xffffffffu, sum, d);
-        const u32 ok = __shfl_up_sync(0xffffffffu, k, d);
-        if (lane >= d && ok == k) sum += o;
+    const i64 r0 = ((static_cast<i64>(blockIdx.x) * kThreads + threadIdx.x) >> 5) * 2;
+    if (r0 >= rows) return;
+    // lanes of the upper half hold the second row
+    const i64 r = r0 + (lane >> 4);
+    const bool has = r < rows;
+    const i32 c = has ? list[r] : 0;
+    const i64 s = has ? temp_off[c] : 0;
+    const int len = has ? static_cast<int>(temp_off[c + 1] - s) : 0;
+    if (!__any_sync(0xffffffffu, len > 16)) {
+        segment_group<16>(has, c, s, len, sentinel, tgt, wt, row_len);
+        return;
     }
-    const u32 next = __shfl_down_sync(0xffffffffu, k, 1);
-    const bool end = valid && (lane == 31 || next != k);
-    const unsigned heads = __ballot_sync(0xffffffffu, head);
-    const int u = __popc(heads & lanemask_lt()) + (head ? 0 : -1);   // index of this lane's run
-    __syncwarp();
-    if (end) { tgt[s + u] = k; wt[s + u] = sum; }
-    if (lane == 0) row_len[c] = __popc(heads);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const i32 hc = __shfl_sync(0xffffffffu, c, half * 16);
+        const i64 hs = __shfl_sync(0xffffffffu, s, half * 16);
+        const int hl = __shfl_sync(0xffffffffu, len, half * 16);
+        if (r0 + half < rows) segment_group<32>(true, hc, hs, hl, sentinel, tgt, wt, row_len);
+    }
 }
 
 // Rows with 33..kWarpSegCap entries: one warp per row, LSD radix sort with

@@ -810,9 +810,9 @@ void sort_rows(Device& d, i64 coarse_n, const Buf<i64>& temp_off_buf, const Buf<
     d.prof_bytes("giant_place_kernel", seg_bytes(6));
     const int key_bits = std::max(1, bit_width_u64(static_cast<u64>(coarse_n)));
     if (rcnt[1])
-        launch(d, "segment_warp_kernel", segment_warp_kernel<W>, blocks_for(static_cast<i64>(rcnt[1]) * 32, kThreads),
-               kThreads, 0, rcnt[1], row_list(1), temp_off, sentinel, tgt, wt,
-               row_len);
+        launch(d, "segment_warp_kernel", segment_warp_kernel<W>,
+               blocks_for((static_cast<i64>(rcnt[1]) + 1) / 2 * 32, kThreads), kThreads, 0, rcnt[1], row_list(1),
+               temp_off, sentinel, tgt, wt, row_len);
     if (rcnt[2]) {
         const size_t smem = static_cast<size_t>(kWarps) * (2 * kWarpSegCap * sizeof(W) +
                                                           (2 * kWarpSegCap + kRadix) * sizeof(u32));

@@ -428,27 +428,6 @@ __device__ void block_radix_sort_segment(K* keys, V* vals, K* keys_alt, V* vals_
     }
 }
 
-// ---------------------------------------------------------------------------
-// Warp bitonic sort of 32 (key, value) pairs, ascending by key.
-// ---------------------------------------------------------------------------
-template <typename K, typename V>
-__device__ __forceinline__ void warp_bitonic_sort(K& key, V& val) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int size = 2; size <= 32; size <<= 1) {
-#pragma unroll
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            const K ok = __shfl_xor_sync(0xffffffffu, key, stride);
-            const V ov = __shfl_xor_sync(0xffffffffu, val, stride);
-            const bool up = (lane & size) == 0;
-            const bool lower = (lane & stride) == 0;
-            // lower lane keeps min when ascending
-            const bool take_other = (lower == up) ? (ok < key) : (ok > key);
-            if (take_other) { key = ok; val = ov; }
-        }
-    }
-}
-
 // Number of significant bits of x (0 for x == 0).
 inline int bit_width_u64(u64 x) {
     int b = 0;
